@@ -54,7 +54,11 @@ __device__ __forceinline__ int64_t place(int x, int y, int z, int P, int rowlen)
   return ((int64_t)z * P + y) * rowlen + x;
 }
 
-template <int NDIMS, bool DECENTERED, bool SQUARE>
+// PACKED: volft_base is a scratch of (re, im, weight, -) float4 per voxel
+// and volw_base unused: one 16-byte reduction per target instead of an
+// 8-byte and a 4-byte one (an L2 reduction costs the same whatever its
+// width), unpacked afterwards by backproject_unpack_kernel.
+template <int NDIMS, bool DECENTERED, bool SQUARE, bool PACKED>
 __global__ void __launch_bounds__(kBpThreads)
 backproject_direct_kernel(float2* __restrict__ volft_base, float* __restrict__ volw_base,
                           const float2* __restrict__ projft, const float* __restrict__ projw,
@@ -78,7 +82,7 @@ backproject_direct_kernel(float2* __restrict__ volft_base, float* __restrict__ v
     const int iv = __ldg(ivolume + slice);
     if (iv < 0) continue;
     int64_t off = (int64_t)iv * a.nvox;
-    if (volft) volft += off;
+    if (volft) volft += PACKED ? 2 * off : off;
     if (volw) volw += off;
   }
   const int half = a.n / 2;
@@ -136,16 +140,38 @@ backproject_direct_kernel(float2* __restrict__ volft_base, float* __restrict__ v
         sim = -sim;
       }
       int64_t o = place<DECENTERED>(tx, ty, tz, a.P, a.rowlen);
-      if (volft) red_add2((float*)(volft + o), iw * sre, iw * sim);
-      if (volw) red_add(volw + o, iw * pw);
+      if (PACKED) {
+        red_add4((float*)(volft + 2 * o), iw * sre, iw * sim, iw * pw, 0.f);
+      } else {
+        if (volft) red_add2((float*)(volft + o), iw * sre, iw * sim);
+        if (volw) red_add(volw + o, iw * pw);
+      }
       if (nx == 0 && (ny != 0 || nz != 0)) {  // x = 0 plane (Backproject.cu:289-319)
         o = place<DECENTERED>(0, -ny, -nz, a.P, a.rowlen);
-        if (volft) red_add2((float*)(volft + o), iw * sre, iw * -sim);
-        if (volw) red_add(volw + o, iw * pw);
+        if (PACKED) {
+          red_add4((float*)(volft + 2 * o), iw * sre, iw * -sim, iw * pw, 0.f);
+        } else {
+          if (volft) red_add2((float*)(volft + o), iw * sre, iw * -sim);
+          if (volw) red_add(volw + o, iw * pw);
+        }
       }
     }
   }
   }  // work loop
+}
+
+// Adds the packed scratch to the volumes; voxels that received nothing are
+// left alone.
+__global__ void __launch_bounds__(256)
+backproject_unpack_kernel(const float4* __restrict__ packed, float2* __restrict__ volft, float* __restrict__ volw,
+                          int64_t n) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const float4 p = packed[i];
+    if (p.x == 0.f && p.y == 0.f && p.z == 0.f) continue;
+    const float2 v = volft[i];
+    volft[i] = make_float2(v.x + p.x, v.y + p.y);
+    volw[i] += p.z;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -677,25 +703,28 @@ backproject_segment_kernel(float2* __restrict__ volft_base, float* __restrict__ 
   }
 }
 
-template <bool DEC, bool SQ>
+template <bool DEC, bool SQ, bool PACKED>
 static void launch_bp_direct(dim3 grid, cudaStream_t stream, float2* vf, float* vw, const float2* pf,
                              const float* pw, const float* mats, const int* ivol, const BpArgs& a,
                              const int* list, const int* nlist, int ndp) {
   if (ndp == 2)
-    backproject_direct_kernel<2, DEC, SQ><<<grid, kBpThreads, 0, stream>>>(vf, vw, pf, pw, mats, ivol, a, list, nlist);
+    backproject_direct_kernel<2, DEC, SQ, PACKED><<<grid, kBpThreads, 0, stream>>>(vf, vw, pf, pw, mats, ivol, a, list,
+                                                                                   nlist);
   else
-    backproject_direct_kernel<3, DEC, SQ><<<grid, kBpThreads, 0, stream>>>(vf, vw, pf, pw, mats, ivol, a, list, nlist);
+    backproject_direct_kernel<3, DEC, SQ, PACKED><<<grid, kBpThreads, 0, stream>>>(vf, vw, pf, pw, mats, ivol, a, list,
+                                                                                   nlist);
 }
 
+template <bool PACKED = false>
 static void launch_bp_direct_any(dim3 grid, cudaStream_t stream, float2* vf, float* vw, const float2* pf,
                                  const float* pw, const float* mats, const int* ivol, const BpArgs& a,
                                  const int* list, const int* nlist, int ndp, int decentered, int square) {
   if (decentered) {
-    if (square) launch_bp_direct<true, true>(grid, stream, vf, vw, pf, pw, mats, ivol, a, list, nlist, ndp);
-    else launch_bp_direct<true, false>(grid, stream, vf, vw, pf, pw, mats, ivol, a, list, nlist, ndp);
+    if (square) launch_bp_direct<true, true, PACKED>(grid, stream, vf, vw, pf, pw, mats, ivol, a, list, nlist, ndp);
+    else launch_bp_direct<true, false, PACKED>(grid, stream, vf, vw, pf, pw, mats, ivol, a, list, nlist, ndp);
   } else {
-    if (square) launch_bp_direct<false, true>(grid, stream, vf, vw, pf, pw, mats, ivol, a, list, nlist, ndp);
-    else launch_bp_direct<false, false>(grid, stream, vf, vw, pf, pw, mats, ivol, a, list, nlist, ndp);
+    if (square) launch_bp_direct<false, true, PACKED>(grid, stream, vf, vw, pf, pw, mats, ivol, a, list, nlist, ndp);
+    else launch_bp_direct<false, false, PACKED>(grid, stream, vf, vw, pf, pw, mats, ivol, a, list, nlist, ndp);
   }
 }
 
@@ -1176,9 +1205,39 @@ static int backproject_launch(float* d_volumeft, float* d_volumeweights, int vx,
                                decentered, square, batch, stream, 1, true, d_ivolume, nvol, fixed_point);
   }
 
-  launch_bp_direct_any(dim3((unsigned)(a.tiles * (int64_t)batch)), stream, (float2*)d_volumeft, d_volumeweights,
-                       (const float2*)d_projft, d_projweights, d_matrices, d_ivolume, a, nullptr, nullptr, ndp,
-                       decentered, square);
+  // The direct kernel, through a packed scratch where that pays: it halves
+  // the reductions (8 instead of 16 per sample, each ~5.5 ps of the L2's
+  // rate) for clearing and adding 16 bytes per voxel (~11 ps) and two small
+  // launches, and its reductions stay in L2 up to a scratch of 160 MB (of
+  // which a sphere is touched).  64^3, 1 000 slices: 145 -> 94 us; 100^3,
+  // 3 333 slices into two volumes: 985 -> 656 us.  Not under stream capture,
+  // where the call allocates nothing.
+  const int nvol = d_ivolume ? nvol_hint : 1;
+  const double samples = (ndp == 3 ? 2.0943951 * rmax : 1.5707963) * (double)rmax * rmax * batch;
+  const int64_t voxels = a.nvox * (int64_t)nvol;
+  const dim3 grid((unsigned)(a.tiles * (int64_t)batch));
+  if (d_volumeft && d_volumeweights && nvol >= 1 && voxels <= (160 << 20) / 16 &&
+      samples >= 0.5 * (double)voxels + 262144.0) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    float4* packed = nullptr;
+    if (cudaStreamIsCapturing(stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone &&
+        pool_alloc((void**)&packed, sizeof(float4) * (size_t)voxels, stream) == GTOMRLN_OK) {
+      cudaError_t e = cudaMemsetAsync(packed, 0, sizeof(float4) * (size_t)voxels, stream);
+      launch_bp_direct_any<true>(grid, stream, (float2*)packed, nullptr, (const float2*)d_projft, d_projweights,
+                                 d_matrices, d_ivolume, a, nullptr, nullptr, ndp, decentered, square);
+      const unsigned blocks = (unsigned)std::min<int64_t>((voxels + 255) / 256, 148 * 16);
+      backproject_unpack_kernel<<<blocks, 256, 0, stream>>>(packed, (float2*)d_volumeft, d_volumeweights, voxels);
+      if (e == cudaSuccess) e = cudaGetLastError();
+      const int st = pool_free(packed, stream);
+      if (e != cudaSuccess)
+        return set_error(GTOMRLN_ERR_CUDA, "launch of the packed backprojector failed: %s", cudaGetErrorString(e));
+      return st;
+    }
+    cudaGetLastError();
+    clear_error();  // no scratch: the plain form
+  }
+  launch_bp_direct_any(grid, stream, (float2*)d_volumeft, d_volumeweights, (const float2*)d_projft, d_projweights,
+                       d_matrices, d_ivolume, a, nullptr, nullptr, ndp, decentered, square);
   GTOMRLN_LAUNCH_CHECK("backproject_direct_kernel");
   return GTOMRLN_OK;
 }
