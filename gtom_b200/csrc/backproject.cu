@@ -23,6 +23,17 @@ namespace gtomrln {
 constexpr int kBpThreads = 256;
 constexpr int kBpPerThread = 2;
 constexpr int kBpTile = kBpThreads * kBpPerThread;
+// The default brick edge (abi.cu), known to the segment kernels at compile
+// time, and the accumulators' row and plane pitch in floats for an edge: a
+// model of the atomics (lanes stepping two voxels along any direction) puts
+// a warp's at 3.04 wavefronts instead of 3.18 with 27 and 27^2.
+constexpr int kBpEdge = 26;
+struct BpPitch {
+  int row, plane;
+};
+__host__ __device__ constexpr BpPitch bp_pitch(int edge) {
+  return edge == kBpEdge ? BpPitch{26, 704} : BpPitch{edge + 1, (edge + 1) * (edge + 1)};
+}
 
 struct BpArgs {
   int n, dimft;
@@ -193,16 +204,17 @@ backproject_unpack_kernel(const float4* __restrict__ packed, float2* __restrict_
 // Fixed-point accumulation of the segment backprojector.  Shared-memory
 // int32 atomics run ~3.3x faster than FP32 ones on B200 (8.9 against 2.6
 // per SM clock, measured), so a work item first accumulates every term as
-// round(w v S) in int32, with S a power of two per item from a radial table
+// round(w v S) in int32, above a bias of 2^30, with S a power of two per item from a radial table
 // of sampled magnitudes: S = 2^25 / (largest sampled |value| in the bands
 // the brick's pixels come from), so a term at that magnitude is 2^25 steps
 // (the terms themselves are formed in FP32 and rounded once).  Every atomic
-// returns the sum before it; if any sum reaches 2^30 in magnitude, or a
-// term exceeds 2^29 (a value 16x above the sampled maximum, or not finite),
+// returns the biased sum before it, whose sign bit is set once the sum
+// reaches 2^30 in magnitude; if any does, or a term exceeds 2^29 (a value 16x above the sampled maximum, or not finite),
 // the item is accumulated again with FP32 atomics, so the result never
 // depends on the sample.  The flush converts the integers with the exact
 // inverse scale.  Squared interpolation weights stay in FP32.
 // ---------------------------------------------------------------------------
+constexpr int kFxBias = 1 << 30;
 constexpr float kFxBand = 16.f;  // voxels of sample radius per band
 constexpr int kFxMaxBands = 128;
 
@@ -334,10 +346,14 @@ __device__ __forceinline__ bool fx_item_scales(const FxBands& f, int3 o, int B, 
 // of place<false> (unsigned compares) instead of being skipped, and every
 // voxel of the faces they fold onto counts as an alias.
 //
+// FACES: neighbouring bricks share the voxels of their faces (the segment
+// kernels' bricks hold every target of their base voxels), which then go by
+// reductions; x = -1 (targets that belong to the mirrored side) is dropped.
+//
 // fx: the accumulators hold fixed-point integers (the segment kernel's
-// fixed-point mode), turned into FP32 by the exact powers of two inv_v (data)
-// and inv_w (weights).
-template <bool DECENTERED, bool CLAMP = false>
+// fixed-point mode) above kFxBias, turned into FP32 by the exact powers of
+// two inv_v (data) and inv_w (weights).
+template <bool DECENTERED, bool CLAMP = false, bool FACES = false>
 __device__ __forceinline__ void bp_flush_brick(float2* __restrict__ volft, float* __restrict__ volw,
                                                const float* are, const float* aim, const float* aw, int B,
                                                int RS, int PS, int3 o, int V, int rowlen, bool exclusive,
@@ -349,12 +365,14 @@ __device__ __forceinline__ void bp_flush_brick(float2* __restrict__ volft, float
       int k = lz * PS + ly * RS + lx;
       float r = are[k], im = aim[k], ww = aw[k];
       if (fx) {
-        r = (float)__float_as_int(r) * inv_v;
-        im = (float)__float_as_int(im) * inv_v;
-        ww = (float)__float_as_int(ww) * inv_w;
+        r = (float)(__float_as_int(r) - kFxBias) * inv_v;
+        im = (float)(__float_as_int(im) - kFxBias) * inv_v;
+        ww = (float)(__float_as_int(ww) - kFxBias) * inv_w;
       }
       if (r == 0.f && im == 0.f && ww == 0.f) continue;
       int x = o.x + lx, y = o.y + ly, z = o.z + lz;
+      if (FACES && x < 0) continue;
+      const bool face = FACES && (lx == 0 || lx == B - 1 || ly == 0 || ly == B - 1 || lz == 0 || lz == B - 1);
       int ys, zs;
       bool alias;
       if (DECENTERED) {
@@ -379,7 +397,7 @@ __device__ __forceinline__ void bp_flush_brick(float2* __restrict__ volft, float
         continue;  // outside the volume: nothing can have been added here
       }
       int64_t idx = ((int64_t)zs * V + ys) * rowlen + x;
-      if (exclusive && !alias) {
+      if (exclusive && !alias && !face) {
         if (volft) {
           float2 c = volft[idx];
           volft[idx] = make_float2(c.x + r, c.y + im);
@@ -488,16 +506,22 @@ backproject_brick_kernel(float2* __restrict__ volft, float* __restrict__ volw,
   }
 }
 
-// Segment variant of the brick backprojector: the same accumulators and
-// flush, but a warp takes a (slice, brick) pair of the segment plan and finds
-// the pixels itself, by row segments (segment.cuh).  Side 0 walks the pixels
-// whose position lies in the brick widened by one voxel below (where their
-// neighbours can reach it) and adds their unconjugated targets, the
-// neighbours with x >= 0; side 1 walks the pixels whose mirrored position
-// does and adds their conjugated targets, the mirrored neighbours (x < 0)
-// and the second insertions on the x = 0 plane.  Each target of each pixel
-// is added once, by the pair of its brick on the side of its conjugation,
-// with the weights and values of the binned variant.
+// Segment variant of the brick backprojector: the warps take records of the
+// segment plan and find the pixels themselves (seg_deal).  Side 0 adds a
+// pixel's unconjugated targets, side 1 the conjugated ones: the mirrored
+// neighbours -n of neighbours n with x < 0, and the second insertions of
+// neighbours on the x = 0 plane, which are -n too.  With the mirrored cube's
+// base voxel -(base + 1) and the roles of the two weights of each axis
+// swapped (the binary16 roundings are then the same operations), side 1 is
+// the same insertion as side 0: the eight voxels of a cube at its base, of
+// which those at x < 0 belong to the other side and, on side 1, the origin
+// receives nothing.  A record's brick owns the cubes whose base voxel lies in
+// it, EDGE - 1 voxels per axis from x = -1 on, and its accumulators hold all
+// their voxels, so every (pixel, side) is walked by one brick only, without
+// tests on its eight targets; neighbouring bricks meet on the voxels of
+// their faces, which the flush adds by reductions, and the plane x = -1 is
+// dropped.  (Bricks that owned the voxels instead visited 12 % of the pixels
+// twice and tested every target.)
 //
 // GEN (centred output only): the general geometry of the reference's
 // insertion — a magnification of the pixel coordinates, the Ewald curvature
@@ -509,24 +533,29 @@ backproject_brick_kernel(float2* __restrict__ volft, float* __restrict__ volw,
 // The grid reaches one voxel past the volume (kept samples come within
 // rmax * scale of the origin) and the flush folds those voxels onto the
 // edge faces with the reference's clamps.
-template <bool DECENTERED, bool SQUARE, bool GEN>
+//
+// EDGE: the accumulators' edge at compile time (the 24 atomics of a sample
+// then share one address register, their offsets immediates), or 0 for the
+// run-time value.
+template <bool DECENTERED, bool SQUARE, bool GEN, int EDGE>
 __global__ void __launch_bounds__(1024)
 backproject_segment_kernel(float2* __restrict__ volft_base, float* __restrict__ volw_base,
                            const float2* __restrict__ projft, const float* __restrict__ projw,
                            const float* __restrict__ mats, BpArgs a, BrickGrid g, PixelSet px, SliceGeom gm,
                            const BrickItem* __restrict__ items, const int* __restrict__ nitems_ptr,
-                           const int* __restrict__ pairs, const PixelBin* __restrict__ bins, int* __restrict__ counter,
-                           FxBands fxb) {
-  extern __shared__ float acc[];
+                           const SegRec* __restrict__ recs, int* __restrict__ counter, FxBands fxb) {
+  extern __shared__ float4 smem4[];  // record slots, then the accumulators
   __shared__ int item_s, next_s, danger_s;
   __shared__ float sv_s, sw_s;
   const int nitems = *nitems_ptr;
-  // Accumulator layout as in backproject_brick_kernel (rows padded to B+1,
-  // planes to (B+1)^2 floats).
-  const int B = g.B, RS = g.B + 1, PS = (g.B + 1) * (g.B + 1), NA = g.B * PS;
-  float* are = acc;
-  float* aim = acc + NA;
-  float* aw = acc + 2 * NA;
+  // accumulators of E voxels per axis
+  const int E = EDGE ? EDGE : g.B + 1, B = E - 1;
+  const int RS = bp_pitch(E).row, PS = bp_pitch(E).plane, NA = E * PS;
+  SegRec* stage = reinterpret_cast<SegRec*>(smem4);
+  float* const acc = reinterpret_cast<float*>(stage + kSegChunk * (blockDim.x >> 5));
+  float* const are = acc;
+  float* const aim = acc + NA;
+  float* const aw = acc + 2 * NA;
   const int lane = threadIdx.x & 31;
   const int V = a.P;
   for (;;) {
@@ -540,129 +569,130 @@ backproject_segment_kernel(float2* __restrict__ volft_base, float* __restrict__ 
     const int3 o = brick_origin(g, it.brick - vol * g.nbricks);
     float2* volft = volft_base && GEN ? volft_base + (int64_t)vol * a.nvox : volft_base;
     float* volw = volw_base && GEN ? volw_base + (int64_t)vol * a.nvox : volw_base;
+    // whether the origin, which side 1 skips, is among the brick's voxels
+    const bool has_origin = o.x <= 0 && o.y <= 0 && o.z <= 0 && o.x + E > 0 && o.y + E > 0 && o.z + E > 0;
 
-    // warps take the item's pairs one at a time, the next one's slice
-    // fetched before the current one is processed; FXM: fixed-point
-    // accumulation (int32 shared atomics of round(w v S)), else FP32
-    // atomics.  Returns with `danger` holding, in its sign bit, whether any
-    // fixed-point sum came within a factor two of overflowing.
-    auto run_pairs = [&](auto fxtag, float sv, float sw, unsigned& danger) {
+    // FXM: fixed-point accumulation (int32 shared atomics of round(w v S)),
+    // else FP32 atomics.  Returns with `danger` holding, in its sign bit,
+    // whether any fixed-point sum came within a factor two of overflowing.
+    auto run_records = [&](auto fxtag, float sv, float sw, unsigned& danger) {
       constexpr bool FXM = decltype(fxtag)::value;
-      auto add3 = [&](int k, float wt, float re, float im, float pwv) {
-        if constexpr (FXM) {
-          const int o1 = atomicAdd(reinterpret_cast<int*>(are) + k, __float2int_rn(wt * re));
-          const int o2 = atomicAdd(reinterpret_cast<int*>(aim) + k, __float2int_rn(wt * im));
-          const int o3 = atomicAdd(reinterpret_cast<int*>(aw) + k, __float2int_rn(wt * pwv));
-          // |old| >= 2^30 sets the sign bit of old + 2^30 (every term is
-          // below 2^29, so no sum can have wrapped while this stays clear)
-          danger |= (unsigned)(o1 + 0x40000000) | (unsigned)(o2 + 0x40000000) | (unsigned)(o3 + 0x40000000);
-        } else {
-          atomicAdd(are + k, wt * re);
-          atomicAdd(aim + k, wt * im);
-          atomicAdd(aw + k, wt * pwv);
-        }
-      };
-      auto take = [&]() {
-        int j = 0;
-        if (lane == 0) j = atomicAdd(&next_s, 1);
-        return __shfl_sync(0xffffffffu, j, 0);
-      };
-      int j = take();
-      int4 pr = j < it.count ? seg_pair(bins, pairs, it.offset + j) : make_int4(0, kSegNoRows, kSegNoRows, 0);
-      while (j < it.count) {
-        const int jn = take();
-        const int4 nx =
-            jn < it.count ? seg_pair(bins, pairs, it.offset + jn) : make_int4(0, kSegNoRows, kSegNoRows, 0);
-        const int slice = pr.x;
-        float m[9];
+      seg_for_each_chunk(recs + it.offset, it.count, stage, &next_s, [&](const SegRec* rec, int rows) {
+        seg_deal(
+            rows,
+            [&](int p, int v, int& ua, int& ub) {
+              const SegWords r = seg_load(rec + p);
+              const bool side = r.ss() & 1;
+              SegBox box = {{r.a.x, r.a.y, r.a.z}, {r.a.w, r.b.x, r.b.y}, {}, {}};
+              float widen = 0.f;
+              if (GEN) {
+                const float* m2 = mats + 9 * (int64_t)(r.ss() >> 1) + 6;
+                const float m[9] = {box.c0[0], box.c0[1], box.c0[2], box.c1[0], box.c1[1],
+                                    box.c1[2], __ldg(m2),  __ldg(m2 + 1), __ldg(m2 + 2)};
+                float me[9];
+                effective_matrix(m, gm, me);
+                widen = curvature_reach(m, gm, px.pmax);
 #pragma unroll
-        for (int k = 0; k < 9; k++) m[k] = __ldg(mats + 9 * (int64_t)slice + k);
-        float me[9];
-        if (GEN) effective_matrix(m, gm, me);
-        const float widen = GEN ? curvature_reach(m, gm, px.pmax) : 0.f;
-        const int64_t sbase = a.elements * slice;
-#pragma unroll 1
-        for (int side = 0; side < 2; side++) {
-          int vlo, vhi;
-          seg_unpack_rows(side ? pr.z : pr.y, vlo, vhi);
-          if (vlo > vhi) continue;  // no pixel of this side
-          const SegBox box = seg_box(GEN ? me : m, side, o, B, 1.f, widen);
-          const bool plane0 = side == 1 && o.x == 0;  // second insertions can land in this brick
-          seg_for_each_pixel_rows(box, px, vlo, vhi, [&](int u, int v, bool valid) {
-            if (!valid) return;
-            float qx = (float)u, qy = (float)v, qz = 0.f;
-            if (GEN) {  // Backproject.cu:176-192, as backproject_direct_kernel
-              qx = fmaf(a.mag.x, (float)u, a.mag.z * (float)v);
-              qy = fmaf(a.mag.y, (float)u, a.mag.w * (float)v);
-              qz = a.ewalddiaminv * (float)(u * u + v * v);
-              if ((int)fmaf(qz, qz, fmaf(qx, qx, qy * qy)) >= a.rmax2) return;
-            }
-            const int idy = v < 0 ? v + a.n : v;
-            const int64_t id = sbase + (int64_t)idy * a.dimft + u;
-            BpSample s = backproject_sample(m, qx, qy, qz);
-            float2 val = projft ? __ldg(projft + id) : make_float2(1.f, 0.f);
-            float pw = projw ? __ldg(projw + id) : 1.f;
-            if (FXM) {  // values in units of the item's fixed-point step
-              val.x *= sv;
-              val.y *= sv;
-              pw *= sw;
-              // larger terms (or non-finite ones) than the scale allows: the
-              // item is redone in FP32
-              if (!(fmaxf(fabsf(val.x), fmaxf(fabsf(val.y), fabsf(pw))) < 536870912.f)) danger |= 0x80000000u;
-            }
-            if (side == 0) {
-              const int lx0 = s.x0 - o.x, ly0 = s.y0 - o.y, lz0 = s.z0 - o.z;
+                for (int k = 0; k < 3; k++) {
+                  box.c0[k] = me[k];
+                  box.c1[k] = me[3 + k];
+                }
+              }
+#pragma unroll
+              for (int k = 0; k < 3; k++) {
+                box.c0[k] = side ? -box.c0[k] : box.c0[k];
+                box.c1[k] = side ? -box.c1[k] : box.c1[k];
+              }
+              seg_box_bounds(box, o, B, widen);
+              seg_row(box, px, v, ua, ub);
+            },
+            [&](int p, int u, int v, bool valid) {
+              if (!valid) return;
+              const SegWords r = seg_load(rec + p);
+              const int slice = r.ss() >> 1;
+              const bool side = r.ss() & 1;
+              float qx = (float)u, qy = (float)v, qz = 0.f;
+              if (GEN) {  // Backproject.cu:176-192, as backproject_direct_kernel
+                qx = fmaf(a.mag.x, (float)u, a.mag.z * (float)v);
+                qy = fmaf(a.mag.y, (float)u, a.mag.w * (float)v);
+                qz = a.ewalddiaminv * (float)(u * u + v * v);
+                if ((int)fmaf(qz, qz, fmaf(qx, qx, qy * qy)) >= a.rmax2) return;
+              }
+              const int64_t id = a.elements * slice + ((v < 0 ? v + a.n : v) * a.dimft + u);
+              float2 val = projft ? __ldg(projft + id) : make_float2(1.f, 0.f);
+              float pw = projw ? __ldg(projw + id) : 1.f;
+              // backproject_sample; the third column meets z = 0 unless GEN
+              float3 pos = make_float3(fmaf(r.a.x, qx, r.a.w * qy), fmaf(r.a.y, qx, r.b.x * qy),
+                                       fmaf(r.a.z, qx, r.b.y * qy));
+              if (GEN) {
+                const float* m2 = mats + 9 * (int64_t)slice + 6;
+                pos.x = fmaf(__ldg(m2), qz, pos.x);
+                pos.y = fmaf(__ldg(m2 + 1), qz, pos.y);
+                pos.z = fmaf(__ldg(m2 + 2), qz, pos.z);
+              }
+              const float x0 = floorf(pos.x + 1e-5f), y0 = floorf(pos.y), z0 = floorf(pos.z);
+              // the cube's base on this side: base, or -(base + 1) mirrored
+              const int sm = side ? -1 : 0;
+              const int lx = ((int)x0 ^ sm) - o.x, ly = ((int)y0 ^ sm) - o.y, lz = ((int)z0 ^ sm) - o.z;
+              if ((unsigned)lx >= (unsigned)B || (unsigned)ly >= (unsigned)B || (unsigned)lz >= (unsigned)B)
+                return;  // another brick's cube
+              const float fx = pos.x - x0, fy = pos.y - y0, fz = pos.z - z0;
+              const float gx = 1.f - fx, gy = 1.f - fy, gz = 1.f - fz;
+              const float ax = side ? fx : gx, bx = side ? gx : fx;
+              const float ay = side ? fy : gy, by = side ? gy : fy;
+              const float az = side ? fz : gz, bz = side ? gz : fz;
+              const float c00 = half_round(ay * az), c10 = half_round(by * az);
+              const float c01 = half_round(ay * bz), c11 = half_round(by * bz);
+              float wt[8] = {half_round(ax * c00), half_round(bx * c00), half_round(ax * c10), half_round(bx * c10),
+                             half_round(ax * c01), half_round(bx * c01), half_round(ax * c11), half_round(bx * c11)};
+              if (SQUARE) {
+#pragma unroll
+                for (int i = 0; i < 8; i++) wt[i] *= wt[i];
+              }
+              if (side) val.y = -val.y;
+              const int k0 = lz * PS + ly * RS + lx;
+              if (has_origin && side) {  // side 1 adds nothing to the origin
+                const int dx = -(o.x + lx), dy = -(o.y + ly), dz = -(o.z + lz);
+                if ((unsigned)dx < 2u && (unsigned)dy < 2u && (unsigned)dz < 2u) {
+#pragma unroll
+                  for (int i = 0; i < 8; i++)
+                    if (i == dx + 2 * dy + 4 * dz) wt[i] = 0.f;
+                }
+              }
+              if (FXM) {  // values in units of the item's fixed-point step
+                val.x *= sv;
+                val.y *= sv;
+                pw *= sw;
+                // larger terms (or non-finite ones) than the scale allows: the
+                // item is redone in FP32
+                if (!(fmaxf(fabsf(val.x), fmaxf(fabsf(val.y), fabsf(pw))) < 536870912.f)) danger |= 0x80000000u;
+              }
 #pragma unroll
               for (int i = 0; i < 8; i++) {
-                const int dx = i & 1, dy = (i >> 1) & 1, dz = (i >> 2) & 1;
-                const int lx = lx0 + dx, ly = ly0 + dy, lz = lz0 + dz;
-                if (s.x0 + dx >= 0 && (unsigned)lx < (unsigned)B && (unsigned)ly < (unsigned)B &&
-                    (unsigned)lz < (unsigned)B) {
-                  const float wt = SQUARE ? s.w[i] * s.w[i] : s.w[i];
-                  add3(lz * PS + ly * RS + lx, wt, val.x, val.y, pw);
+                const int k = k0 + (i & 1) + ((i >> 1) & 1) * RS + ((i >> 2) & 1) * PS;
+                if constexpr (FXM) {
+                  const int o1 = atomicAdd(reinterpret_cast<int*>(are) + k, __float2int_rn(wt[i] * val.x));
+                  const int o2 = atomicAdd(reinterpret_cast<int*>(aim) + k, __float2int_rn(wt[i] * val.y));
+                  const int o3 = atomicAdd(reinterpret_cast<int*>(aw) + k, __float2int_rn(wt[i] * pw));
+                  // a biased sum is negative once |sum| >= 2^30 (every term is
+                  // below 2^29, so no sum can have wrapped while none is)
+                  danger |= (unsigned)o1 | (unsigned)o2 | (unsigned)o3;
+                } else {
+                  atomicAdd(are + k, wt[i] * val.x);
+                  atomicAdd(aim + k, wt[i] * val.y);
+                  atomicAdd(aw + k, wt[i] * pw);
                 }
               }
-            } else {
-              // mirrored neighbour -n of n = base + (dx, dy, dz), local coordinates
-              const int lx0 = -s.x0 - o.x, ly0 = -s.y0 - o.y, lz0 = -s.z0 - o.z;
-#pragma unroll
-              for (int i = 0; i < 8; i++) {
-                const int dx = i & 1, dy = (i >> 1) & 1, dz = (i >> 2) & 1;
-                const int lx = lx0 - dx, ly = ly0 - dy, lz = lz0 - dz;
-                if (s.x0 + dx < 0 && (unsigned)lx < (unsigned)B && (unsigned)ly < (unsigned)B &&
-                    (unsigned)lz < (unsigned)B) {
-                  const float wt = SQUARE ? s.w[i] * s.w[i] : s.w[i];
-                  add3(lz * PS + ly * RS + lx, wt, val.x, -val.y, pw);
-                }
-              }
-              if (plane0) {
-                // second insertion at (0, -ny, -nz) of each neighbour with
-                // nx == 0 and (ny, nz) != 0; here o.x == 0, so local x is 0
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                  const int dx = i & 1, dy = (i >> 1) & 1, dz = (i >> 2) & 1;
-                  const int ny = s.y0 + dy, nz = s.z0 + dz;
-                  const int ly = -ny - o.y, lz = -nz - o.z;
-                  if (s.x0 + dx == 0 && (ny != 0 || nz != 0) && (unsigned)ly < (unsigned)B &&
-                      (unsigned)lz < (unsigned)B) {
-                    const float wt = SQUARE ? s.w[i] * s.w[i] : s.w[i];
-                    add3(lz * PS + ly * RS, wt, val.x, -val.y, pw);
-                  }
-                }
-              }
-            }
-          });
-        }
-        j = jn;
-        pr = nx;
-      }
+            });
+      });
     };
 
     // Fixed point first where a scale is known; if any sum of the item came
     // near overflow, the item is accumulated again in FP32.
     bool fx = !SQUARE && fxb.vmax != nullptr;
     for (;;) {
-      for (int k = threadIdx.x; k < 3 * NA; k += blockDim.x) acc[k] = 0.f;
+      const float zero = fx ? __int_as_float(kFxBias) : 0.f;
+      for (int k = threadIdx.x; k < 3 * NA; k += blockDim.x) acc[k] = zero;
       if (threadIdx.x == 0) {
         next_s = 0;
         danger_s = 0;
@@ -684,9 +714,9 @@ backproject_segment_kernel(float2* __restrict__ volft_base, float* __restrict__ 
       }
       unsigned danger = 0;
       if (fx)
-        run_pairs(std::true_type(), sv_s, sw_s, danger);
+        run_records(std::true_type(), sv_s, sw_s, danger);
       else
-        run_pairs(std::false_type(), 1.f, 1.f, danger);
+        run_records(std::false_type(), 1.f, 1.f, danger);
       if (fx && __any_sync(0xffffffffu, (int)danger < 0) && lane == 0) danger_s = 1;
       __syncthreads();
       if (fx && danger_s) {
@@ -698,8 +728,8 @@ backproject_segment_kernel(float2* __restrict__ volft_base, float* __restrict__ 
     }
 
     // flush the brick into the volume
-    bp_flush_brick<DECENTERED, GEN>(volft, volw, are, aim, aw, B, RS, PS, o, V, a.rowlen, it.exclusive != 0, fx,
-                                    fx ? 1.f / sv_s : 1.f, fx ? 1.f / sw_s : 1.f);
+    bp_flush_brick<DECENTERED, GEN, true>(volft, volw, are, aim, aw, E, RS, PS, o, V, a.rowlen, it.exclusive != 0, fx,
+                                          fx ? 1.f / sv_s : 1.f, fx ? 1.f / sw_s : 1.f);
   }
 }
 
@@ -764,6 +794,17 @@ static int device_max_index(const int* d_iv, unsigned n, cudaStream_t stream, in
   return GTOMRLN_OK;
 }
 
+// The segment kernel's instance for a geometry and output.
+template <int EDGE>
+static auto segment_kernel(bool gen, int decentered, int square) {
+  return gen ? (square ? backproject_segment_kernel<false, true, true, EDGE>
+                       : backproject_segment_kernel<false, false, true, EDGE>)
+         : decentered ? (square ? backproject_segment_kernel<true, true, false, EDGE>
+                                : backproject_segment_kernel<true, false, false, EDGE>)
+                      : (square ? backproject_segment_kernel<false, true, false, EDGE>
+                                : backproject_segment_kernel<false, false, false, EDGE>);
+}
+
 // The brick path: plan, brick kernel, and the direct kernel for any slice the
 // plan could not take.  Nothing synchronises.  gen: magnification, Ewald
 // curvature or per-slice volumes (centred output, row segments only;
@@ -782,15 +823,17 @@ static int backproject_brick(float* d_volumeft, float* d_volumeweights, const fl
   const int ext = gen ? 1 : 0;
   const float limit = (float)(std::min(V / 2, yhi) + ext) - 1e-4f;
   const BrickTuning tune = brick_tuning(GTOMRLN_OP_BACKPROJECT);
-  BrickGrid g = make_brick_grid(V, tune.edge, V / 2 + ext, -(V / 2) - ext, yhi + ext);
-  size_t smem = sizeof(float) * 3 * (size_t)tune.edge * (tune.edge + 1) * (tune.edge + 1);
+  // Segment bricks own cubes by their base voxel (x from -1 on: cubes that
+  // straddle x = 0) and store one voxel more per axis, tune.edge in all.
+  BrickGrid g = segments ? make_brick_grid(V, tune.edge - 1, V / 2 + ext - 1, -(V / 2) - ext, yhi + ext - 1, -1)
+                         : make_brick_grid(V, tune.edge, V / 2 + ext, -(V / 2) - ext, yhi + ext);
+  const size_t smem = segments ? sizeof(float) * 3 * (size_t)tune.edge * bp_pitch(tune.edge).plane +
+                                     seg_stage_bytes(tune.threads)
+                               : sizeof(float) * 3 * (size_t)tune.edge * (tune.edge + 1) * (tune.edge + 1);
   auto kern = decentered ? (square ? backproject_brick_kernel<true, true> : backproject_brick_kernel<true, false>)
                          : (square ? backproject_brick_kernel<false, true> : backproject_brick_kernel<false, false>);
-  auto skern = gen ? (square ? backproject_segment_kernel<false, true, true>
-                             : backproject_segment_kernel<false, false, true>)
-               : decentered
-                   ? (square ? backproject_segment_kernel<true, true, false> : backproject_segment_kernel<true, false, false>)
-                   : (square ? backproject_segment_kernel<false, true, false> : backproject_segment_kernel<false, false, false>);
+  const auto skern = tune.edge == kBpEdge ? segment_kernel<kBpEdge>(gen, decentered, square)
+                                          : segment_kernel<0>(gen, decentered, square);
   cudaError_t e = segments ? cudaFuncSetAttribute(skern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
                            : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess)
@@ -862,7 +905,7 @@ static int backproject_brick(float* d_volumeft, float* d_volumeweights, const fl
   if (segments)
     skern<<<sms * std::max(occ, 1), tune.threads, smem, stream>>>(
         (float2*)d_volumeft, d_volumeweights, (const float2*)d_projft, d_projweights, d_mats, a, g, px, gm,
-        plan.items, plan.nitems, plan.pairs, plan.bins, plan.counter, fxb);
+        plan.items, plan.nitems, plan.recs, plan.counter, fxb);
   else
     kern<<<sms * std::max(occ, 1), tune.threads, smem, stream>>>(
         (float2*)d_volumeft, d_volumeweights, (const float2*)d_projft, d_projweights, d_mats, a, g, plan.items,
@@ -968,27 +1011,29 @@ backproject_shifted_kernel(float2* __restrict__ volft, float* __restrict__ volw,
 // position's base voxel, the sample times exp(i phi) and the slice's weight),
 // with the targets accumulated per shared-memory brick as in
 // backproject_segment_kernel.  Side 0 walks the unflipped samples, side 1
-// the flipped ones (negated positions), each over the brick widened by one
-// voxel below; a sample's eight targets are added by the pairs of their
-// bricks on the side of its flip.  Centred output.  The brick grid reaches one
-// voxel past the volume (the insertion takes the whole rmax disk, so at
-// padding 2 the rim's cubes reach x = V/2 + 1), and the flush folds those
-// voxels onto the edge with the direct kernel's clamps.
+// the flipped ones (the records' columns are negated there), each added by
+// the brick of its base voxel.  Centred output.  The insertion takes the
+// whole rmax disk, so at padding 2 the rim's cubes reach one voxel past the
+// volume (x = V/2 + 1), and the flush folds those voxels onto the edge with
+// the direct kernel's clamps.
+template <int EDGE>
 __global__ void __launch_bounds__(1024)
 backproject_shifted_segment_kernel(float2* __restrict__ volft, float* __restrict__ volw,
                                    const float2* __restrict__ projft, const float* __restrict__ projw,
-                                   const float* __restrict__ mats, const float* __restrict__ shifts,
-                                   const float* __restrict__ gweights, BpArgs a, BrickGrid g, PixelSet px,
-                                   const BrickItem* __restrict__ items, const int* __restrict__ nitems_ptr,
-                                   const int* __restrict__ pairs, const PixelBin* __restrict__ bins, int* __restrict__ counter) {
-  extern __shared__ float acc[];
+                                   const float* __restrict__ shifts, const float* __restrict__ gweights, BpArgs a,
+                                   BrickGrid g, PixelSet px, const BrickItem* __restrict__ items,
+                                   const int* __restrict__ nitems_ptr, const SegRec* __restrict__ recs,
+                                   int* __restrict__ counter) {
+  extern __shared__ float4 smem4[];  // record slots, then the accumulators
   __shared__ int item_s, next_s;
   const int nitems = *nitems_ptr;
-  const int B = g.B, RS = g.B + 1, PS = (g.B + 1) * (g.B + 1), NA = g.B * PS;
-  float* are = acc;
-  float* aim = acc + NA;
-  float* aw = acc + 2 * NA;
-  const int lane = threadIdx.x & 31;
+  const int E = EDGE ? EDGE : g.B + 1, B = E - 1;
+  const int RS = bp_pitch(E).row, PS = bp_pitch(E).plane, NA = E * PS;
+  SegRec* stage = reinterpret_cast<SegRec*>(smem4);
+  float* const acc = reinterpret_cast<float*>(stage + kSegChunk * (blockDim.x >> 5));
+  float* const are = acc;
+  float* const aim = acc + NA;
+  float* const aw = acc + 2 * NA;
   const int V = a.P;
   for (;;) {
     __syncthreads();
@@ -1002,81 +1047,58 @@ backproject_shifted_segment_kernel(float2* __restrict__ volft, float* __restrict
     if (w >= nitems) break;
     const BrickItem it = items[w];
     const int3 o = brick_origin(g, it.brick);
-    auto take = [&]() {
-      int j = 0;
-      if (lane == 0) j = atomicAdd(&next_s, 1);
-      return __shfl_sync(0xffffffffu, j, 0);
-    };
-    int j = take();
-    int4 pr = j < it.count ? seg_pair(bins, pairs, it.offset + j) : make_int4(0, kSegNoRows, kSegNoRows, 0);
-    while (j < it.count) {
-      const int jn = take();
-      const int4 nx = jn < it.count ? seg_pair(bins, pairs, it.offset + jn) : make_int4(0, kSegNoRows, kSegNoRows, 0);
-      const int slice = pr.x;
-      float m[9];
+    seg_for_each_chunk(recs + it.offset, it.count, stage, &next_s, [&](const SegRec* rec, int rows) {
+      seg_deal(
+          rows,
+          [&](int p, int v, int& ua, int& ub) {
+            const SegWords r = seg_load(rec + p);
+            SegBox box = {{r.a.x, r.a.y, r.a.z}, {r.a.w, r.b.x, r.b.y}, {}, {}};
+            seg_box_bounds(box, o, B, 0.f);
+            seg_row(box, px, v, ua, ub);
+          },
+          [&](int p, int u, int v, bool valid) {
+            if (!valid) return;
+            const SegWords r = seg_load(rec + p);
+            const int slice = r.ss() >> 1;
+            const bool side = r.ss() & 1;
+            const float fu = (float)u, fv = (float)v;
+            const float qx = fmaf(r.a.x, fu, r.a.w * fv), qy = fmaf(r.a.y, fu, r.b.x * fv),
+                        qz = fmaf(r.a.z, fu, r.b.y * fv);
+            const bool flip = (side ? -qx : qx) + 1e-5f < 0.f;
+            if (flip != side) return;  // the other side's sample
+            const float x0 = floorf(qx + 1e-5f), y0 = floorf(qy), z0 = floorf(qz);
+            const int lx = (int)x0 - o.x, ly = (int)y0 - o.y, lz = (int)z0 - o.z;
+            if ((unsigned)lx >= (unsigned)B || (unsigned)ly >= (unsigned)B || (unsigned)lz >= (unsigned)B)
+              return;  // another brick's cube
+            const float fx = qx - x0, fy = qy - y0, fz = qz - z0;
+            const float c0 = 1.f - fz, c1 = fz;
+            const float c00 = (1.f - fy) * c0, c10 = fy * c0, c01 = (1.f - fy) * c1, c11 = fy * c1;
+            const float wt[8] = {(1.f - fx) * c00, fx * c00, (1.f - fx) * c10, fx * c10,
+                                 (1.f - fx) * c01, fx * c01, (1.f - fx) * c11, fx * c11};
+            const int64_t id = a.elements * slice + ((v < 0 ? v + a.n : v) * a.dimft + u);
+            const float2 val = projft ? __ldg(projft + id) : make_float2(1.f, 0.f);
+            const float sx = __ldg(shifts + 3 * (int64_t)slice), sy = __ldg(shifts + 3 * (int64_t)slice + 1);
+            const float gw = __ldg(gweights + slice);
+            float phase = fmaf(fu, sx, fv * sy);
+            phase = -phase;
+            const float c = __cosf(phase), sn = __sinf(phase);
+            float re = fmaf(val.x, c, -(val.y * sn)), im = fmaf(val.x, sn, val.y * c);
+            im *= side ? -1.f : 1.f;
+            re *= gw;
+            im *= gw;
+            const float pw = (projw ? __ldg(projw + id) : 1.f) * gw;
+            const int k0 = lz * PS + ly * RS + lx;
 #pragma unroll
-      for (int k = 0; k < 9; k++) m[k] = __ldg(mats + 9 * (int64_t)slice + k);
-      const float sx = __ldg(shifts + 3 * (int64_t)slice), sy = __ldg(shifts + 3 * (int64_t)slice + 1);
-      const float gw = __ldg(gweights + slice);
-      const int64_t sbase = a.elements * slice;
-#pragma unroll 1
-      for (int side = 0; side < 2; side++) {
-        int vlo, vhi;
-        seg_unpack_rows(side ? pr.z : pr.y, vlo, vhi);
-        if (vlo > vhi) continue;  // no pixel of this side
-        const SegBox box = seg_box(m, side, o, B, 1.f);
-        seg_for_each_pixel_rows(box, px, vlo, vhi, [&](int u, int v, bool valid) {
-          if (!valid) return;
-          float3 pos = mat_apply(m, (float)u, (float)v, 0.f);
-          const bool flip = pos.x + 1e-5f < 0.f;
-          if (flip != (side == 1)) return;  // the other side's sample
-          float sign = 1.f;
-          if (flip) {
-            pos.x = fabsf(pos.x);
-            pos.y = -pos.y;
-            pos.z = -pos.z;
-            sign = -1.f;
-          }
-          const int x0 = (int)floorf(pos.x + 1e-5f);
-          const float fx = pos.x - (float)x0;
-          const int y0 = (int)floorf(pos.y);
-          const float fy = pos.y - (float)y0;
-          const int z0 = (int)floorf(pos.z);
-          const float fz = pos.z - (float)z0;
-          const int lx0 = x0 - o.x, ly0 = y0 - o.y, lz0 = z0 - o.z;
-          if (lx0 < -1 || lx0 >= B || ly0 < -1 || ly0 >= B || lz0 < -1 || lz0 >= B) return;
-          const float c0 = 1.f - fz, c1 = fz;
-          const float c00 = (1.f - fy) * c0, c10 = fy * c0, c01 = (1.f - fy) * c1, c11 = fy * c1;
-          const float wt[8] = {(1.f - fx) * c00, fx * c00, (1.f - fx) * c10, fx * c10,
-                               (1.f - fx) * c01, fx * c01, (1.f - fx) * c11, fx * c11};
-          const int idy = v < 0 ? v + a.n : v;
-          const int64_t id = sbase + (int64_t)idy * a.dimft + u;
-          const float2 val = projft ? __ldg(projft + id) : make_float2(1.f, 0.f);
-          float phase = fmaf((float)u, sx, (float)v * sy);
-          phase = -phase;
-          const float c = __cosf(phase), sn = __sinf(phase);
-          float re = fmaf(val.x, c, -(val.y * sn)), im = fmaf(val.x, sn, val.y * c);
-          im *= sign;
-          re *= gw;
-          im *= gw;
-          const float pw = (projw ? __ldg(projw + id) : 1.f) * gw;
-#pragma unroll
-          for (int i = 0; i < 8; i++) {
-            const int lx = lx0 + (i & 1), ly = ly0 + ((i >> 1) & 1), lz = lz0 + ((i >> 2) & 1);
-            if ((unsigned)lx < (unsigned)B && (unsigned)ly < (unsigned)B && (unsigned)lz < (unsigned)B) {
-              const int k = lz * PS + ly * RS + lx;
+            for (int i = 0; i < 8; i++) {
+              const int k = k0 + (i & 1) + ((i >> 1) & 1) * RS + ((i >> 2) & 1) * PS;
               atomicAdd(are + k, wt[i] * re);
               atomicAdd(aim + k, wt[i] * im);
               atomicAdd(aw + k, wt[i] * pw);
             }
-          }
-        });
-      }
-      j = jn;
-      pr = nx;
-    }
+          });
+    });
     __syncthreads();
-    bp_flush_brick<false, true>(volft, volw, are, aim, aw, B, RS, PS, o, V, a.rowlen, it.exclusive != 0);
+    bp_flush_brick<false, true, true>(volft, volw, are, aim, aw, E, RS, PS, o, V, a.rowlen, it.exclusive != 0);
   }
 }
 
@@ -1087,21 +1109,22 @@ static int backproject_shifted_brick(float* d_volumeft, float* d_volumeweights, 
                                      const float* d_gweights, const BpArgs& a, int rmax, unsigned batch,
                                      cudaStream_t stream) {
   const int V = a.P;
-  // While every sample radius stays below V/2 + 0.99, the cubes' voxels lie
-  // in x [0, V/2 + 1] and y, z [-V/2 - 1, V/2 + 1] (centred, before clamps).
+  // While every sample radius stays below V/2 + 0.99, the cubes' base voxels
+  // lie in x [0, V/2] and y, z [-V/2 - 1, V/2] (centred, before clamps).
   const float limit = (float)(V / 2) + 0.99f;
   const BrickTuning tune = brick_tuning(GTOMRLN_OP_BACKPROJECT);
-  BrickGrid g = make_brick_grid(V, tune.edge, V / 2 + 1, -(V / 2) - 1, V / 2 + 1);
-  size_t smem = sizeof(float) * 3 * (size_t)tune.edge * (tune.edge + 1) * (tune.edge + 1);
-  cudaError_t e = cudaFuncSetAttribute(backproject_shifted_segment_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  BrickGrid g = make_brick_grid(V, tune.edge - 1, V / 2, -(V / 2) - 1, V / 2);
+  const size_t smem = sizeof(float) * 3 * (size_t)tune.edge * bp_pitch(tune.edge).plane + seg_stage_bytes(tune.threads);
+  const auto kern = tune.edge == kBpEdge ? backproject_shifted_segment_kernel<kBpEdge>
+                                         : backproject_shifted_segment_kernel<0>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess)
     return set_error(GTOMRLN_ERR_CUDA, "shifted brick backprojector: %zu B of shared memory refused: %s", smem,
                      cudaGetErrorString(e));
   int dev = 0, sms = 148, occ = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, backproject_shifted_segment_kernel, tune.threads, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, tune.threads, smem);
   PixelSet px;
   px.n = a.n;
   px.dimft = a.dimft;
@@ -1110,12 +1133,14 @@ static int backproject_shifted_brick(float* d_volumeft, float* d_volumeweights, 
   px.strict = 0;  // r^2 <= rmax^2, the whole x = 0 column
   px.pmax = (float)rmax;
   BrickPlan plan;
-  int st = build_brick_plan(GTOMRLN_OP_BACKPROJECT, d_mats, (int)batch, g, px, limit, tune.chunk, stream, &plan,
-                            1);
+  SliceGeom gm;
+  gm.negate = 1;
+  int st = build_brick_plan(GTOMRLN_OP_BACKPROJECT, d_mats, (int)batch, g, px, limit, tune.chunk, stream, &plan, 1,
+                            nullptr, gm);
   if (st) return st;
-  backproject_shifted_segment_kernel<<<sms * std::max(occ, 1), tune.threads, smem, stream>>>(
-      (float2*)d_volumeft, d_volumeweights, (const float2*)d_projft, d_projweights, d_mats, d_shifts, d_gweights,
-      a, g, px, plan.items, plan.nitems, plan.pairs, plan.bins, plan.counter);
+  kern<<<sms * std::max(occ, 1), tune.threads, smem, stream>>>(
+      (float2*)d_volumeft, d_volumeweights, (const float2*)d_projft, d_projweights, d_shifts, d_gweights, a, g, px,
+      plan.items, plan.nitems, plan.recs, plan.counter);
   backproject_shifted_kernel<2><<<sms * 4, kBpThreads, 0, stream>>>(
       (float2*)d_volumeft, d_volumeweights, (const float2*)d_projft, d_projweights, d_mats, d_shifts, d_gweights,
       a, rmax, plan.fallback, plan.nfallback);

@@ -15,6 +15,10 @@
 //     mirroring and the x = 0 plane's second insertion), and counting-sorts
 //     its pixel ids by brick: one "bin" per (slice, brick);
 //  2. the bins are grouped by brick and cut into work items.
+//
+// The segment plan replaces the bins by one record per (slice, side, brick)
+// whose box the slice's plane crosses, and the kernels find the pixels
+// themselves (segment.cuh).
 #pragma once
 
 #include "common.cuh"
@@ -27,21 +31,22 @@ struct BrickGrid {
   int nbx, nby, nbz;
   int ylo, zlo;  // signed coordinate of brick row/plane 0
   int nbricks;
+  int xlo;       // and of brick column 0
 };
+
+struct SegRec;  // segment.cuh
 
 struct BrickItem {
   int brick;      // brick index
-  int offset;     // first entry in the pair list
-  int count;      // bins (slice, pixel run) in this item
+  int offset;     // first entry in the pair list (segment plan: first record)
+  int count;      // bins (slice, pixel run) or records in this item
   int exclusive;  // 1 if this is the brick's only item (no other CTA writes it)
 };
 
 // A (slice, brick) bin: `count` pixel ids starting at entries[start]; the
 // first `interior` of them are pixels whose whole 2x2x2 target cube (direct
 // or mirrored, away from the x = 0 plane) lies inside the brick, so a warp
-// can treat them with one branch-free path.  In a segment plan the bin
-// lists no pixels: start and count hold the packed row ranges of the
-// pair's side 0 and side 1 (seg_pack_rows).
+// can treat them with one branch-free path.
 struct PixelBin {
   int slice, start, count, brick, interior, pad0, pad1, pad2;
 };
@@ -51,7 +56,7 @@ __host__ __device__ inline int3 brick_origin(const BrickGrid& g, int b) {
   int t = b / g.nbx;
   int by = t % g.nby;
   int bz = t / g.nby;
-  return make_int3(bx * g.B, g.ylo + by * g.B, g.zlo + bz * g.B);
+  return make_int3(g.xlo + bx * g.B, g.ylo + by * g.B, g.zlo + bz * g.B);
 }
 
 // floor(x / B) for 0 <= x < 2^20 without an integer division: a float
@@ -82,11 +87,12 @@ __device__ __forceinline__ float plane_scale(const float* m) {
   return sqrtf(0.5f * (g00 + g11) + sqrtf(h * h + g01 * g01)) * (1.f + 1e-6f);
 }
 
-inline BrickGrid make_brick_grid(int V, int B, int xhi, int ylo, int yhi) {
+inline BrickGrid make_brick_grid(int V, int B, int xhi, int ylo, int yhi, int xlo = 0) {
   BrickGrid g;
   g.V = V;
   g.B = B;
-  g.nbx = (xhi + 1 + B - 1) / B;
+  g.xlo = xlo;
+  g.nbx = (xhi - xlo + 1 + B - 1) / B;
   g.nby = (yhi - ylo + 1 + B - 1) / B;
   g.nbz = g.nby;
   g.ylo = ylo;
@@ -116,6 +122,7 @@ struct SliceGeom {
   const int* ivolume = nullptr;  // per-slice volume index (device), or none
   int nvol = 1;                  // volumes the plan spans (ivolume values in [0, nvol))
   float qmax = -1.f;  // bound on |q| of the samples kept (magnified radius test); < 0: the pixel set's pmax
+  int negate = 0;     // the records' columns are negated on side 1 (kernels that flip the whole sample)
 };
 
 // The map pixel (u, v) -> u c0' + v c1' of the enumeration: the matrix's
@@ -146,7 +153,8 @@ struct BrickPlan {
   int max_items = 0;
   BrickItem* items = nullptr;
   int* nitems = nullptr;      // number of valid items
-  int* pairs = nullptr;       // per brick: indices into bins
+  SegRec* recs = nullptr;     // segment plan: the records, grouped by brick
+  int* pairs = nullptr;       // binning plan: per brick, indices into bins
   PixelBin* bins = nullptr;
   int* entries = nullptr;     // pixel ids, grouped by bin
   int* counter = nullptr;     // work counter of the persistent kernel (starts at 0)
@@ -161,15 +169,16 @@ struct BrickPlan {
 // voxel).  A slice whose samples could reach radius `limit` (beyond which
 // the brick kernels would need the reference's clamps) is not planned but
 // listed in plan->fallback for the direct kernels.  chunk caps the bins per
-// work item.  segments = 1 builds the segment plan instead: bins without
-// entries, one per (slice, brick) pair whose brick the slice's plane
-// crosses, and the kernels enumerate the pixels themselves (segment.cuh).
+// work item.  segments = 1 builds the segment plan instead: one record per
+// (slice, side, brick) whose brick can hold base voxels of the slice's
+// samples (side 0) or of their mirrored positions (side 1), and the kernels
+// enumerate the pixels themselves (segment.cuh).
 // With a segment plan, zero_out (the projector's output, complex, elements
 // per slice as px) receives the zeros outside px's radius for every planned
 // slice, in the plan's own per-slice pass.
 // geom (segment plans only): magnification, curvature and per-slice volumes
-// of the backprojector's general case; the plan then lists one pair per
-// (slice, volume-brick key) and its enumeration boxes are widened by the
+// of the backprojector's general case; the plan then lists records by
+// volume-brick key and its enumeration boxes are widened by the
 // curvature's reach.
 int build_brick_plan(int op, const float* d_mats, int batch, const BrickGrid& g, const PixelSet& px,
                      float limit, int chunk, cudaStream_t stream, BrickPlan* plan, int segments = 0,

@@ -5,13 +5,13 @@
 //                       shared-memory histogram over bricks, the slice's bins
 //                       and its pixel ids sorted by brick;
 //   segment_pairs_kernel  (segment plan, instead of the above) one CTA per
-//                       slice: the bricks its plane crosses, as bins
-//                       without pixel lists;
-//   pairs_scan_kernel   one CTA: per-brick bin offsets and work items, bricks
+//                       slice: the bricks its plane crosses, per side, each
+//                       with its row range and its rank within the brick;
+//   pairs_scan_kernel   one CTA: per-brick offsets and the work items, bricks
 //                       in order of increasing distance from the origin so
 //                       that the heaviest items start first;
 //   pairs_fill_kernel   groups the bins by brick;
-//   plan_items_kernel   writes the work items.
+//   segment_fill_kernel (segment plan, instead) writes the records, grouped.
 #include <algorithm>
 #include <cmath>
 #include <map>
@@ -252,26 +252,30 @@ bin_slices_kernel(const float* __restrict__ mats, BrickGrid g, PixelSet px, floa
   });
 }
 
-// Segment plan: one CTA per slice lists the bricks whose box, widened by
-// `below` voxels on the low side and by the segment margin, meets the
-// slice's plane within the radius its samples reach.  Each becomes a bin
-// without entries; the brick kernel finds the pixels by row segments
+// Segment plan: one CTA per slice lists the bricks whose box, widened by the
+// segment margin, meets the slice's plane within the radius its samples
+// reach, per side (0: positions, 1: mirrored positions) where it can hold
+// rows of the slice.  The brick kernels find the pixels by row segments
 // (segment.cuh).  Positions of a slice lie on the plane through the origin
 // spanned by the first two (magnified) matrix columns and within
 // plane_scale * pmax of the origin, mirrored positions too, so the list
 // covers every brick a pixel of the slice (or its mirror) can reach; with
 // the Ewald curvature the samples leave the plane by at most its reach,
-// which widens every box.  With per-slice volumes a pair's key is
+// which widens every box.  With per-slice volumes the key is
 // volume * nbricks + brick; a slice whose volume index is outside
-// [0, nvol) takes the direct path.
+// [0, nvol), or whose third column is not finite (the kernels of flat
+// slices leave it out), takes the direct path.
+struct SegBin {
+  int ss, rows, key, rank;  // as in SegRec; the volume-brick key and the bin's rank within it
+};
 constexpr int kPairThreads = 256;
 __global__ void __launch_bounds__(kPairThreads)
-segment_pairs_kernel(const float* __restrict__ mats, BrickGrid g, float pmax, float limit, float below,
-                     PixelBin* __restrict__ bins, int64_t bins_cap, unsigned long long* __restrict__ counters,
+segment_pairs_kernel(const float* __restrict__ mats, BrickGrid g, float pmax, float limit,
+                     SegBin* __restrict__ bins, int64_t bins_cap, unsigned long long* __restrict__ counters,
                      int* __restrict__ brick_pairs, int* __restrict__ fallback, int* __restrict__ nfallback,
                      float2* __restrict__ zero_out, PixelSet zpx, SliceGeom gm) {
   extern __shared__ int hits[];  // brick ids of this slice, then a bitmap of the bricks
-  __shared__ int s_n;
+  __shared__ int s_n, s_m, s_put;
   __shared__ int s_wsum[kPairThreads / 32];
   __shared__ long long s_base;
   const int slice = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
@@ -284,7 +288,7 @@ segment_pairs_kernel(const float* __restrict__ mats, BrickGrid g, float pmax, fl
   const float widen = curvature_reach(m0, gm, pmax);
   const float R = plane_scale(m0) * (gm.qmax < 0.f ? pmax : gm.qmax) + widen;
   const int vol = gm.ivolume ? __ldg(gm.ivolume + slice) : 0;
-  if (!(R < limit) || vol < 0 || vol >= gm.nvol) {  // uniform over the block
+  if (!(R < limit) || vol < 0 || vol >= gm.nvol || !isfinite(m0[6] + m0[7] + m0[8])) {  // uniform over the block
     if (tid == 0) fallback[atomicAdd(nfallback, 1)] = slice;
     return;
   }
@@ -300,11 +304,11 @@ segment_pairs_kernel(const float* __restrict__ mats, BrickGrid g, float pmax, fl
       for (int x = x0 + lane; x < zpx.dimft; x += 32) out[(int64_t)idy * zpx.dimft + x] = make_float2(0.f, 0.f);
     }
   }
-  if (tid == 0) s_n = 0;
+  if (tid == 0) s_n = s_m = s_put = 0;
   __syncthreads();
   const float n0 = m[1] * m[5] - m[2] * m[4], n1 = m[2] * m[3] - m[0] * m[5], n2 = m[0] * m[4] - m[1] * m[3];
   const float R2 = R * R * (1.f + 1e-5f) + 1e-3f;
-  const float lo_pad = below + widen + kSegMargin, hi_pad = (float)g.B + widen + kSegMargin;
+  const float lo_pad = widen + kSegMargin, hi_pad = (float)g.B + widen + kSegMargin;
   // The exact test of brick b: its widened box meets the slice's plane and
   // the sphere of radius R.
   auto crosses = [&](int b) {
@@ -340,7 +344,7 @@ segment_pairs_kernel(const float* __restrict__ mats, BrickGrid g, float pmax, fl
     for (int w = tid; w < nwords; w += kPairThreads) bits[w] = 0u;
     __syncthreads();
     const int nb[3] = {g.nbx, g.nby, g.nbz};
-    const float base[3] = {0.f, (float)g.ylo, (float)g.zlo};
+    const float base[3] = {(float)g.xlo, (float)g.ylo, (float)g.zlo};
     const float nv[3] = {n0, n1, n2};
     const int i = k == 0 ? 1 : 0, j = k == 2 ? 1 : 2;  // the other two axes
     const float d = 0.5f * (hi_pad - lo_pad), h = 0.5f * (hi_pad + lo_pad);
@@ -411,44 +415,68 @@ segment_pairs_kernel(const float* __restrict__ mats, BrickGrid g, float pmax, fl
   }
   __syncthreads();
   const int nh = s_n;
-  if (tid == 0) s_base = (long long)atomicAdd(counters + 1, (unsigned long long)nh);
+  // The row range of each side of each hit brick (the box as the brick
+  // kernels build it), walked twice: counted, so that the slice reserves its
+  // bins with one atomic, then written.
+  const SegRows sr = seg_rows_setup(m, zpx);
+  const float half = 0.5f * (float)g.B, hw = half + widen + kSegMargin;
+  int mine = 0, vlo[2], vhi[2];
+  for (int k = tid; k < nh; k += kPairThreads) {
+    const int3 o = brick_origin(g, hits[k]);
+    seg_rows(sr, zpx, o.x + half, o.y + half, o.z + half, hw, vlo, vhi);
+    mine += (vlo[0] <= vhi[0]) + (vlo[1] <= vhi[1]);
+  }
+  for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+  if (lane == 0 && mine) atomicAdd(&s_m, mine);
   __syncthreads();
-  if (s_base + nh > bins_cap) {  // out of room: direct path
-    for (long long k = s_base + tid; k < s_base + nh && k < bins_cap; k += kPairThreads) bins[k].brick = -1;
+  const int nm = s_m;
+  if (tid == 0) s_base = (long long)atomicAdd(counters + 1, (unsigned long long)nm);
+  __syncthreads();
+  if (s_base + nm > bins_cap) {  // out of room: direct path
+    for (long long k = s_base + tid; k < s_base + nm && k < bins_cap; k += kPairThreads) bins[k].key = -1;
     if (tid == 0) fallback[atomicAdd(nfallback, 1)] = slice;
     return;
   }
-  // Each pair carries the row range of its two sides (the brick's box as the
-  // brick kernels build it: widened by `below` on the low side, by the
-  // curvature's reach and the margin on all), so that the kernels neither
-  // recompute it per warp nor walk a side with no pixels.
   for (int k = tid; k < nh; k += kPairThreads) {
     const int local = hits[k];
     const int3 o = brick_origin(g, local);
-    int rows[2];
-#pragma unroll
-    for (int side = 0; side < 2; side++) {
-      const SegBox box = seg_box(m, side, o, g.B, below, widen);
-      int vlo, vhi;
-      rows[side] = seg_rows(box, zpx, vlo, vhi) ? seg_pack_rows(vlo, vhi) : kSegNoRows;
-    }
+    seg_rows(sr, zpx, o.x + half, o.y + half, o.z + half, hw, vlo, vhi);
     const int b = vol * g.nbricks + local;
-    bins[s_base + k] = {slice, rows[0], rows[1], b, 0, 0, 0, 0};
-    atomicAdd(brick_pairs + b, 1);
+#pragma unroll
+    for (int side = 0; side < 2; side++)
+      if (vlo[side] <= vhi[side])
+        reinterpret_cast<int4*>(bins)[s_base + atomicAdd(&s_put, 1)] = make_int4(
+            2 * slice + side, seg_pack_rows(vlo[side], vhi[side]), b, atomicAdd(brick_pairs + b, 1));
+  }
+}
+
+// Writes the records of a segment plan, grouped by key: bin i goes to its
+// rank within its key.
+__global__ void segment_fill_kernel(const SegBin* __restrict__ bins, const float* __restrict__ mats,
+                                    const unsigned long long* __restrict__ counters, int64_t bins_cap,
+                                    const int* __restrict__ offsets, int negate, SegRec* __restrict__ recs) {
+  const int64_t nb = (int64_t)min(counters[1], (unsigned long long)bins_cap);
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += (int64_t)gridDim.x * blockDim.x) {
+    const int4 bn = __ldg(reinterpret_cast<const int4*>(bins) + i);
+    if (bn.z < 0) continue;  // reserved by a slice that fell back
+    const float* m = mats + 9 * (int64_t)(bn.x >> 1);
+    const float sg = negate && (bn.x & 1) ? -1.f : 1.f;
+    float4* r = reinterpret_cast<float4*>(recs + __ldg(offsets + bn.z) + bn.w);
+    r[0] = make_float4(sg * __ldg(m), sg * __ldg(m + 1), sg * __ldg(m + 2), sg * __ldg(m + 3));
+    r[1] = make_float4(sg * __ldg(m + 4), sg * __ldg(m + 5), __int_as_float(bn.x), __int_as_float(bn.y));
   }
 }
 
 // Single block.  Bricks are visited in `order` (increasing distance from the
-// origin); writes bin-list offsets, per-brick item offsets and the item count.
+// origin); writes the bin-list offsets, the work items and their count.
 constexpr int kScanThreads = 1024;
 __global__ void __launch_bounds__(kScanThreads)
 pairs_scan_kernel(const int* __restrict__ counts, const int* __restrict__ order, int nbricks, int nvol, int chunk,
-                  int* __restrict__ offsets, int* __restrict__ item_off, int* __restrict__ cursor,
+                  int* __restrict__ offsets, BrickItem* __restrict__ items, int* __restrict__ cursor,
                   int* __restrict__ nitems) {
-  __shared__ int s_c[kScanThreads], s_i[kScanThreads];
-  __shared__ int carry_c, carry_i;
-  if (threadIdx.x == 0) carry_c = carry_i = 0;
-  __syncthreads();
+  __shared__ int s_c[kScanThreads / 32], s_i[kScanThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int carry_c = 0, carry_i = 0;
   // keys volume * nbricks + brick, the volumes interleaved brick by brick so
   // that every volume's central bricks start first
   const int nkeys = nbricks * nvol;
@@ -457,28 +485,41 @@ pairs_scan_kernel(const int* __restrict__ counts, const int* __restrict__ order,
     int b = t < nkeys ? (t % nvol) * nbricks + order[t / nvol] : -1;
     int c = b >= 0 ? counts[b] : 0;
     int ni = (c + chunk - 1) / chunk;
-    s_c[threadIdx.x] = c;
-    s_i[threadIdx.x] = ni;
-    __syncthreads();
-    for (int o = 1; o < kScanThreads; o <<= 1) {  // inclusive Hillis-Steele scan
-      int vc = threadIdx.x >= o ? s_c[threadIdx.x - o] : 0;
-      int vi = threadIdx.x >= o ? s_i[threadIdx.x - o] : 0;
-      __syncthreads();
-      s_c[threadIdx.x] += vc;
-      s_i[threadIdx.x] += vi;
-      __syncthreads();
+    int ic = c, ii = ni;  // inclusive sums: within the warp, then over the warps
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int vc = __shfl_up_sync(0xffffffffu, ic, o), vi = __shfl_up_sync(0xffffffffu, ii, o);
+      if (lane >= o) {
+        ic += vc;
+        ii += vi;
+      }
     }
+    if (lane == 31) {
+      s_c[warp] = ic;
+      s_i[warp] = ii;
+    }
+    __syncthreads();
+    int wc = s_c[lane], wi = s_i[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int vc = __shfl_up_sync(0xffffffffu, wc, o), vi = __shfl_up_sync(0xffffffffu, wi, o);
+      if (lane >= o) {
+        wc += vc;
+        wi += vi;
+      }
+    }
+    const int pc = __shfl_sync(0xffffffffu, wc, (warp + 31) & 31), pi = __shfl_sync(0xffffffffu, wi, (warp + 31) & 31);
+    const int off = carry_c + (warp ? pc : 0) + ic - c, ioff = carry_i + (warp ? pi : 0) + ii - ni;
     if (b >= 0) {
-      offsets[b] = carry_c + s_c[threadIdx.x] - c;
-      item_off[b] = carry_i + s_i[threadIdx.x] - ni;
+      offsets[b] = off;
       cursor[b] = 0;
+      const int size = ni ? (c + ni - 1) / ni : 0;  // equal shares
+      for (int k = 0; k < ni; k++)
+        items[ioff + k] = {b, off + k * size, min(size, c - k * size), ni == 1 ? 1 : 0};
     }
-    __syncthreads();
-    if (threadIdx.x == kScanThreads - 1) {
-      carry_c += s_c[threadIdx.x];
-      carry_i += s_i[threadIdx.x];
-    }
-    __syncthreads();
+    carry_c += __shfl_sync(0xffffffffu, wc, 31);
+    carry_i += __shfl_sync(0xffffffffu, wi, 31);
+    __syncthreads();  // the sums are read before the next round writes them
   }
   if (threadIdx.x == 0) *nitems = carry_i;
 }
@@ -497,18 +538,6 @@ __global__ void pairs_fill_kernel(const PixelBin* __restrict__ bins,
     int s = atomicAdd(cursor + b, 1);
     if (s < counts[b]) pairs[offsets[b] + s] = (int)i;
   }
-}
-
-__global__ void plan_items_kernel(const int* __restrict__ counts, const int* __restrict__ offsets,
-                                  const int* __restrict__ item_off, int nbricks, int chunk,
-                                  BrickItem* __restrict__ items) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nbricks) return;
-  int c = counts[b];
-  if (!c) return;
-  int nch = (c + chunk - 1) / chunk;
-  for (int k = 0; k < nch; k++)
-    items[item_off[b] + k] = {b, offsets[b] + k * chunk, min(chunk, c - k * chunk), nch == 1 ? 1 : 0};
 }
 
 // Brick visiting order per grid, cached per device and context.
@@ -534,7 +563,7 @@ static int brick_order(const BrickGrid& g, const int** out) {
   int dev = 0;
   GTOMRLN_CUDA_TRY(cudaGetDevice(&dev));
   const unsigned long long ctx = context_id();
-  auto key = std::make_tuple(dev, ctx, g.V, g.B, g.nbx, g.nby, g.ylo);
+  auto key = std::make_tuple(dev, ctx, g.V, g.B, g.nbx * 2 + (g.xlo ? 1 : 0), g.nby, g.ylo);
   std::lock_guard<std::mutex> lock(g_order_mutex);
   auto it = g_orders.find(key);
   if (it != g_orders.end()) {
@@ -593,16 +622,32 @@ int build_brick_plan(int op, const float* d_mats, int batch, const BrickGrid& g,
   }
   int64_t entries_cap =
       segments ? 1 : std::max<int64_t>(1, (int64_t)batch * npix * (op == GTOMRLN_OP_PROJECT ? 1 : 2));
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   int per_slice = std::min(g.nbricks, kMaxBinsPerSlice);
   if (segments) {
     // A crossed brick's centre lies within h = sqrt(3)/2 * B' (B' the widened
     // edge) of the plane and within limit + h of the origin: about
-    // pi (limit + h)^2 * 2h / B^3 lattice points per slice; half as much
-    // again is reserved (the cap is an average over the batch).
-    const double Bw = g.B + (op == GTOMRLN_OP_PROJECT ? 0.0 : 1.0) + 2.0 * kSegMargin;
+    // pi (limit + h)^2 * 2h / B^3 lattice points per slice, of which about
+    // half hold rows on one side and a few on both; half as much again is
+    // reserved (the cap is an average over the batch).
+    const double Bw = g.B + 2.0 * kSegMargin;
     const double h = 0.8660254037844386 * Bw, R = (double)limit + h;
     const double est = 3.141592653589793 * R * R * 2.0 * h / ((double)g.B * g.B * g.B);
-    per_slice = (int)std::min<double>(g.nbricks, 1.5 * est + 64.0);
+    per_slice = (int)std::min<double>(2.0 * g.nbricks, 1.5 * est + 64.0);
+    // Work items of at most an eighth of an SM's share of the records (about
+    // 0.4 est per slice; a shared brick is staged, or flushed, once more per
+    // item, which costs as much as a few dozen records): with larger ones the
+    // central bricks, which every slice crosses, keep single CTAs busy after
+    // the others have finished.  The backprojector's are not cut below 512,
+    // where its extra flushes by reductions cost more than they even out, and
+    // on volumes that only a forced path brings here items stay whole.
+    const double share = 0.4 * est * batch / (8.0 * sms);
+    if (op == GTOMRLN_OP_PROJECT)
+      chunk = (int)std::min<double>(chunk, std::max(128.0, share));
+    else if (g.V >= 256)
+      chunk = (int)std::min<double>(chunk, std::max(512.0, share));
   }
   int64_t bins_cap = std::max<int64_t>(1, (int64_t)batch * per_slice);
   if (entries_cap > 0x7fffffffLL || bins_cap > 0x7fffffffLL)
@@ -614,14 +659,13 @@ int build_brick_plan(int op, const float* d_mats, int batch, const BrickGrid& g,
   size_t nb = (size_t)nkeys;
   size_t o_counts = 0;
   size_t o_offsets = o_counts + al(nb * 4);
-  size_t o_itemoff = o_offsets + al(nb * 4);
-  size_t o_cursor = o_itemoff + al(nb * 4);
+  size_t o_cursor = o_offsets + al(nb * 4);
   size_t o_misc = o_cursor + al(nb * 4);  // counters (2 x u64), work counter, nitems, nfallback
   size_t o_fallback = o_misc + 256;
   size_t o_items = o_fallback + al((size_t)std::max(batch, 1) * 4);
   size_t o_bins = o_items + al((size_t)cap_items * sizeof(BrickItem));
-  size_t o_pairs = o_bins + al((size_t)bins_cap * sizeof(PixelBin));
-  size_t o_entries = o_pairs + al((size_t)bins_cap * 4);
+  size_t o_pairs = o_bins + al((size_t)bins_cap * (segments ? sizeof(SegBin) : sizeof(PixelBin)));
+  size_t o_entries = o_pairs + al((size_t)bins_cap * (segments ? sizeof(SegRec) : 4));
   size_t bytes = o_entries + al((size_t)entries_cap * 4);
   char* base = nullptr;
   st = scratch_alloc((void**)&base, bytes, stream);
@@ -629,7 +673,6 @@ int build_brick_plan(int op, const float* d_mats, int batch, const BrickGrid& g,
   plan->scratch = base;
   int* counts = (int*)(base + o_counts);
   int* offsets = (int*)(base + o_offsets);
-  int* item_off = (int*)(base + o_itemoff);
   int* cursor = (int*)(base + o_cursor);
   unsigned long long* counters = (unsigned long long*)(base + o_misc);
   plan->counter = (int*)(base + o_misc + 16);
@@ -637,8 +680,13 @@ int build_brick_plan(int op, const float* d_mats, int batch, const BrickGrid& g,
   plan->nfallback = (int*)(base + o_misc + 24);
   plan->fallback = (int*)(base + o_fallback);
   plan->items = (BrickItem*)(base + o_items);
-  plan->bins = (PixelBin*)(base + o_bins);
-  plan->pairs = (int*)(base + o_pairs);
+  SegBin* seg_bins = (SegBin*)(base + o_bins);
+  if (segments) {
+    plan->recs = (SegRec*)(base + o_pairs);
+  } else {
+    plan->bins = (PixelBin*)(base + o_bins);
+    plan->pairs = (int*)(base + o_pairs);
+  }
   plan->entries = (int*)(base + o_entries);
   plan->max_items = (int)std::min<int64_t>(cap_items, 0x7fffffff);
 
@@ -646,12 +694,9 @@ int build_brick_plan(int op, const float* d_mats, int batch, const BrickGrid& g,
   if (e == cudaSuccess) e = cudaMemsetAsync(base + o_misc, 0, 256, stream);
   if (e == cudaSuccess && batch > 0) {
     if (segments) {
-      // The projector's samples reach the brick of their base voxel, the
-      // backprojector's also the bricks of the voxel above it on each axis.
-      const float below = op == GTOMRLN_OP_PROJECT ? 0.f : 1.f;
       cudaFuncSetAttribute(segment_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
       segment_pairs_kernel<<<batch, kPairThreads, smem_bytes, stream>>>(
-          d_mats, g, px.pmax, limit, below, plan->bins, bins_cap, counters, counts, plan->fallback,
+          d_mats, g, px.pmax, limit, seg_bins, bins_cap, counters, counts, plan->fallback,
           plan->nfallback, (float2*)zero_out, px, geom);
     } else if (op == GTOMRLN_OP_PROJECT) {
       cudaFuncSetAttribute(bin_slices_kernel<GTOMRLN_OP_PROJECT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -667,14 +712,13 @@ int build_brick_plan(int op, const float* d_mats, int batch, const BrickGrid& g,
           plan->fallback, plan->nfallback, use_codes);
     }
     pairs_scan_kernel<<<1, kScanThreads, 0, stream>>>(counts, d_order, g.nbricks, geom.nvol, chunk, offsets,
-                                                      item_off, cursor, plan->nitems);
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    pairs_fill_kernel<<<sms * 4, 256, 0, stream>>>(plan->bins, counters, bins_cap, counts, offsets, cursor,
-                                                   plan->pairs);
-    plan_items_kernel<<<(int)((nkeys + 255) / 256), 256, 0, stream>>>(counts, offsets, item_off, (int)nkeys, chunk,
-                                                                      plan->items);
+                                                      plan->items, cursor, plan->nitems);
+    if (segments)
+      segment_fill_kernel<<<sms * 8, 256, 0, stream>>>(seg_bins, d_mats, counters, bins_cap, offsets, geom.negate,
+                                                       plan->recs);
+    else
+      pairs_fill_kernel<<<sms * 4, 256, 0, stream>>>(plan->bins, counters, bins_cap, counts, offsets, cursor,
+                                                     plan->pairs);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) {

@@ -235,23 +235,47 @@ project_brick_kernel(const float2* __restrict__ vol, float2* __restrict__ proj,
 }
 
 // Segment variant of the brick projector: the same staging and arithmetic,
-// but a warp takes a (slice, brick) pair of the segment plan and finds the
-// pixels itself, by row segments (segment.cuh), among those whose position
-// (side 0) or mirrored position (side 1) falls in the brick.  A pixel is
-// written by the pair whose brick holds its base voxel, on the side of its
-// Friedel flip: exactly one pair, as in the binned variant.  Post turns the
-// interpolated value into the stored one (identity, or the phase shift and
-// weight of d_rlnProjectShifted), as in the direct kernel.
-template <class Post = NoPost>
+// but the warps take records of the segment plan and find the pixels
+// themselves (seg_deal), among those whose position (side 0) or mirrored
+// position (side 1) falls in the brick.  A pixel is written by the record
+// whose brick holds its base voxel, on the side of its Friedel flip: exactly
+// one, as in the binned variant.  The records' columns are negated on side
+// 1, so the flipped position comes out directly (negation is exact).  Post
+// turns the interpolated value into the stored one (identity, or the phase
+// shift and weight of d_rlnProjectShifted), as in the direct kernel.  EDGE:
+// the brick edge at compile time (the corner offsets become immediates), or
+// 0 for the run-time value.  The staged rows and planes are padded
+// (proj_pitch): a model of the corner loads (lanes stepping two voxels along
+// any direction) puts a half-warp's 8-byte load at 2.73 wavefronts instead
+// of 2.95.
+constexpr int kProjEdge = 29;  // the default brick edge (abi.cu), known to the kernel at compile time
+struct ProjPitch {
+  int row, plane;  // in float2
+};
+__host__ __device__ constexpr ProjPitch proj_pitch(int edge) {
+  return edge == kProjEdge ? ProjPitch{31, 934} : ProjPitch{edge + 1, (edge + 1) * (edge + 1)};
+}
+
+// An asynchronous 8-byte copy global -> shared.
+__device__ __forceinline__ void copy_async8(float2* dst, const float2* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <int EDGE, class Post = NoPost>
 __global__ void __launch_bounds__(1024)
-project_segment_kernel(const float2* __restrict__ vol, float2* __restrict__ proj,
-                       const float* __restrict__ mats, ProjArgs a, BrickGrid g, PixelSet px,
+project_segment_kernel(const float2* __restrict__ vol, float2* __restrict__ proj, ProjArgs a, BrickGrid g, PixelSet px,
                        const BrickItem* __restrict__ items, const int* __restrict__ nitems_ptr,
-                       const int* __restrict__ pairs, const PixelBin* __restrict__ bins, int* __restrict__ counter, Post post = Post()) {
-  extern __shared__ float2 tile[];
+                       const SegRec* __restrict__ recs, int* __restrict__ counter, Post post = Post()) {
+  extern __shared__ float4 smem4[];  // record slots, then the brick
   __shared__ int item_s, next_s;
   const int nitems = *nitems_ptr;
-  const int B = g.B, T = g.B + 1;
+  const int B = EDGE ? EDGE : g.B, T = B + 1;
+  const ProjPitch pitch = proj_pitch(EDGE);
+  const int RS = EDGE ? pitch.row : T, PS = EDGE ? pitch.plane : T * T;
+  SegRec* stage = reinterpret_cast<SegRec*>(smem4);
+  float2* tile = reinterpret_cast<float2*>(stage + kSegChunk * (blockDim.x >> 5));
   const int rowlen = a.P / 2 + 1;
   const int64_t last = a.nvox - 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -266,7 +290,8 @@ project_segment_kernel(const float2* __restrict__ vol, float2* __restrict__ proj
     if (w >= nitems) break;
     const BrickItem it = items[w];
     const int3 o = brick_origin(g, it.brick);
-    // stage the brick and its halo, one warp per (y, z) row, lanes along x
+    // stage the brick and its halo, one warp per (y, z) row, lanes along x,
+    // every copy in flight at once
     for (int r = warp; r < T * T; r += nwarps) {
       const int ty = r % T, tz = r / T;
       const int y = o.y + ty, z = o.z + tz;
@@ -275,50 +300,45 @@ project_segment_kernel(const float2* __restrict__ vol, float2* __restrict__ proj
       for (int tx = lane; tx < T; tx += 32) {
         int64_t i = row + tx;
         i = i < 0 ? 0 : (i > last ? last : i);
-        tile[r * T + tx] = __ldg(vol + i);
+        copy_async8(tile + tz * PS + ty * RS + tx, vol + i);
       }
     }
+    copy_async_wait();
     __syncthreads();
-    // warps take the item's pairs one at a time, the next one's slice
-    // fetched before the current one is processed
-    auto take = [&]() {
-      int j = 0;
-      if (lane == 0) j = atomicAdd(&next_s, 1);
-      return __shfl_sync(0xffffffffu, j, 0);
-    };
-    int j = take();
-    int4 pr = j < it.count ? seg_pair(bins, pairs, it.offset + j) : make_int4(0, kSegNoRows, kSegNoRows, 0);
-    while (j < it.count) {
-      const int jn = take();
-      const int4 nx = jn < it.count ? seg_pair(bins, pairs, it.offset + jn) : make_int4(0, kSegNoRows, kSegNoRows, 0);
-      const int slice = pr.x;
-      float m[9];
-#pragma unroll
-      for (int k = 0; k < 9; k++) m[k] = __ldg(mats + 9 * (int64_t)slice + k);
-      float2* out = proj + a.elements * slice;
-#pragma unroll 1
-      for (int side = 0; side < 2; side++) {
-        int vlo, vhi;
-        seg_unpack_rows(side ? pr.z : pr.y, vlo, vhi);
-        if (vlo > vhi) continue;  // no pixel of this side
-        const SegBox box = seg_box(m, side, o, B, 0.f);
-        seg_for_each_pixel_rows(box, px, vlo, vhi, [&](int u, int v, bool valid) {
-          if (!valid) return;
-          ProjSample s = project_sample(m, u, v, 0);
-          if ((s.sign < 0.f) != (side == 1)) return;  // the other side's pixel
-          int lx = s.x0 - o.x, ly = s.y0 - o.y, lz = s.z0 - o.z;
-          if ((unsigned)lx >= (unsigned)B || (unsigned)ly >= (unsigned)B || (unsigned)lz >= (unsigned)B)
-            return;  // another brick's pixel
-          const float2* c = tile + (lz * T + ly) * T + lx;
-          const int idy = v < 0 ? v + a.n : v;
-          const float2 val = trilerp(s, c[0], c[1], c[T], c[T + 1], c[T * T], c[T * T + 1], c[T * T + T],
-                                     c[T * T + T + 1]);
-          out[(int64_t)idy * a.dimft + u] = post.template apply<2>(slice, u, v, 0, val);
-        });
-      }
-      j = jn;
-      pr = nx;
-    }
+    seg_for_each_chunk(recs + it.offset, it.count, stage, &next_s, [&](const SegRec* rec, int rows) {
+      seg_deal(
+          rows,
+          [&](int p, int v, int& ua, int& ub) {
+            const SegWords r = seg_load(rec + p);
+            SegBox box = {{r.a.x, r.a.y, r.a.z}, {r.a.w, r.b.x, r.b.y}, {}, {}};
+            seg_box_bounds(box, o, B, 0.f);
+            seg_row(box, px, v, ua, ub);
+          },
+          [&](int p, int u, int v, bool valid) {
+            if (!valid) return;
+            const SegWords r = seg_load(rec + p);
+            const bool side = r.ss() & 1;
+            const float fu = (float)u, fv = (float)v;
+            // project_sample with the flip taken by the record
+            const float qx = fmaf(r.a.x, fu, r.a.w * fv), qy = fmaf(r.a.y, fu, r.b.x * fv),
+                        qz = fmaf(r.a.z, fu, r.b.y * fv);
+            if (side ? !(qx > 1e-5f) : qx < -1e-5f) return;  // the other side's pixel
+            const float fx0 = floorf(qx + 1e-5f), fy0 = floorf(qy), fz0 = floorf(qz);
+            ProjSample s;
+            s.fx = qx - fx0;
+            s.fy = qy - fy0;
+            s.fz = qz - fz0;
+            s.sign = side ? -1.f : 1.f;
+            const int lx = (int)fx0 - o.x, ly = (int)fy0 - o.y, lz = (int)fz0 - o.z;
+            if ((unsigned)lx >= (unsigned)B || (unsigned)ly >= (unsigned)B || (unsigned)lz >= (unsigned)B)
+              return;  // another brick's pixel
+            const float2* c = tile + lz * PS + ly * RS + lx;
+            const int slice = r.ss() >> 1;
+            const float2 val = trilerp(s, c[0], c[1], c[RS], c[RS + 1], c[PS], c[PS + 1], c[PS + RS], c[PS + RS + 1]);
+            proj[a.elements * slice + ((v < 0 ? v + a.n : v) * a.dimft + u)] =
+                post.template apply<2>(slice, u, v, 0, val);
+          });
+    });
   }
 }
 
@@ -357,8 +377,10 @@ static int project_brick(const float* d_volumeft, float* d_proj, const float* d_
   // While every sample radius stays below P/2 + 0.99, the base voxels lie in
   // x [0, P/2] and y, z [-P/2 - 1, P/2].
   BrickGrid g = make_brick_grid(P, tune.edge, P / 2, -(P / 2) - 1, P / 2);
-  size_t smem = sizeof(float2) * (size_t)(tune.edge + 1) * (tune.edge + 1) * (tune.edge + 1);
-  auto kern = project_segment_kernel<Post>;
+  const size_t smem = segments ? sizeof(float2) * (size_t)(tune.edge + 1) * proj_pitch(tune.edge).plane +
+                                     seg_stage_bytes(tune.threads)
+                               : sizeof(float2) * (size_t)(tune.edge + 1) * (tune.edge + 1) * (tune.edge + 1);
+  auto kern = tune.edge == kProjEdge ? project_segment_kernel<kProjEdge, Post> : project_segment_kernel<0, Post>;
   cudaError_t e = segments ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
                            : cudaFuncSetAttribute(project_brick_kernel,
                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -382,8 +404,10 @@ static int project_brick(const float* d_volumeft, float* d_proj, const float* d_
   BrickPlan plan;
   // the segment plan writes the zeros outside rmax of the slices it plans
   // (the direct kernel those of the slices it leaves over)
+  SliceGeom geom;
+  geom.negate = 1;
   int st = build_brick_plan(GTOMRLN_OP_PROJECT, d_mats, (int)batch, g, px, (float)(P / 2) + 0.99f, tune.chunk,
-                            stream, &plan, segments, segments ? d_proj : nullptr);
+                            stream, &plan, segments, segments ? d_proj : nullptr, geom);
   if (st) return st;
   if (!segments) {
     int64_t rows = (int64_t)a.n * batch;  // 2D slices: n rows of dimft elements each
@@ -391,8 +415,8 @@ static int project_brick(const float* d_volumeft, float* d_proj, const float* d_
   }
   if (segments)
     kern<<<sms * std::max(occ, 1), tune.threads, smem, stream>>>(
-        (const float2*)d_volumeft, (float2*)d_proj, d_mats, a, g, px, plan.items, plan.nitems, plan.pairs,
-        plan.bins, plan.counter, post);
+        (const float2*)d_volumeft, (float2*)d_proj, a, g, px, plan.items, plan.nitems, plan.recs, plan.counter,
+        post);
   else
     project_brick_kernel<<<sms * std::max(occ, 1), tune.threads, smem, stream>>>(
         (const float2*)d_volumeft, (float2*)d_proj, d_mats, a, g, plan.items, plan.nitems, plan.pairs, plan.bins,

@@ -7,10 +7,9 @@
 //   lo_r <= u * c0_r + v * c1_r <= hi_r,
 // and the rows that can hold such a pixel lie between the extremes over the
 // box of the linear function v(p) that recovers v from a point of the plane.
-// A warp walks one (slice, box) pair: 32 rows at a time, one lane per row
-// computes the row's u interval (clipped to the slice's pixel set), the
-// lanes scan the interval lengths, and the pixels are dealt out 32 per wave,
-// each lane finding its row by a binary search over the scan.  The boxes
+// The plan (brick_plan.cu) stores one record per (slice, side, brick) with
+// such rows; a warp takes a few records of its brick at a time and deals
+// their rows out to its lanes, then the rows' pixels (seg_deal).  The boxes
 // are widened by a margin well above the float error of both the positions
 // and these bounds, so the candidates are a superset of the pixels the box
 // holds; the caller applies the exact test with the kernels' own
@@ -26,22 +25,24 @@ namespace gtomrln {
 // interval bounds below (relative 1e-6 of the same magnitudes).
 constexpr float kSegMargin = 0.01f;
 
-// The box and the pixel -> position map of one (slice, brick, side): the
-// columns are read from the slice matrix (negated for the mirror side) and
-// the box from the brick origin when needed, so that nothing beyond the
-// matrix and the origin stays live in registers.
+// A box and the pixel -> position map of one (slice, side): c0, c1 the
+// matrix columns (negated for the mirror side).
 struct SegBox {
-  const float* m;  // slice matrix (9 floats, column-major)
-  float sg;        // +1: positions; -1: negated positions
-  int3 o;          // brick origin
-  float below;     // widening below the brick, before the margin
-  float above;     // brick edge plus the margin
-  __device__ __forceinline__ float c0(int r) const { return sg * m[r]; }
-  __device__ __forceinline__ float c1(int r) const { return sg * m[3 + r]; }
-  __device__ __forceinline__ float org(int r) const { return (float)(r == 0 ? o.x : (r == 1 ? o.y : o.z)); }
-  __device__ __forceinline__ float lo(int r) const { return org(r) - below; }
-  __device__ __forceinline__ float hi(int r) const { return org(r) + above; }
+  float c0[3], c1[3], lo[3], hi[3];
 };
+
+// The box of brick origin o, edge B, widened by `widen` (a bound on how far
+// samples leave the flat map, e.g. by the Ewald curvature) and the margin.
+__device__ __forceinline__ void seg_box_bounds(SegBox& b, int3 o, int B, float widen) {
+  const float w = widen + kSegMargin;
+  b.lo[0] = (float)o.x - w;
+  b.lo[1] = (float)o.y - w;
+  b.lo[2] = (float)o.z - w;
+  const float e = (float)B + w;
+  b.hi[0] = (float)o.x + e;
+  b.hi[1] = (float)o.y + e;
+  b.hi[2] = (float)o.z + e;
+}
 
 // Largest u with u^2 <= rem (0 <= rem < 2^24: radii below 4 096), exactly:
 // the approximate square root is within a unit of the truth there, which the
@@ -62,41 +63,62 @@ __device__ __forceinline__ float seg_rcp(float a) {
   return r;
 }
 
-// Row range [vlo, vhi] (signed v) that can hold a pixel of the box, clipped
-// to the slice rows within the pixel set's radius.  Returns false if empty.
-__device__ __forceinline__ bool seg_rows(const SegBox& b, const PixelSet& px, int& vlo, int& vhi) {
+// The linear functions of a slice that bound its rows in a box: on the plane
+// v(p) = w . p and u(p) = w' . p, w = (g00 c1 - g01 c0) / det, w' =
+// (g11 c0 - g01 c1) / det, whose extremes over the box bound the rows and
+// reject a box that lies wholly at u < 0 (the other side's pixels).
+// Near-parallel columns (det small against g00 g11) keep the full range;
+// well-conditioned ones (det above a quarter of g00 g11: an error of a few
+// 1e-6 of the magnitudes) need little padding.
+struct SegRows {
+  float wv[3], wu[3];  // w and w'
+  float av, au;        // sums of their magnitudes
+  float pad0, padr;    // padding: absolute, and relative to the magnitudes
+  int vmin, vmax;      // the slice's rows within the pixel set's radius
+  bool plane;          // whether w, w' exist
+};
+__device__ __forceinline__ SegRows seg_rows_setup(const float* m, const PixelSet& px) {
+  SegRows s;
   const int rlim = seg_isqrt(px.strict ? px.rmax2 - 1 : px.rmax2);
-  vlo = max(px.n / 2 + 1 - px.n, -rlim);  // rows idy > n/2 hold v = idy - n
-  vhi = min(px.n / 2, rlim);
-  const float g00 = b.c0(0) * b.c0(0) + b.c0(1) * b.c0(1) + b.c0(2) * b.c0(2);
-  const float g11 = b.c1(0) * b.c1(0) + b.c1(1) * b.c1(1) + b.c1(2) * b.c1(2);
-  const float g01 = b.c0(0) * b.c1(0) + b.c0(1) * b.c1(1) + b.c0(2) * b.c1(2);
+  s.vmin = max(px.n / 2 + 1 - px.n, -rlim);  // rows idy > n/2 hold v = idy - n
+  s.vmax = min(px.n / 2, rlim);
+  const float g00 = m[0] * m[0] + m[1] * m[1] + m[2] * m[2];
+  const float g11 = m[3] * m[3] + m[4] * m[4] + m[5] * m[5];
+  const float g01 = m[0] * m[3] + m[1] * m[4] + m[2] * m[5];
   const float det = g00 * g11 - g01 * g01;
-  // v(p) = w . p and u(p) = w' . p on the plane, w = (g00 c1 - g01 c0) / det,
-  // w' = (g11 c0 - g01 c1) / det: their extremes over the box bound the rows
-  // and reject a box that lies wholly at u < 0 (the other side's pixels).
-  // Near-parallel columns (det small against g00 g11) keep the full range.
-  if (det > 1e-3f * g00 * g11 && g00 > 0.f) {
-    const float inv = 1.f / det;
-    float vc = 0.f, vh = 0.f, uc = 0.f, uh = 0.f;
+  s.plane = det > 1e-3f * g00 * g11 && g00 > 0.f;
+  const bool well = det > 0.25f * g00 * g11;
+  s.pad0 = well ? 0.02f : 0.5f;
+  s.padr = well ? 1e-4f : 1e-3f;
+  const float inv = 1.f / det;
+  s.av = s.au = 0.f;
 #pragma unroll
-    for (int r = 0; r < 3; r++) {
-      const float w = (g00 * b.c1(r) - g01 * b.c0(r)) * inv;
-      const float wu = (g11 * b.c0(r) - g01 * b.c1(r)) * inv;
-      const float c = 0.5f * (b.lo(r) + b.hi(r)), h = 0.5f * (b.hi(r) - b.lo(r));
-      vc = fmaf(w, c, vc);
-      vh = fmaf(fabsf(w), h, vh);
-      uc = fmaf(wu, c, uc);
-      uh = fmaf(fabsf(wu), h, uh);
-    }
-    const float upad = 0.5f + 1e-3f * (fabsf(uc) + uh);
-    if (uc + uh + upad < 0.f || uc - uh - upad > (float)(px.dimft - 1)) return false;
-    const float pad = 0.5f + 1e-3f * (fabsf(vc) + vh);
-    const float flo = fmaxf(vc - vh - pad, -1e6f), fhi = fminf(vc + vh + pad, 1e6f);
-    vlo = max(vlo, (int)floorf(flo));
-    vhi = min(vhi, (int)ceilf(fhi));
+  for (int r = 0; r < 3; r++) {
+    s.wv[r] = (g00 * m[3 + r] - g01 * m[r]) * inv;
+    s.wu[r] = (g11 * m[r] - g01 * m[3 + r]) * inv;
+    s.av += fabsf(s.wv[r]);
+    s.au += fabsf(s.wu[r]);
   }
-  return vlo <= vhi;
+  return s;
+}
+// Row ranges of side 0 and side 1 (mirrored: the functions negated) in the
+// cube of centre (cx, cy, cz) and half edge h; empty as vlo > vhi.
+__device__ __forceinline__ void seg_rows(const SegRows& s, const PixelSet& px, float cx, float cy, float cz, float h,
+                                         int vlo[2], int vhi[2]) {
+  const float vc = s.wv[0] * cx + s.wv[1] * cy + s.wv[2] * cz, uc = s.wu[0] * cx + s.wu[1] * cy + s.wu[2] * cz;
+  const float vh = s.av * h, uh = s.au * h;
+  const float pu = uh + s.pad0 + s.padr * (fabsf(uc) + uh), pv = vh + s.pad0 + s.padr * (fabsf(vc) + vh);
+#pragma unroll
+  for (int side = 0; side < 2; side++) {
+    const float u = side ? -uc : uc, v = side ? -vc : vc;
+    vlo[side] = s.vmin;
+    vhi[side] = s.vmax;
+    if (s.plane) {
+      vlo[side] = max(s.vmin, (int)ceilf(fmaxf(v - pv, -1e6f)));
+      vhi[side] = min(s.vmax, (int)floorf(fminf(v + pv, 1e6f)));
+      if (u + pu < 0.f || u - pu > (float)(px.dimft - 1)) vhi[side] = vlo[side] - 1;
+    }
+  }
 }
 
 // Pixel interval [ua, ub] of row v holding the box, clipped to the pixel set
@@ -106,8 +128,8 @@ __device__ __forceinline__ void seg_row(const SegBox& b, const PixelSet& px, int
   float umin = -1.f, umax = (float)px.dimft;
 #pragma unroll
   for (int r = 0; r < 3; r++) {
-    const float a = b.c0(r), t = (float)v * b.c1(r);
-    const float l = b.lo(r) - t, h = b.hi(r) - t;
+    const float a = b.c0[r], t = (float)v * b.c1[r];
+    const float l = b.lo[r] - t, h = b.hi[r] - t;
     // |a| <= 1e-20 moves a * u by < 1e-16 over the row: a u-free test, which
     // the margin keeps conservative (and 1 / a stays finite otherwise)
     if (fabsf(a) > 1e-20f) {
@@ -130,83 +152,151 @@ __device__ __forceinline__ void seg_row(const SegBox& b, const PixelSet& px, int
   ub = min((int)floorf(umax), min(seg_isqrt(rem), px.dimft - 1));
 }
 
-// Row range of a (slice, brick, side) as the plan stores it: vlo in the low
-// and vhi in the high 16 bits; an empty side as vlo = 1, vhi = 0.
-__host__ __device__ __forceinline__ int seg_pack_rows(int vlo, int vhi) {
-  return (int)(((unsigned)vlo & 0xffffu) | ((unsigned)vhi << 16));
-}
-__device__ __forceinline__ void seg_unpack_rows(int packed, int& vlo, int& vhi) {
-  vlo = (int)(short)(packed & 0xffff);
-  vhi = packed >> 16;
-}
-constexpr int kSegNoRows = (int)(1u | (0u << 16));
+// One (slice, side, brick) of a segment plan, grouped by brick: the slice
+// matrix's first two columns (negated on side 1 where the plan's geometry
+// asks for it), the slice and side, and the row range.
+struct __align__(32) SegRec {
+  float c0[3], c1[3];
+  int ss;    // 2 * slice + side
+  int rows;  // first row in the low 16 bits (signed), row count above
+};
+static_assert(sizeof(SegRec) == 32, "SegRec is read as two 16-byte words");
 
-// A segment plan's pair k: (slice, packed rows of side 0, of side 1, brick).
-__device__ __forceinline__ int4 seg_pair(const PixelBin* __restrict__ bins, const int* __restrict__ pairs,
-                                         int k) {
-  return __ldg(reinterpret_cast<const int4*>(bins + __ldg(pairs + k)));
+// A record's two 16-byte words: {c0, c1.x} and {c1.y, c1.z, ss, rows}.
+struct SegWords {
+  float4 a, b;
+  __device__ __forceinline__ int ss() const { return __float_as_int(b.z); }
+};
+__device__ __forceinline__ SegWords seg_load(const SegRec* rec) {  // from shared memory
+  const float4* p = reinterpret_cast<const float4*>(rec);
+  SegWords w;
+  w.a = p[0];
+  w.b = p[1];
+  return w;
 }
 
-// Calls f(u, v, valid) once per lane per wave of 32 candidate pixels of the
-// box in rows vlo .. vhi (from seg_rows; valid false on idle lanes of the
-// last wave).  Warp-synchronous: all 32 lanes must call it together with the
-// same box; f may use warp collectives.
-template <class F>
-__device__ __forceinline__ void seg_for_each_pixel_rows(const SegBox& b, const PixelSet& px, int vlo, int vhi,
-                                                        F&& f) {
+__device__ __forceinline__ int seg_pack_rows(int vlo, int vhi) {
+  return (int)(((unsigned)vlo & 0xffffu) | ((unsigned)(vhi - vlo + 1) << 16));
+}
+
+// Records a warp takes at a time.  A record has ~13 rows of ~8 pixels at
+// padding 2 (256^2 slices, 25..29-voxel bricks), so eight of them fill the
+// lanes of three to four row passes and the pixels of a pass seven waves.
+constexpr int kSegChunk = 8;
+
+// Deals the pixels of np <= kSegChunk consecutive records out to the warp:
+// their rows 32 at a time to the lanes, each lane bounding its row's pixel
+// interval (bounds(p, v, ua, ub): record p, row v), then the pixels of those
+// rows 32 per wave, f(p, u, v, valid) once per lane and wave (valid false on
+// idle lanes of a last wave, whose p stays a record of the chunk).  rows:
+// the record's packed rows on lane p, 0 on lanes >= np.  Taking one record
+// at a time instead left most row lanes and every record's last wave
+// part-filled and cost 380 instructions per 32 samples in the projector.
+// Warp-synchronous.
+template <class Bounds, class F>
+__device__ __forceinline__ void seg_deal(int rows, Bounds&& bounds, F&& f) {
+  constexpr unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  for (int vb = vlo; vb <= vhi; vb += 32) {
-    const int v = vb + lane;
-    int ua = 1, ub = 0;
-    if (v <= vhi) seg_row(b, px, v, ua, ub);
-    const int cnt = max(0, ub - ua + 1);
-    int incl = cnt;
+  const int nr = rows >> 16;
+  int incl = nr;
+#pragma unroll
+  for (int o = 1; o < kSegChunk; o <<= 1) {
+    const int t = __shfl_up_sync(full, incl, o);
+    if (lane >= o) incl += t;
+  }
+  const int total = __shfl_sync(full, incl, kSegChunk - 1);
+  const int vs = (int)(short)(rows & 0xffff) - (incl - nr);  // row k of the chunk is v = vs + k
+  const unsigned le = full >> (31 - lane);
+  for (int rb = 0; rb < total; rb += 32) {
+    const int k = rb + lane;
+    // record of row k: the number of records whose rows end at or before k
+    int p = 0;
+#pragma unroll
+    for (int step = kSegChunk / 2; step > 0; step >>= 1) {
+      const int t = __shfl_sync(full, incl, p + step - 1);
+      if (t <= k) p += step;
+    }
+    const int v = __shfl_sync(full, vs, p) + k;
+    int ua = 0, cnt = 0;
+    if (k < total) {
+      int ub;
+      bounds(p, v, ua, ub);
+      cnt = max(0, ub - ua + 1);
+    }
+    const unsigned nz = __ballot_sync(full, cnt > 0);
+    if (!nz) continue;
+    int inc2 = cnt;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
+      const int t = __shfl_up_sync(full, inc2, o);
+      if (lane >= o) inc2 += t;
     }
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    const int start = incl - cnt;
-    for (int base = 0; base < total; base += 32) {
-      const int k = base + lane;
-      // row of candidate k: the number of rows whose inclusive end is <= k
-      int r = 0;
+    const int tot = __shfl_sync(full, inc2, 31);
+    // the non-empty rows moved to the first lanes: lane i gets the row at
+    // the (i+1)-th set bit of nz
+    int r = 0;
 #pragma unroll
-      for (int step = 16; step > 0; step >>= 1) {
-        const int t = __shfl_sync(0xffffffffu, incl, r + step - 1);
-        if (t <= k) r += step;
-      }
-      const int rv = __shfl_sync(0xffffffffu, v, r & 31);
-      const int ra = __shfl_sync(0xffffffffu, ua, r & 31);
-      const int rs = __shfl_sync(0xffffffffu, start, r & 31);
-      const bool valid = k < total;
-      f(valid ? ra + (k - rs) : 0, valid ? rv : 0, valid);
+    for (int step = 16; step > 0; step >>= 1)
+      if (__popc(nz & ((1u << (r + step)) - 1u)) <= lane) r += step;
+    const int key = __shfl_sync(full, (p << 16) | (v & 0xffff), r);
+    const int st = __shfl_sync(full, inc2 - cnt, r);
+    const int off = __shfl_sync(full, ua, r) - st;
+    const int start = lane < __popc(nz) ? st : 0x7fffffff;
+    // wave by wave: the rows that start in the wave mark their first lane,
+    // and a lane's row is the last one started at or before it
+    int row0 = -1;
+    for (int base = 0; base < tot; base += 32) {
+      const unsigned d = (unsigned)(start - base);
+      const unsigned m = __reduce_or_sync(full, d < 32u ? 1u << d : 0u);
+      const int row = row0 + __popc(m & le);
+      row0 += __popc(m);
+      const int kk = __shfl_sync(full, key, row), ko = __shfl_sync(full, off, row);
+      const int q = base + lane;
+      f(kk >> 16, ko + q, (int)(short)(kk & 0xffff), q < tot);
     }
   }
 }
 
-// The same, finding the row range first.
-template <class F>
-__device__ __forceinline__ void seg_for_each_pixel(const SegBox& b, const PixelSet& px, F&& f) {
-  int vlo, vhi;
-  if (!seg_rows(b, px, vlo, vhi)) return;
-  seg_for_each_pixel_rows(b, px, vlo, vhi, f);
+// The warps of a CTA take the records of a work item a few at a time:
+// run(rec, rows) per chunk with the chunk's records in the warp's slots of
+// shared memory (stage: kSegChunk per warp, 16-byte aligned), the next chunk
+// fetched into registers before the current one is processed.  next_s: the
+// item's shared cursor, 0 at the start.  Small items are dealt in smaller
+// chunks, so that every warp gets several (an item's end waits for its last
+// warp).
+template <class Run>
+__device__ __forceinline__ void seg_for_each_chunk(const SegRec* __restrict__ recs, int count, SegRec* stage,
+                                                   int* next_s, Run&& run) {
+  const int lane = threadIdx.x & 31;
+  const int nwarps = blockDim.x >> 5;
+  const int step = count >= nwarps * kSegChunk * 4 ? kSegChunk : (count >= nwarps * 8 ? 4 : 2);
+  SegRec* slots = stage + (threadIdx.x >> 5) * kSegChunk;
+  auto take = [&]() {
+    int j = 0;
+    if (lane == 0) j = atomicAdd(next_s, step);
+    return __shfl_sync(0xffffffffu, j, 0);
+  };
+  // lane l holds word l of the chunk (two words a record)
+  auto fetch = [&](int j) {
+    return lane < 2 * step && j + (lane >> 1) < count ? __ldg(reinterpret_cast<const float4*>(recs + j) + lane)
+                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  int j = take();
+  float4 w = fetch(j);
+  while (j < count) {
+    const int jn = take();
+    const float4 wn = fetch(jn);
+    __syncwarp();  // the previous chunk is done with the slots
+    if (lane < 2 * kSegChunk) reinterpret_cast<float4*>(slots)[lane] = w;
+    const int rows = __shfl_sync(0xffffffffu, __float_as_int(w.w), 2 * lane + 1 < 32 ? 2 * lane + 1 : 0);
+    __syncwarp();
+    run(slots, lane < kSegChunk ? rows : 0);
+    j = jn;
+    w = wn;
+  }
 }
 
-// The box of brick origin o, edge B, widened by `below` voxels on the low
-// side, by `widen` (a bound on how far samples leave the flat map, e.g. by
-// the Ewald curvature) and the margin on both, for side 0 (positions) or
-// side 1 (negated positions) of matrix m.
-__device__ __forceinline__ SegBox seg_box(const float* m, int side, int3 o, int B, float below,
-                                          float widen = 0.f) {
-  SegBox b;
-  b.m = m;
-  b.sg = side ? -1.f : 1.f;
-  b.o = o;
-  b.below = below + widen + kSegMargin;
-  b.above = (float)B + widen + kSegMargin;
-  return b;
-}
+// Shared memory of the record slots.
+inline size_t seg_stage_bytes(int threads) { return sizeof(SegRec) * kSegChunk * (size_t)(threads / 32); }
 
 }  // namespace gtomrln
