@@ -1,0 +1,424 @@
+// Dense squared differences and cross-correlations on the tensor cores.
+//
+//   diff2[p][r][s] = 0.5 sum_i w_i |c_pi ref_ri - part_pi shift_si|^2
+//                  = 0.5 (A_pr + B_ps) - C_prs,
+// with a = sqrt(w) c ref, b = sqrt(w) part shift, A = sum |a|^2, B = sum |b|^2
+// and C = sum Re(a conj b): per particle a real matrix product over 2 x
+// elements terms (real and imaginary parts), which runs as tcgen05.mma
+// (kind::tf32, FP32 accumulators in tensor memory).
+//
+// Precision.  Every operand is split exactly into hi (its leading 11 bits)
+// and lo (the rest, of which the instruction keeps 11 bits), and hi hi +
+// hi lo + lo hi is accumulated: 22 bits of each product.  hi hi and the
+// cross terms have accumulators of their own, and every 64 elements (16
+// steps of 8) the accumulators are added to FP32 sums in registers with
+// round-to-nearest, because the tensor core's own additions truncate: left
+// alone for the whole sum their bias would reach 1e-4.  A, B and the final
+// combination are summed in double.  The expansion cancels where a and b are
+// close, so a tile of outputs with any diff2 below a quarter of (A + B) / 2
+// (or not finite) is computed again by the direct kernel (estep.cu), whose
+// FP32 sums of |a - b|^2 do not cancel: the relative error stays below the
+// direct kernel's everywhere.  In single-particle data the noise alone keeps
+// diff2 well above that.
+//
+// One CTA: 128 references x 64 shifts of one particle over a range of
+// elements (split so that every SM has two CTAs' work).  Its 256 threads
+// form the operands of 16 elements at a time in shared memory (128-byte
+// swizzled rows, hi and lo, 48 KB a stage, two stages), one thread issues
+// the 12 matrix instructions of a stage, and a commit on the stage's
+// mbarrier frees it.  Two accumulator sets in tensor memory alternate, so a
+// set is drained while the next is filled.
+//
+// 16 particles x 600 references x 49 shifts at 128^2: 1.54 ms by the direct
+// kernel (bound by its FP32 instructions), 0.33 ms here.
+#include <algorithm>
+#include <cstdint>
+
+#include "common.cuh"
+#include "diff2_tc.cuh"
+
+namespace gtomrln {
+
+namespace {
+
+constexpr int kM = 128, kN = 64, kE = 16;  // references, shifts, elements per stage
+constexpr int kThreads = 256;
+constexpr int kGroup = 4;  // stages per accumulator set
+constexpr unsigned kABytes = kM * kE * 8, kBBytes = kN * kE * 8;  // one of hi, lo
+constexpr unsigned kStageBytes = 2 * (kABytes + kBBytes);
+constexpr unsigned kTmemCols = 4 * kN;  // two sets of (hi hi, cross terms)
+constexpr size_t kSmem = 1024 + 2 * kStageBytes;
+constexpr unsigned long long kWaitNs = 1000000000ull;  // 1 s
+constexpr float kCloseFraction = 0.25f;
+
+// kind::tf32, FP32 accumulators, both operands K-major, 128 x 64.
+constexpr unsigned kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((kN / 8) << 17) | ((kM / 16) << 24);
+
+__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+// Shared-memory descriptor of a K-major tile of 128-byte swizzled rows
+// (eight rows per 1024 bytes).
+__device__ __forceinline__ unsigned long long tile_desc(unsigned addr) {
+  return (unsigned long long)((addr >> 4) & 0x3fffu) | (1ull << 16) | ((unsigned long long)(1024 >> 4) << 32) |
+         (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ void mma_tf32(unsigned d, unsigned long long a, unsigned long long b, unsigned accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+      "l"(a), "l"(b), "r"(kIdesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ bool bar_try(unsigned bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// False if the phase has not completed after kWaitNs.
+__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity) {
+  if (bar_try(bar, parity)) return true;
+  unsigned long long t0, t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+  for (;;) {
+    if (bar_try(bar, parity)) return true;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    if (t - t0 > kWaitNs) return false;
+  }
+}
+__device__ __forceinline__ void tmem_load32(unsigned addr, float* v) {
+  unsigned r[32];
+  // one statement: nothing may read the registers before the wait
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(addr)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 32; i++) v[i] += __uint_as_float(r[i]);
+}
+
+// Splits v into its leading 11 bits and the exact rest.
+__device__ __forceinline__ void split4(float4 v, float4& hi, float4& lo) {
+  auto top = [](float x) { return __uint_as_float(__float_as_uint(x) & 0xffffe000u); };
+  hi = make_float4(top(v.x), top(v.y), top(v.z), top(v.w));
+  lo = make_float4(v.x - hi.x, v.y - hi.y, v.z - hi.z, v.w - hi.w);
+}
+
+// Two consecutive complex elements of a row, zero past the end.  vec: rows
+// start on 16-byte boundaries.
+__device__ __forceinline__ float4 load2(const float2* __restrict__ row, int64_t i, int64_t end, bool vec) {
+  if (vec && i + 1 < end) return __ldg(reinterpret_cast<const float4*>(row + i));
+  const float2 a = i < end ? __ldg(row + i) : make_float2(0.f, 0.f);
+  const float2 b = i + 1 < end ? __ldg(row + i + 1) : make_float2(0.f, 0.f);
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+struct TcArgs {
+  const float2* particle;
+  const float* minvsigma2;
+  const float* ctf;
+  int64_t elements;
+  const float2* shifts;
+  const float2* refs;
+  unsigned nparticles, nrefs, nshifts;
+  int mtiles, ntiles, splits, cc, vec;
+  float* part;  // C: [split][particle][ref][shift]
+  float* sa;    // A: [split][particle][ref]
+  float* sb;    // B: [split][particle][shift]
+};
+
+__global__ void __launch_bounds__(kThreads, 2) diff2_tc_kernel(const TcArgs a) {
+  extern __shared__ unsigned char raw[];
+  __shared__ unsigned long long bars[2];
+  __shared__ unsigned tmem_s;
+  const unsigned base = (smem_u32(raw) + 1023u) & ~1023u;
+  unsigned char* stage0 = raw + (base - smem_u32(raw));
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  unsigned b = blockIdx.x;
+  const int split = b % a.splits;
+  b /= a.splits;
+  const int nt = b % a.ntiles;
+  b /= a.ntiles;
+  const int mt = b % a.mtiles;
+  const unsigned p = b / a.mtiles;
+  const unsigned r0 = mt * kM, s0 = nt * kN;
+  const int64_t chunks = (a.elements + kE - 1) / kE;
+  const int64_t c0 = chunks * split / a.splits, c1 = chunks * (split + 1) / a.splits;
+  const int nch = (int)(c1 - c0);
+  const int64_t end = a.elements;
+
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bars[0])) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bars[1])) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_s)),
+                 "r"(kTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const unsigned tmem = tmem_s;
+
+  // thread -> 16-byte unit j (two elements) of rows row0 + 32 k
+  const int j = tid & 7, row0 = tid >> 3;
+  const unsigned swz = (unsigned)((j ^ (row0 & 7)) << 4) + (unsigned)(row0 & 7) * 128 + (unsigned)(row0 >> 3) * 1024;
+  const float2* pp = a.particle + a.elements * p;
+  const float* cp = a.ctf ? a.ctf + a.elements * p : nullptr;
+  float sa[4] = {0.f, 0.f, 0.f, 0.f}, sb[2] = {0.f, 0.f};
+  float acc[32];
+#pragma unroll
+  for (int i = 0; i < 32; i++) acc[i] = 0.f;
+
+  float4 rv[4], sv[2], pv;
+  float cs[2];
+  auto fetch = [&](int t) {  // the raw operands of chunk t
+    const int64_t i = (c0 + t) * kE + 2 * j;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const unsigned r = r0 + row0 + 32 * k;
+      rv[k] = r < a.nrefs ? load2(a.refs + a.elements * r, i, end, a.vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const unsigned s = s0 + row0 + 32 * k;
+      sv[k] = s < a.nshifts ? load2(a.shifts + a.elements * s, i, end, a.vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    pv = load2(pp, i, end, a.vec);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const bool in = i + h < end;
+      const float w = a.cc || !a.minvsigma2 || !in ? 1.f : sqrtf(__ldg(a.minvsigma2 + i + h));
+      cs[h] = (cp && in ? __ldg(cp + i + h) : 1.f) * w;
+      if (h == 0) {
+        pv.x *= w;
+        pv.y *= w;
+      } else {
+        pv.z *= w;
+        pv.w *= w;
+      }
+    }
+  };
+  // warps 0-3 drain columns 0-31 of their lanes' rows, warps 4-7 the others
+  auto drain = [&](int group) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const unsigned at = tmem + (unsigned)((group & 1) * 2 * kN + (warp >> 2) * 32) + ((unsigned)(warp & 3) << 21);
+    tmem_load32(at, acc);
+    tmem_load32(at + kN, acc);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  };
+
+  bool ok = true;
+  int drained = 0;
+  if (nch > 0) fetch(0);
+  for (int t = 0; t < nch; t++) {
+    const int s = t & 1;
+    if (t >= 2) {  // the stage's earlier matrix instructions are done
+      const bool w = bar_wait(smem_u32(&bars[s]), (unsigned)((t >> 1) - 1) & 1u);
+      if (!__syncthreads_and(w)) {
+        ok = false;
+        break;
+      }
+      if (t % kGroup == 1) drain(drained++);  // and with chunk t - 2 its accumulator set
+    }
+    unsigned char* st = stage0 + s * kStageBytes;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const float4 v = make_float4(rv[k].x * cs[0], rv[k].y * cs[0], rv[k].z * cs[1], rv[k].w * cs[1]);
+      sa[k] = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, sa[k]))));
+      float4 hi, lo;
+      split4(v, hi, lo);
+      *reinterpret_cast<float4*>(st + swz + k * 4096) = hi;
+      *reinterpret_cast<float4*>(st + kABytes + swz + k * 4096) = lo;
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const float4 v = make_float4(pv.x * sv[k].x - pv.y * sv[k].y, pv.x * sv[k].y + pv.y * sv[k].x,
+                                   pv.z * sv[k].z - pv.w * sv[k].w, pv.z * sv[k].w + pv.w * sv[k].z);
+      sb[k] = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, sb[k]))));
+      float4 hi, lo;
+      split4(v, hi, lo);
+      *reinterpret_cast<float4*>(st + 2 * kABytes + swz + k * 4096) = hi;
+      *reinterpret_cast<float4*>(st + 2 * kABytes + kBBytes + swz + k * 4096) = lo;
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (tid == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const unsigned sb0 = base + s * kStageBytes;
+      const unsigned long long ah = tile_desc(sb0), al = tile_desc(sb0 + kABytes), bh = tile_desc(sb0 + 2 * kABytes),
+                               bl = tile_desc(sb0 + 2 * kABytes + kBBytes);
+      const unsigned d = tmem + (unsigned)(((t / kGroup) & 1) * 2 * kN);
+      const unsigned first = t % kGroup == 0;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {  // 8 values (32 bytes) a step
+        mma_tf32(d, ah + 2 * k, bh + 2 * k, !(first && k == 0));
+        mma_tf32(d + kN, ah + 2 * k, bl + 2 * k, !(first && k == 0));
+        mma_tf32(d + kN, al + 2 * k, bh + 2 * k, 1);
+      }
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                       smem_u32(&bars[s]))
+                   : "memory");
+    }
+    if (t + 1 < nch) fetch(t + 1);
+  }
+  // the last commit covers everything issued before it
+  if (nch > 0 && ok) {
+    const int t = nch - 1;
+    ok = bar_wait(smem_u32(&bars[t & 1]), (unsigned)(t >> 1) & 1u);
+    ok = __syncthreads_and(ok);
+    if (ok)
+      while (drained <= t / kGroup) drain(drained++);
+  }
+  // a wait that ran out (nothing of this kernel's own can cause it): NaN,
+  // after one more wait for the matrix instructions in flight
+  if (!ok) bar_wait(smem_u32(&bars[0]), 0u);
+  const float bad = ok ? 0.f : __int_as_float(0x7fc00000);
+  {
+    const unsigned r = r0 + (warp & 3) * 32 + lane;
+    if (r < a.nrefs) {
+      float* out = a.part + (((int64_t)split * a.nparticles + p) * a.nrefs + r) * a.nshifts;
+#pragma unroll
+      for (int i = 0; i < 32; i++) {
+        const unsigned s = s0 + (warp >> 2) * 32 + i;
+        if (s < a.nshifts) out[s] = acc[i] + bad;
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) sa[k] += __shfl_xor_sync(0xffffffffu, sa[k], o);
+#pragma unroll
+    for (int k = 0; k < 2; k++) sb[k] += __shfl_xor_sync(0xffffffffu, sb[k], o);
+  }
+  if (j == 0) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const unsigned r = r0 + row0 + 32 * k;
+      if (nt == 0 && r < a.nrefs) a.sa[((int64_t)split * a.nparticles + p) * a.nrefs + r] = sa[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const unsigned s = s0 + row0 + 32 * k;
+      if (mt == 0 && s < a.nshifts) a.sb[((int64_t)split * a.nparticles + p) * a.nshifts + s] = sb[k];
+    }
+  }
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+}
+
+// Combines the splits, writes the outputs and marks the 64 x 64 tiles (of the
+// direct kernel) that hold a close match or a value that is not finite.
+__global__ void __launch_bounds__(256)
+diff2_tc_combine_kernel(const TcArgs a, float* __restrict__ diff2, int* __restrict__ flags) {
+  const int64_t n = (int64_t)a.nparticles * a.nrefs * a.nshifts;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t pr = i / a.nshifts;
+    const unsigned s = (unsigned)(i - pr * a.nshifts);
+    const int64_t p = pr / a.nrefs;
+    const unsigned r = (unsigned)(pr - p * a.nrefs);
+    double c = 0, sa = 0, sb = 0;
+    for (int k = 0; k < a.splits; k++) {
+      c += (double)a.part[k * n + i];
+      sa += (double)a.sa[((int64_t)k * a.nparticles) * a.nrefs + pr];
+      if (!a.cc) sb += (double)a.sb[((int64_t)k * a.nparticles + p) * a.nshifts + s];
+    }
+    const double half = 0.5 * (sa + sb);
+    const float v = a.cc ? (float)(-c / sqrt(sa)) : (float)(half - c);
+    diff2[i] = v;
+    if (a.cc ? !isfinite(v) : !(v >= kCloseFraction * (float)half) || !isfinite(v)) {
+      const unsigned rt = (a.nrefs + kDiffTile - 1) / kDiffTile, st = (a.nshifts + kDiffTile - 1) / kDiffTile;
+      flags[(p * rt + r / kDiffTile) * st + s / kDiffTile] = 1;
+    }
+  }
+}
+
+}  // namespace
+
+int diff2_tensor(const float2* particle, const float* minvsigma2, const float* ctf, int64_t elements,
+                 const float2* shifts, const float2* refs, float* diff2, unsigned nparticles, unsigned nrefs,
+                 unsigned nshifts, bool cc, cudaStream_t stream) {
+  TcArgs a;
+  a.particle = particle;
+  a.minvsigma2 = minvsigma2;
+  a.ctf = ctf;
+  a.elements = elements;
+  a.shifts = shifts;
+  a.refs = refs;
+  a.nparticles = nparticles;
+  a.nrefs = nrefs;
+  a.nshifts = nshifts;
+  a.mtiles = (int)((nrefs + kM - 1) / kM);
+  a.ntiles = (int)((nshifts + kN - 1) / kN);
+  a.cc = cc ? 1 : 0;
+  a.vec = elements % 2 == 0 && ((uintptr_t)particle | (uintptr_t)shifts | (uintptr_t)refs) % 16 == 0;
+  int dev = 0, sms = 148;
+  GTOMRLN_CUDA_TRY(cudaGetDevice(&dev));
+  GTOMRLN_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int64_t units = (int64_t)nparticles * a.mtiles * a.ntiles, slots = 2 * sms;
+  const int64_t chunks = (elements + kE - 1) / kE;
+  // the split of the elements that fills whole waves of two CTAs per SM
+  // best, each part 16 stages at least and a set-up of about four
+  double best = 1e30;
+  a.splits = 1;
+  for (int k = 1; k <= 32 && (k == 1 || chunks / k >= 16); k++) {
+    const double waves = (double)((units * k + slots - 1) / slots);
+    const double cost = waves * ((double)chunks / k + 4.0);
+    if (cost < best * 0.97) {
+      best = cost;
+      a.splits = k;
+    }
+  }
+  const int64_t n = (int64_t)nparticles * nrefs * nshifts;
+  const size_t tiles = (size_t)nparticles * ((nrefs + kDiffTile - 1) / kDiffTile) * ((nshifts + kDiffTile - 1) / kDiffTile);
+  if (units * a.splits > 0x7fffffffLL) return set_error(GTOMRLN_ERR_INVALID, "squared differences: too many tiles");
+  const size_t nsa = (size_t)nparticles * nrefs * a.splits, nsb = (size_t)nparticles * nshifts * a.splits;
+  float* scratch = nullptr;
+  if (pool_alloc((void**)&scratch, sizeof(float) * ((size_t)n * a.splits + nsa + nsb + tiles), stream)) {
+    clear_error();  // no room for the partial products: the direct kernel needs none
+    return diff2_direct(particle, minvsigma2, ctf, elements, shifts, refs, diff2, nparticles, nrefs, nshifts, cc,
+                        nullptr, stream);
+  }
+  a.part = scratch;
+  a.sa = a.part + (size_t)n * a.splits;
+  a.sb = a.sa + nsa;
+  int* flags = reinterpret_cast<int*>(a.sb + nsb);
+  cudaError_t e = cudaMemsetAsync(flags, 0, tiles * sizeof(int), stream);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(diff2_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+  if (e == cudaSuccess) {
+    diff2_tc_kernel<<<(unsigned)(units * a.splits), kThreads, kSmem, stream>>>(a);
+    diff2_tc_combine_kernel<<<(unsigned)std::min<int64_t>((n + 255) / 256, 16 * sms), 256, 0, stream>>>(a, diff2,
+                                                                                                      flags);
+    e = cudaGetLastError();
+  }
+  int st = GTOMRLN_OK;
+  if (e == cudaSuccess)
+    st = diff2_direct(particle, minvsigma2, ctf, elements, shifts, refs, diff2, nparticles, nrefs, nshifts, cc, flags,
+                      stream);
+  const int st2 = pool_free(scratch, stream);
+  if (e != cudaSuccess)
+    return set_error(GTOMRLN_ERR_CUDA, "launch of diff2_tc_kernel failed: %s", cudaGetErrorString(e));
+  return st ? st : st2;
+}
+
+}  // namespace gtomrln

@@ -11,6 +11,7 @@
 #include <cub/device/device_select.cuh>
 
 #include "common.cuh"
+#include "diff2_tc.cuh"
 
 namespace gtomrln {
 
@@ -128,7 +129,7 @@ diff2_group_kernel(const float2* __restrict__ particle, const float* __restrict_
 // instructions instead of five (the extra rounding of the scaled operands
 // is of the order of the products' own; the expanded form, which would
 // cancel for close matches, is not used).
-constexpr int kDT = 64;        // references and shifts per tile
+constexpr int kDT = kDiffTile;  // references and shifts per tile
 constexpr int kDK = 32;        // elements per staged chunk
 constexpr int kDThreads = 256;
 template <bool CC>
@@ -136,7 +137,8 @@ __global__ void __launch_bounds__(kDThreads)
 diff2_dense_tiled_kernel(const float2* __restrict__ particle, const float* __restrict__ minvsigma2,
                          const float* __restrict__ ctf, int64_t elements, const float2* __restrict__ shifts,
                          const float2* __restrict__ refs, float* __restrict__ diff2, unsigned nrefs,
-                         unsigned nshifts) {
+                         unsigned nshifts, const int* __restrict__ flags) {
+  if (flags && !flags[((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x]) return;
   __shared__ float2 As[kDK][kDT + 1];  // c * ref
   __shared__ float2 Bs[kDK][kDT + 1];  // particle * shift
   const unsigned part = blockIdx.z, r0 = blockIdx.y * kDT, s0 = blockIdx.x * kDT;
@@ -398,6 +400,20 @@ struct Positive {
 };
 
 }  // namespace
+int diff2_direct(const float2* particle, const float* minvsigma2, const float* ctf, int64_t elements,
+                 const float2* shifts, const float2* refs, float* diff2, unsigned nparticles, unsigned nrefs,
+                 unsigned nshifts, bool cc, const int* flags, cudaStream_t stream) {
+  const dim3 grid((nshifts + kDT - 1) / kDT, (nrefs + kDT - 1) / kDT, nparticles);
+  if (cc)
+    diff2_dense_tiled_kernel<true><<<grid, kDThreads, 0, stream>>>(particle, minvsigma2, ctf, elements, shifts, refs,
+                                                                   diff2, nrefs, nshifts, flags);
+  else
+    diff2_dense_tiled_kernel<false><<<grid, kDThreads, 0, stream>>>(particle, minvsigma2, ctf, elements, shifts, refs,
+                                                                    diff2, nrefs, nshifts, flags);
+  GTOMRLN_LAUNCH_CHECK("diff2_dense_tiled_kernel");
+  return GTOMRLN_OK;
+}
+
 }  // namespace gtomrln
 
 using namespace gtomrln;
@@ -442,18 +458,17 @@ int gtomrln_squared_differences(const float* d_particleft, const float* d_minvsi
     return set_error(GTOMRLN_ERR_INVALID, "squared_differences: group size %u not 1, 2, 4 or 8", tile);
   if (nparticles > 65535)
     return set_error(GTOMRLN_ERR_INVALID, "squared_differences: more than 65535 particles per call");
-  // The dense layout does not depend on the group size: one tiled kernel.
-  dim3 grid((nshifts + kDT - 1) / kDT, (nrefs + kDT - 1) / kDT, nparticles);
-  if (dofirstitercc)
-    diff2_dense_tiled_kernel<true><<<grid, kDThreads, 0, (cudaStream_t)stream>>>(
-        (const float2*)d_particleft, d_minvsigma2, d_ctf, elements, (const float2*)d_precalcshifts,
-        (const float2*)d_refft, d_diff2, nrefs, nshifts);
-  else
-    diff2_dense_tiled_kernel<false><<<grid, kDThreads, 0, (cudaStream_t)stream>>>(
-        (const float2*)d_particleft, d_minvsigma2, d_ctf, elements, (const float2*)d_precalcshifts,
-        (const float2*)d_refft, d_diff2, nrefs, nshifts);
-  GTOMRLN_LAUNCH_CHECK("diff2_dense_tiled_kernel");
-  return GTOMRLN_OK;
+  // The dense layout does not depend on the group size.  The tensor cores
+  // take it where the sums are long enough to pay for the partial products'
+  // second pass (a few microseconds), outside stream capture (they need
+  // scratch).
+  cudaStream_t s = (cudaStream_t)stream;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusActive;
+  if (elements >= 512 && cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone)
+    return diff2_tensor((const float2*)d_particleft, d_minvsigma2, d_ctf, elements, (const float2*)d_precalcshifts,
+                        (const float2*)d_refft, d_diff2, nparticles, nrefs, nshifts, dofirstitercc != 0, s);
+  return diff2_direct((const float2*)d_particleft, d_minvsigma2, d_ctf, elements, (const float2*)d_precalcshifts,
+                      (const float2*)d_refft, d_diff2, nparticles, nrefs, nshifts, dofirstitercc != 0, nullptr, s);
 }
 
 int gtomrln_convert_weights_dense(float* d_weights, unsigned nparticles, unsigned nclasses, unsigned nrot,
