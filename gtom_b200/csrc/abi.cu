@@ -418,15 +418,25 @@ static std::atomic<int> g_path[3] = {{GTOMRLN_PATH_AUTO}, {GTOMRLN_PATH_AUTO}, {
 
 int path_choice(int op) { return (op >= 0 && op <= 2) ? g_path[op].load() : GTOMRLN_PATH_AUTO; }
 
-// Crossovers measured at padding 2 (direct vs row-segment, ms):
-// backprojector  n = 128: 1 000 slices 0.48 vs 0.76, 3 000: 1.40 vs 1.97,
-//                10 000: 4.56 vs 3.23; n = 192: 300 slices 0.64 vs 0.52;
-//                n = 96, 10 000: 2.65 vs 2.97;
-// projector      n = 192: 3 000 slices 0.86 vs 1.05, 10 000: 2.99 vs 2.08;
-//                n = 256: 300 slices 0.26 vs 0.50, 1 000: 0.83 vs 0.72.
-bool brick_path_pays(int op, int V, unsigned batch) {
-  if (op == GTOMRLN_OP_BACKPROJECT) return (V >= 384 && batch >= 300) || (V >= 256 && batch >= 6000);
-  return (V >= 512 && batch >= 1000) || (V >= 384 && batch >= 6000);
+// Samples from which the row-segment kernels win, by volume edge, from sweeps
+// at padding 2 (n = V / 2; us, direct against segment):
+// projector      n = 256: 300 slices 282 vs 292, 1 000: 866 vs 493; n = 192:
+//                1 000: 318 vs 330, 3 000: 901 vs 640; n = 160: 1 000: 193 vs
+//                251, 3 000: 531 vs 505; n = 128: 3 000: 341 vs 396, 10 000:
+//                1 068 vs 898; n = 96, 10 000: 610 vs 645;
+// backprojector  n = 256: 100 slices 664 vs 851, 300: 1 769 vs 976; n = 192:
+//                100: 302 vs 408, 300: 773 vs 464; n = 160: 100: 170 vs 268,
+//                300: 388 vs 308; n = 128: 300: 187 vs 210, 1 000: 401 vs 315;
+//                n = 96, 3 000: 477 vs 410; n = 64: 3 000: 240 vs 243, 10 000:
+//                670 vs 543; n = 48, 10 000: 407 vs 395 (below V = 321 the
+//                direct kernel reduces into a packed scratch).
+// The direct kernels' cost per sample grows once the volume leaves L2; the
+// segment kernels pay a plan and the staging or flush of every brick first.
+bool brick_path_pays(int op, int V, double rmax, unsigned batch) {
+  const double samples = 1.5707963 * rmax * rmax * batch;
+  if (op == GTOMRLN_OP_BACKPROJECT)
+    return V >= 256 ? samples >= 2.5e6 : V >= 128 && batch >= 2000 && samples >= 6e6;
+  return samples >= (V >= 512 ? 11e6 : V >= 384 ? 19e6 : V >= 320 ? 24e6 : V >= 256 ? 28e6 : 1e300);
 }
 
 // Defaults measured on the B200 at 256^3 (padding 2) with 10,000-slice

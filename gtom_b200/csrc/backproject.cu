@@ -176,6 +176,7 @@ backproject_direct_kernel(float2* __restrict__ volft_base, float* __restrict__ v
 __global__ void __launch_bounds__(256)
 backproject_unpack_kernel(const float4* __restrict__ packed, float2* __restrict__ volft, float* __restrict__ volw,
                           int64_t n) {
+  grid_dependency_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const float4 p = packed[i];
     if (p.x == 0.f && p.y == 0.f && p.z == 0.f) continue;
@@ -215,6 +216,17 @@ backproject_unpack_kernel(const float4* __restrict__ packed, float2* __restrict_
 // inverse scale.  Squared interpolation weights stay in FP32.
 // ---------------------------------------------------------------------------
 constexpr int kFxBias = 1 << 30;
+
+// Asks for a row segment's slice values and weights ahead of the waves that
+// read them (a wave otherwise waits for HBM, and registers allow no second
+// wave in flight).
+__device__ __forceinline__ void prefetch_row(const float2* projft, const float* projw, int64_t first, int count) {
+  if (projft) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(projft + first));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(projft + first + count - 1));
+  }
+  if (projw) asm volatile("prefetch.global.L2 [%0];" ::"l"(projw + first));
+}
 constexpr float kFxBand = 16.f;  // voxels of sample radius per band
 constexpr int kFxMaxBands = 128;
 
@@ -251,6 +263,7 @@ __global__ void fx_band_sample_kernel(const float2* __restrict__ projft, const f
                                       unsigned* __restrict__ count) {
   __shared__ unsigned sv[kFxMaxBands], sw[kFxMaxBands], sc[kFxMaxBands];
   __shared__ float ssv[kFxMaxBands], ssw[kFxMaxBands];
+  grid_dependency_wait();
   for (int b = threadIdx.x; b < nbands; b += blockDim.x) {
     sv[b] = sw[b] = sc[b] = 0u;
     ssv[b] = ssw[b] = 0.f;
@@ -311,7 +324,9 @@ __device__ __forceinline__ bool fx_scale(float m, float& s) {
 // The item's scales: the largest sampled magnitudes over the bands its
 // pixels can come from (the brick widened by its neighbours' reach, one band
 // of margin either way).  False (FP32) where those bands hold no non-zero
-// sample or magnitudes too spread out.
+// sample or magnitudes too spread out.  By one warp, its lanes over the
+// bands (one thread's chain of loads took ~10 us an item); every lane
+// returns the same.
 __device__ __forceinline__ bool fx_item_scales(const FxBands& f, int3 o, int B, float& sv, float& sw) {
   const float lo[3] = {(float)o.x - 2.f, (float)o.y - 2.f, (float)o.z - 2.f};
   const float hi[3] = {(float)(o.x + B) + 1.f, (float)(o.y + B) + 1.f, (float)(o.z + B) + 1.f};
@@ -325,16 +340,18 @@ __device__ __forceinline__ bool fx_item_scales(const FxBands& f, int3 o, int B, 
   const int b0 = max(0, (int)(sqrtf(dmin2) * (1.f / kFxBand)) - 1);
   const int b1 = min(f.nbands - 1, (int)(sqrtf(dmax2) * (1.f / kFxBand)) + 1);
   unsigned mv = 0u, mw = 0u;
-  for (int b = b0; b <= b1; b++) {
-    mv = max(mv, f.vmax[b]);
-    mw = max(mw, f.wmax[b]);
-    const unsigned c = f.count[b];
-    if (c && (__uint_as_float(f.vmax[b]) * (float)c > kFxMaxSpread * f.vsum[b] ||
-              __uint_as_float(f.wmax[b]) * (float)c > kFxMaxSpread * f.wsum[b]))
-      return false;  // magnitudes too spread out in this band for fixed point
+  bool spread = false;  // magnitudes too spread out in a band for fixed point
+  for (int b = b0 + (int)(threadIdx.x & 31); b <= b1; b += 32) {
+    const unsigned bv = f.vmax[b], bw = f.wmax[b], c = f.count[b];
+    mv = max(mv, bv);
+    mw = max(mw, bw);
+    spread |= c && (__uint_as_float(bv) * (float)c > kFxMaxSpread * f.vsum[b] ||
+                    __uint_as_float(bw) * (float)c > kFxMaxSpread * f.wsum[b]);
   }
+  mv = __reduce_max_sync(0xffffffffu, mv);
+  mw = __reduce_max_sync(0xffffffffu, mw);
   // no magnitude sampled where this brick's pixels come from: FP32
-  if (mv == 0u || mw == 0u) return false;
+  if (__any_sync(0xffffffffu, spread) || mv == 0u || mw == 0u) return false;
   return fx_scale(__uint_as_float(mv), sv) && fx_scale(__uint_as_float(mw), sw);
 }
 
@@ -358,54 +375,75 @@ __device__ __forceinline__ void bp_flush_brick(float2* __restrict__ volft, float
                                                const float* are, const float* aim, const float* aw, int B,
                                                int RS, int PS, int3 o, int V, int rowlen, bool exclusive,
                                                bool fx = false, float inv_v = 1.f, float inv_w = 1.f) {
+  constexpr int kRows = 4;  // rows in flight per warp: their read-add-writes wait for HBM together
   const int lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  for (int row = threadIdx.x >> 5; row < B * B; row += nwarps) {  // one warp per (y, z) row
-    const int ly = row % B, lz = row / B;
+  for (int row0 = threadIdx.x >> 5; row0 < B * B; row0 += kRows * nwarps) {  // one warp per (y, z) row
     for (int lx = lane; lx < B; lx += 32) {
-      int k = lz * PS + ly * RS + lx;
-      float r = are[k], im = aim[k], ww = aw[k];
-      if (fx) {
-        r = (float)(__float_as_int(r) - kFxBias) * inv_v;
-        im = (float)(__float_as_int(im) - kFxBias) * inv_v;
-        ww = (float)(__float_as_int(ww) - kFxBias) * inv_w;
-      }
-      if (r == 0.f && im == 0.f && ww == 0.f) continue;
-      int x = o.x + lx, y = o.y + ly, z = o.z + lz;
-      if (FACES && x < 0) continue;
-      const bool face = FACES && (lx == 0 || lx == B - 1 || ly == 0 || ly == B - 1 || lz == 0 || lz == B - 1);
-      int ys, zs;
-      bool alias;
-      if (DECENTERED) {
-        ys = y < 0 ? y + V : y;
-        zs = z < 0 ? z + V : z;
-        alias = (y == V / 2 || y == -(V / 2) || z == V / 2 || z == -(V / 2));
-      } else {
-        ys = y + V / 2;
-        zs = z + V / 2;
-        alias = false;
-      }
-      if (CLAMP && !DECENTERED) {
-        const unsigned cx = min((unsigned)x, (unsigned)(V / 2)), cy = min((unsigned)ys, (unsigned)(V - 1)),
-                       cz = min((unsigned)zs, (unsigned)(V - 1));
-        // every voxel on a face the clamps fold onto, not only the folded
-        // ones: a plain read-add-write there would race with their reductions
-        alias = cx == (unsigned)(V / 2) || cy == (unsigned)(V - 1) || cz == (unsigned)(V - 1);
-        x = (int)cx;
-        ys = (int)cy;
-        zs = (int)cz;
-      } else if ((unsigned)x > (unsigned)(V / 2) || (unsigned)ys >= (unsigned)V || (unsigned)zs >= (unsigned)V) {
-        continue;  // outside the volume: nothing can have been added here
-      }
-      int64_t idx = ((int64_t)zs * V + ys) * rowlen + x;
-      if (exclusive && !alias && !face) {
-        if (volft) {
-          float2 c = volft[idx];
-          volft[idx] = make_float2(c.x + r, c.y + im);
+      float r[kRows], im[kRows], ww[kRows], cw[kRows];
+      float2 cv[kRows];
+      int64_t idx[kRows];  // -1: nothing to add
+      bool plain[kRows];
+#pragma unroll
+      for (int q = 0; q < kRows; q++) {
+        const int row = row0 + q * nwarps;
+        idx[q] = -1;
+        plain[q] = false;
+        if (row >= B * B) continue;
+        const int ly = row % B, lz = row / B;
+        const int k = lz * PS + ly * RS + lx;
+        r[q] = are[k];
+        im[q] = aim[k];
+        ww[q] = aw[k];
+        if (fx) {
+          r[q] = (float)(__float_as_int(r[q]) - kFxBias) * inv_v;
+          im[q] = (float)(__float_as_int(im[q]) - kFxBias) * inv_v;
+          ww[q] = (float)(__float_as_int(ww[q]) - kFxBias) * inv_w;
         }
-        if (volw) volw[idx] += ww;
-      } else {
-        if (volft) red_add2((float*)(volft + idx), r, im);
-        if (volw) red_add(volw + idx, ww);
+        if (r[q] == 0.f && im[q] == 0.f && ww[q] == 0.f) continue;
+        int x = o.x + lx;
+        const int y = o.y + ly, z = o.z + lz;
+        if (FACES && x < 0) continue;
+        const bool face = FACES && (lx == 0 || lx == B - 1 || ly == 0 || ly == B - 1 || lz == 0 || lz == B - 1);
+        int ys, zs;
+        bool alias;
+        if (DECENTERED) {
+          ys = y < 0 ? y + V : y;
+          zs = z < 0 ? z + V : z;
+          alias = (y == V / 2 || y == -(V / 2) || z == V / 2 || z == -(V / 2));
+        } else {
+          ys = y + V / 2;
+          zs = z + V / 2;
+          alias = false;
+        }
+        if (CLAMP && !DECENTERED) {
+          const unsigned cx = min((unsigned)x, (unsigned)(V / 2)), cy = min((unsigned)ys, (unsigned)(V - 1)),
+                         cz = min((unsigned)zs, (unsigned)(V - 1));
+          // every voxel on a face the clamps fold onto, not only the folded
+          // ones: a plain read-add-write there would race with their reductions
+          alias = cx == (unsigned)(V / 2) || cy == (unsigned)(V - 1) || cz == (unsigned)(V - 1);
+          x = (int)cx;
+          ys = (int)cy;
+          zs = (int)cz;
+        } else if ((unsigned)x > (unsigned)(V / 2) || (unsigned)ys >= (unsigned)V || (unsigned)zs >= (unsigned)V) {
+          continue;  // outside the volume: nothing can have been added here
+        }
+        idx[q] = ((int64_t)zs * V + ys) * rowlen + x;
+        plain[q] = exclusive && !alias && !face;
+        if (plain[q]) {
+          if (volft) cv[q] = volft[idx[q]];
+          if (volw) cw[q] = volw[idx[q]];
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kRows; q++) {
+        if (idx[q] < 0) continue;
+        if (plain[q]) {
+          if (volft) volft[idx[q]] = make_float2(cv[q].x + r[q], cv[q].y + im[q]);
+          if (volw) volw[idx[q]] = cw[q] + ww[q];
+        } else {
+          if (volft) red_add2((float*)(volft + idx[q]), r[q], im[q]);
+          if (volw) red_add(volw + idx[q], ww[q]);
+        }
       }
     }
   }
@@ -547,6 +585,7 @@ backproject_segment_kernel(float2* __restrict__ volft_base, float* __restrict__ 
   extern __shared__ float4 smem4[];  // record slots, then the accumulators
   __shared__ int item_s, next_s, danger_s;
   __shared__ float sv_s, sw_s;
+  grid_dependency_wait();
   const int nitems = *nitems_ptr;
   // accumulators of E voxels per axis
   const int E = EDGE ? EDGE : g.B + 1, B = E - 1;
@@ -605,6 +644,9 @@ backproject_segment_kernel(float2* __restrict__ volft_base, float* __restrict__ 
               }
               seg_box_bounds(box, o, B, widen);
               seg_row(box, px, v, ua, ub);
+              if (ub >= ua)
+                prefetch_row(projft, projw, a.elements * (r.ss() >> 1) + ((v < 0 ? v + a.n : v) * a.dimft + ua),
+                             ub - ua + 1);
             },
             [&](int p, int u, int v, bool valid) {
               if (!valid) return;
@@ -693,17 +735,14 @@ backproject_segment_kernel(float2* __restrict__ volft_base, float* __restrict__ 
     for (;;) {
       const float zero = fx ? __int_as_float(kFxBias) : 0.f;
       for (int k = threadIdx.x; k < 3 * NA; k += blockDim.x) acc[k] = zero;
-      if (threadIdx.x == 0) {
-        next_s = 0;
-        danger_s = 0;
-        if (fx) {
-          float svv, sww;
-          if (fx_item_scales(fxb, o, B, svv, sww)) {
-            sv_s = svv;
-            sw_s = sww;
-          } else {
-            danger_s = 1;  // no usable scale: FP32
-          }
+      if (threadIdx.x < 32) {
+        float svv = 1.f, sww = 1.f;
+        const bool scaled = fx && fx_item_scales(fxb, o, B, svv, sww);
+        if (threadIdx.x == 0) {
+          next_s = 0;
+          sv_s = svv;
+          sw_s = sww;
+          danger_s = fx && !scaled;  // no usable scale: FP32
         }
       }
       __syncthreads();
@@ -903,9 +942,9 @@ static int backproject_brick(float* d_volumeft, float* d_volumeweights, const fl
     }
   }
   if (segments)
-    skern<<<sms * std::max(occ, 1), tune.threads, smem, stream>>>(
-        (float2*)d_volumeft, d_volumeweights, (const float2*)d_projft, d_projweights, d_mats, a, g, px, gm,
-        plan.items, plan.nitems, plan.recs, plan.counter, fxb);
+    launch_dependent(skern, sms * std::max(occ, 1), tune.threads, smem, stream, (float2*)d_volumeft, d_volumeweights,
+                     (const float2*)d_projft, d_projweights, d_mats, a, g, px, gm, plan.items, plan.nitems, plan.recs,
+                     plan.counter, fxb);
   else
     kern<<<sms * std::max(occ, 1), tune.threads, smem, stream>>>(
         (float2*)d_volumeft, d_volumeweights, (const float2*)d_projft, d_projweights, d_mats, a, g, plan.items,
@@ -1026,6 +1065,7 @@ backproject_shifted_segment_kernel(float2* __restrict__ volft, float* __restrict
                                    int* __restrict__ counter) {
   extern __shared__ float4 smem4[];  // record slots, then the accumulators
   __shared__ int item_s, next_s;
+  grid_dependency_wait();
   const int nitems = *nitems_ptr;
   const int E = EDGE ? EDGE : g.B + 1, B = E - 1;
   const int RS = bp_pitch(E).row, PS = bp_pitch(E).plane, NA = E * PS;
@@ -1055,6 +1095,9 @@ backproject_shifted_segment_kernel(float2* __restrict__ volft, float* __restrict
             SegBox box = {{r.a.x, r.a.y, r.a.z}, {r.a.w, r.b.x, r.b.y}, {}, {}};
             seg_box_bounds(box, o, B, 0.f);
             seg_row(box, px, v, ua, ub);
+            if (ub >= ua)
+              prefetch_row(projft, projw, a.elements * (r.ss() >> 1) + ((v < 0 ? v + a.n : v) * a.dimft + ua),
+                             ub - ua + 1);
           },
           [&](int p, int u, int v, bool valid) {
             if (!valid) return;
@@ -1138,9 +1181,9 @@ static int backproject_shifted_brick(float* d_volumeft, float* d_volumeweights, 
   int st = build_brick_plan(GTOMRLN_OP_BACKPROJECT, d_mats, (int)batch, g, px, limit, tune.chunk, stream, &plan, 1,
                             nullptr, gm);
   if (st) return st;
-  kern<<<sms * std::max(occ, 1), tune.threads, smem, stream>>>(
-      (float2*)d_volumeft, d_volumeweights, (const float2*)d_projft, d_projweights, d_shifts, d_gweights, a, g, px,
-      plan.items, plan.nitems, plan.recs, plan.counter);
+  launch_dependent(kern, sms * std::max(occ, 1), tune.threads, smem, stream, (float2*)d_volumeft, d_volumeweights,
+                   (const float2*)d_projft, d_projweights, d_shifts, d_gweights, a, g, px, plan.items, plan.nitems,
+                   plan.recs, plan.counter);
   backproject_shifted_kernel<2><<<sms * 4, kBpThreads, 0, stream>>>(
       (float2*)d_volumeft, d_volumeweights, (const float2*)d_projft, d_projweights, d_mats, d_shifts, d_gweights,
       a, rmax, plan.fallback, plan.nfallback);
@@ -1195,7 +1238,7 @@ static int backproject_launch(float* d_volumeft, float* d_volumeweights, int vx,
                      (d_volumeft || d_volumeweights) &&
                      (choice == GTOMRLN_PATH_BRICK || choice == GTOMRLN_PATH_SEGMENT ||
                       choice == GTOMRLN_PATH_SEGMENT_FP32 ||
-                      (choice == GTOMRLN_PATH_AUTO && brick_path_pays(GTOMRLN_OP_BACKPROJECT, vx, batch)));
+                      (choice == GTOMRLN_PATH_AUTO && brick_path_pays(GTOMRLN_OP_BACKPROJECT, vx, (double)rmax, batch)));
   const bool fixed_point = choice != GTOMRLN_PATH_SEGMENT_FP32;
   if (brick && plain)
     return backproject_brick(d_volumeft, d_volumeweights, d_projft, d_projweights, d_matrices, a, (int)rmax,
@@ -1251,7 +1294,8 @@ static int backproject_launch(float* d_volumeft, float* d_volumeweights, int vx,
       launch_bp_direct_any<true>(grid, stream, (float2*)packed, nullptr, (const float2*)d_projft, d_projweights,
                                  d_matrices, d_ivolume, a, nullptr, nullptr, ndp, decentered, square);
       const unsigned blocks = (unsigned)std::min<int64_t>((voxels + 255) / 256, 148 * 16);
-      backproject_unpack_kernel<<<blocks, 256, 0, stream>>>(packed, (float2*)d_volumeft, d_volumeweights, voxels);
+      launch_dependent(backproject_unpack_kernel, blocks, 256, 0, stream, packed, (float2*)d_volumeft, d_volumeweights,
+                       voxels);
       if (e == cudaSuccess) e = cudaGetLastError();
       const int st = pool_free(packed, stream);
       if (e != cudaSuccess)
@@ -1353,7 +1397,7 @@ int gtomrln_backproject_shifted(float* d_volumeft, float* d_volumeweights, int v
   const int choice = path_choice(GTOMRLN_OP_BACKPROJECT);
   if (ndp == 2 && vx == vy && vx == vz && vx >= 4 && a.rmax2 <= (1 << 24) && (d_volumeft || d_volumeweights) &&
       (choice == GTOMRLN_PATH_BRICK || choice == GTOMRLN_PATH_SEGMENT ||
-       (choice == GTOMRLN_PATH_AUTO && brick_path_pays(GTOMRLN_OP_BACKPROJECT, vx, batch))))
+       (choice == GTOMRLN_PATH_AUTO && brick_path_pays(GTOMRLN_OP_BACKPROJECT, vx, (double)rmax, batch))))
     return backproject_shifted_brick(d_volumeft, d_volumeweights, d_projft, d_projweights, d_matrices, d_shifts,
                                      d_globalweights, a, (int)rmax, batch, (cudaStream_t)stream);
   dim3 grid((unsigned)(a.tiles * (int64_t)batch));

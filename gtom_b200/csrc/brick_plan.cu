@@ -268,15 +268,14 @@ bin_slices_kernel(const float* __restrict__ mats, BrickGrid g, PixelSet px, floa
 struct SegBin {
   int ss, rows, key, rank;  // as in SegRec; the volume-brick key and the bin's rank within it
 };
-constexpr int kPairThreads = 256;
+constexpr int kPairThreads = 128;
 __global__ void __launch_bounds__(kPairThreads)
-segment_pairs_kernel(const float* __restrict__ mats, BrickGrid g, float pmax, float limit,
+segment_pairs_kernel(const float* __restrict__ mats, BrickGrid g, float pmax, float limit, int list_cap,
                      SegBin* __restrict__ bins, int64_t bins_cap, unsigned long long* __restrict__ counters,
                      int* __restrict__ brick_pairs, int* __restrict__ fallback, int* __restrict__ nfallback,
                      float2* __restrict__ zero_out, PixelSet zpx, SliceGeom gm) {
-  extern __shared__ int hits[];  // brick ids of this slice, then a bitmap of the bricks
-  __shared__ int s_n, s_m, s_put;
-  __shared__ int s_wsum[kPairThreads / 32];
+  extern __shared__ int2 list[];  // the slice's records: {packed rows, 2 * brick + side}
+  __shared__ int s_m;
   __shared__ long long s_base;
   const int slice = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
   float m0[9], m[9];
@@ -292,6 +291,78 @@ segment_pairs_kernel(const float* __restrict__ mats, BrickGrid g, float pmax, fl
     if (tid == 0) fallback[atomicAdd(nfallback, 1)] = slice;
     return;
   }
+  if (tid == 0) s_m = 0;
+  __syncthreads();
+  const SegRows sr = seg_rows_setup(m, zpx);
+  const float half = 0.5f * (float)g.B, hw = half + widen + kSegMargin;
+  const float n0 = m[1] * m[5] - m[2] * m[4], n1 = m[2] * m[3] - m[0] * m[5], n2 = m[0] * m[4] - m[1] * m[3];
+  const float an0 = fabsf(n0), an1 = fabsf(n1), an2 = fabsf(n2);
+  const float R2 = R * R * (1.f + 1e-5f) + 1e-3f;
+  const float reach = (an0 + an1 + an2) * hw;
+  // Brick b: whether its widened box meets the slice's plane and the sphere
+  // of radius R, and then its sides that can hold rows of the slice.
+  auto test = [&](int b) {
+    const int3 o = brick_origin(g, b);
+    const float c0 = o.x + half, c1 = o.y + half, c2 = o.z + half;
+    const float dist = fabsf(n0 * c0 + n1 * c1 + n2 * c2);
+    const float eps = 1e-5f * (an0 * (fabsf(c0) + hw) + an1 * (fabsf(c1) + hw) + an2 * (fabsf(c2) + hw));
+    if (dist > reach + eps) return;  // (a NaN normal keeps every brick)
+    const float d0 = fmaxf(0.f, fabsf(c0) - hw), d1 = fmaxf(0.f, fabsf(c1) - hw), d2 = fmaxf(0.f, fabsf(c2) - hw);
+    if (!(d0 * d0 + d1 * d1 + d2 * d2 <= R2)) return;
+    int vlo[2], vhi[2];
+    seg_rows(sr, zpx, c0, c1, c2, hw, vlo, vhi);
+#pragma unroll
+    for (int side = 0; side < 2; side++)
+      if (vlo[side] <= vhi[side]) {
+        const int at = atomicAdd(&s_m, 1);
+        if (at < list_cap) list[at] = make_int2(seg_pack_rows(vlo[side], vhi[side]), 2 * b + side);
+      }
+  };
+  // Candidates: along the axis k where the normal is largest, a column of
+  // bricks (fixed indices on the other two axes) meets the plane only where
+  // the centre's k coordinate is within (reach + eps) / |n_k| of the plane's
+  // over the column; that range, widened well beyond the float error of the
+  // test, is searched with the exact test, so the hits are the ones testing
+  // every brick finds (in another order).  A zero or non-finite normal tests
+  // every brick.
+  const int k = an0 >= an1 && an0 >= an2 ? 0 : (an1 >= an2 ? 1 : 2);
+  const float ank = k == 0 ? an0 : (k == 1 ? an1 : an2);
+  if (ank > 1e-30f && isfinite(n0) && isfinite(n1) && isfinite(n2) && isfinite(R2)) {
+    const int nb[3] = {g.nbx, g.nby, g.nbz};
+    const float base[3] = {(float)g.xlo, (float)g.ylo, (float)g.zlo};
+    const float nv[3] = {n0, n1, n2};
+    const int i = k == 0 ? 1 : 0, j = k == 2 ? 1 : 2;  // the other two axes
+    // |c| <= extent of the grid on every axis: a bound on the test's eps
+    const float cmax = fmaxf(fmaxf((float)(g.nbx * g.B), fabsf(base[1])), fabsf(base[2])) +
+                       (float)(g.nby > g.nbz ? g.nby : g.nbz) * (float)g.B + hw;
+    const float slack = reach + 1e-5f * (an0 + an1 + an2) * (cmax + hw);
+    const float invB = 1.f / (float)g.B;
+    const int ncol = nb[i] * nb[j];
+    for (int col = tid; col < ncol; col += kPairThreads) {
+      const int bj = col / nb[i], ai = col - bj * nb[i];
+      const float ci = base[i] + (float)(ai * g.B) + half, cj = base[j] + (float)(bj * g.B) + half;
+      const float sp = nv[i] * ci + nv[j] * cj;
+      // centre k coordinate c with |n_k c + sp| <= slack
+      const float mid = -sp / nv[k], halfw = slack / ank;
+      const float margin = 1e-3f * (fabsf(mid) + halfw) + 0.01f * (float)g.B;
+      float flo = (mid - halfw - margin - base[k] - half) * invB;
+      float fhi = (mid + halfw + margin - base[k] - half) * invB;
+      if (!(flo <= fhi)) continue;
+      flo = fminf(fmaxf(flo, -1.f), (float)nb[k]);
+      fhi = fminf(fmaxf(fhi, -1.f), (float)nb[k]);
+      const int l0 = max(0, (int)floorf(flo)), l1 = min(nb[k] - 1, (int)ceilf(fhi));
+      for (int l = l0; l <= l1; l++) {
+        const int bx = k == 0 ? l : (i == 0 ? ai : bj), by = k == 1 ? l : (i == 1 ? ai : bj),
+                  bz = k == 2 ? l : bj;
+        test(bx + g.nbx * (by + g.nby * bz));
+      }
+    }
+  } else {
+    for (int b = tid; b < g.nbricks; b += kPairThreads) test(b);
+  }
+  __syncthreads();
+  const int nm = s_m;
+  if (tid == 0) s_base = (long long)atomicAdd(counters + 1, (unsigned long long)nm);
   if (zero_out) {
     // the projector's zeros outside rmax (Project.cu:111-115): in each row
     // the tail x > sqrt(rmax^2 - y^2), one warp per row (slices taking the
@@ -304,149 +375,18 @@ segment_pairs_kernel(const float* __restrict__ mats, BrickGrid g, float pmax, fl
       for (int x = x0 + lane; x < zpx.dimft; x += 32) out[(int64_t)idy * zpx.dimft + x] = make_float2(0.f, 0.f);
     }
   }
-  if (tid == 0) s_n = s_m = s_put = 0;
   __syncthreads();
-  const float n0 = m[1] * m[5] - m[2] * m[4], n1 = m[2] * m[3] - m[0] * m[5], n2 = m[0] * m[4] - m[1] * m[3];
-  const float R2 = R * R * (1.f + 1e-5f) + 1e-3f;
-  const float lo_pad = widen + kSegMargin, hi_pad = (float)g.B + widen + kSegMargin;
-  // The exact test of brick b: its widened box meets the slice's plane and
-  // the sphere of radius R.
-  auto crosses = [&](int b) {
-    const int3 o = brick_origin(g, b);
-    const float lo0 = o.x - lo_pad, lo1 = o.y - lo_pad, lo2 = o.z - lo_pad;
-    const float hi0 = o.x + hi_pad, hi1 = o.y + hi_pad, hi2 = o.z + hi_pad;
-    const float c0 = 0.5f * (lo0 + hi0), c1 = 0.5f * (lo1 + hi1), c2 = 0.5f * (lo2 + hi2);
-    const float h0 = 0.5f * (hi0 - lo0), h1 = 0.5f * (hi1 - lo1), h2 = 0.5f * (hi2 - lo2);
-    const float dist = fabsf(n0 * c0 + n1 * c1 + n2 * c2);
-    const float reach = fabsf(n0) * h0 + fabsf(n1) * h1 + fabsf(n2) * h2;
-    const float eps = 1e-5f * (fabsf(n0) * (fabsf(c0) + h0) + fabsf(n1) * (fabsf(c1) + h1) +
-                               fabsf(n2) * (fabsf(c2) + h2));
-    const float d0 = fmaxf(0.f, fmaxf(lo0, -hi0)), d1 = fmaxf(0.f, fmaxf(lo1, -hi1)),
-                d2 = fmaxf(0.f, fmaxf(lo2, -hi2));
-    return dist <= reach + eps && d0 * d0 + d1 * d1 + d2 * d2 <= R2;
-  };
-  // Candidates: along the axis k where the normal is largest, a column of
-  // bricks (fixed indices on the other two axes) meets the plane only where
-  // the centre's k coordinate is within (reach + eps) / |n_k| of the plane's
-  // over the column; that range, widened well beyond the float error of the
-  // test, is searched with the exact test, so the hits are the ones testing
-  // every brick finds (in another order).  A zero or non-finite normal tests
-  // every brick.
-  const float an0 = fabsf(n0), an1 = fabsf(n1), an2 = fabsf(n2);
-  const int k = an0 >= an1 && an0 >= an2 ? 0 : (an1 >= an2 ? 1 : 2);
-  const float ank = k == 0 ? an0 : (k == 1 ? an1 : an2);
-  const bool columns = ank > 1e-30f && isfinite(n0) && isfinite(n1) && isfinite(n2) && isfinite(R2);
-  if (columns) {
-    // hits marked in a bitmap, then listed in brick order (pairs_fill_kernel's
-    // per-brick atomics from consecutive bins then fall on neighbouring words)
-    unsigned* bits = reinterpret_cast<unsigned*>(hits + g.nbricks);
-    const int nwords = (g.nbricks + 31) / 32;
-    for (int w = tid; w < nwords; w += kPairThreads) bits[w] = 0u;
-    __syncthreads();
-    const int nb[3] = {g.nbx, g.nby, g.nbz};
-    const float base[3] = {(float)g.xlo, (float)g.ylo, (float)g.zlo};
-    const float nv[3] = {n0, n1, n2};
-    const int i = k == 0 ? 1 : 0, j = k == 2 ? 1 : 2;  // the other two axes
-    const float d = 0.5f * (hi_pad - lo_pad), h = 0.5f * (hi_pad + lo_pad);
-    const float reach = (an0 + an1 + an2) * h;
-    // |c| <= extent of the grid on every axis: a bound on the test's eps
-    const float cmax = fmaxf(fmaxf((float)(g.nbx * g.B), fabsf(base[1])), fabsf(base[2])) +
-                       (float)(g.nby > g.nbz ? g.nby : g.nbz) * (float)g.B + h;
-    const float slack = reach + 1e-5f * (an0 + an1 + an2) * (cmax + h);
-    const float invB = 1.f / (float)g.B;
-    const int ncol = nb[i] * nb[j];
-    for (int col = tid; col < ncol; col += kPairThreads) {
-      const int a = col % nb[i], bj = col / nb[i];
-      const float ci = base[i] + (float)(a * g.B) + d, cj = base[j] + (float)(bj * g.B) + d;
-      const float sp = nv[i] * ci + nv[j] * cj;
-      // centre k coordinate c with |n_k c + sp| <= slack
-      const float mid = -sp / nv[k], half = slack / ank;
-      const float margin = 1e-3f * (fabsf(mid) + half) + 0.01f * (float)g.B;
-      float flo = (mid - half - margin - base[k] - d) * invB;
-      float fhi = (mid + half + margin - base[k] - d) * invB;
-      if (!(flo <= fhi)) continue;
-      flo = fminf(fmaxf(flo, -1.f), (float)nb[k]);
-      fhi = fminf(fmaxf(fhi, -1.f), (float)nb[k]);
-      const int l0 = max(0, (int)floorf(flo)), l1 = min(nb[k] - 1, (int)ceilf(fhi));
-      for (int l = l0; l <= l1; l++) {
-        int idx[3];
-        idx[k] = l;
-        idx[i] = a;
-        idx[j] = bj;
-        const int b = idx[0] + g.nbx * (idx[1] + g.nby * idx[2]);
-        if (crosses(b)) atomicOr(bits + (b >> 5), 1u << (b & 31));
-      }
-    }
-    __syncthreads();
-    // thread t lists the set bits of words [t W, (t+1) W) at its offset in a
-    // block-wide scan of the words' counts
-    const int W = (nwords + kPairThreads - 1) / kPairThreads;
-    const int w0 = min(tid * W, nwords), w1 = min(w0 + W, nwords);
-    int cnt = 0;
-    for (int w = w0; w < w1; w++) cnt += __popc(bits[w]);
-    int incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t2 = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t2;
-    }
-    if (lane == 31) s_wsum[tid >> 5] = incl;
-    __syncthreads();
-    int pos = incl - cnt;
-    for (int k2 = 0; k2 < (tid >> 5); k2++) pos += s_wsum[k2];
-    for (int w = w0; w < w1; w++) {
-      unsigned m = bits[w];
-      while (m) {
-        hits[pos++] = 32 * w + __ffs(m) - 1;
-        m &= m - 1u;
-      }
-    }
-    if (tid == kPairThreads - 1) s_n = pos;
-  } else {
-    for (int base = 0; base < g.nbricks; base += kPairThreads) {
-      const int b = base + tid;
-      const bool hit = b < g.nbricks && crosses(b);
-      const unsigned mask = __ballot_sync(0xffffffffu, hit);
-      int wbase = 0;
-      if (lane == 0 && mask) wbase = atomicAdd(&s_n, __popc(mask));
-      wbase = __shfl_sync(0xffffffffu, wbase, 0);
-      if (hit) hits[wbase + __popc(mask & ((1u << lane) - 1u))] = b;
-    }
-  }
-  __syncthreads();
-  const int nh = s_n;
-  // The row range of each side of each hit brick (the box as the brick
-  // kernels build it), walked twice: counted, so that the slice reserves its
-  // bins with one atomic, then written.
-  const SegRows sr = seg_rows_setup(m, zpx);
-  const float half = 0.5f * (float)g.B, hw = half + widen + kSegMargin;
-  int mine = 0, vlo[2], vhi[2];
-  for (int k = tid; k < nh; k += kPairThreads) {
-    const int3 o = brick_origin(g, hits[k]);
-    seg_rows(sr, zpx, o.x + half, o.y + half, o.z + half, hw, vlo, vhi);
-    mine += (vlo[0] <= vhi[0]) + (vlo[1] <= vhi[1]);
-  }
-  for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-  if (lane == 0 && mine) atomicAdd(&s_m, mine);
-  __syncthreads();
-  const int nm = s_m;
-  if (tid == 0) s_base = (long long)atomicAdd(counters + 1, (unsigned long long)nm);
-  __syncthreads();
-  if (s_base + nm > bins_cap) {  // out of room: direct path
-    for (long long k = s_base + tid; k < s_base + nm && k < bins_cap; k += kPairThreads) bins[k].key = -1;
+  const int64_t at = s_base;
+  if (nm > list_cap || at + nm > bins_cap) {  // out of room: direct path
+    for (int64_t q = at + tid; q < at + nm && q < bins_cap; q += kPairThreads) bins[q].key = -1;
     if (tid == 0) fallback[atomicAdd(nfallback, 1)] = slice;
     return;
   }
-  for (int k = tid; k < nh; k += kPairThreads) {
-    const int local = hits[k];
-    const int3 o = brick_origin(g, local);
-    seg_rows(sr, zpx, o.x + half, o.y + half, o.z + half, hw, vlo, vhi);
-    const int b = vol * g.nbricks + local;
-#pragma unroll
-    for (int side = 0; side < 2; side++)
-      if (vlo[side] <= vhi[side])
-        reinterpret_cast<int4*>(bins)[s_base + atomicAdd(&s_put, 1)] = make_int4(
-            2 * slice + side, seg_pack_rows(vlo[side], vhi[side]), b, atomicAdd(brick_pairs + b, 1));
+  for (int q = tid; q < nm; q += kPairThreads) {
+    const int2 r = list[q];
+    const int b = vol * g.nbricks + (r.y >> 1);
+    reinterpret_cast<int4*>(bins)[at + q] =
+        make_int4(2 * slice + (r.y & 1), r.x, b, atomicAdd(brick_pairs + b, 1));
   }
 }
 
@@ -455,6 +395,7 @@ segment_pairs_kernel(const float* __restrict__ mats, BrickGrid g, float pmax, fl
 __global__ void segment_fill_kernel(const SegBin* __restrict__ bins, const float* __restrict__ mats,
                                     const unsigned long long* __restrict__ counters, int64_t bins_cap,
                                     const int* __restrict__ offsets, int negate, SegRec* __restrict__ recs) {
+  grid_dependency_wait();
   const int64_t nb = (int64_t)min(counters[1], (unsigned long long)bins_cap);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += (int64_t)gridDim.x * blockDim.x) {
     const int4 bn = __ldg(reinterpret_cast<const int4*>(bins) + i);
@@ -477,6 +418,7 @@ pairs_scan_kernel(const int* __restrict__ counts, const int* __restrict__ order,
   __shared__ int s_c[kScanThreads / 32], s_i[kScanThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int carry_c = 0, carry_i = 0;
+  grid_dependency_wait();
   // keys volume * nbricks + brick, the volumes interleaved brick by brick so
   // that every volume's central bricks start first
   const int nkeys = nbricks * nvol;
@@ -603,9 +545,6 @@ int build_brick_plan(int op, const float* d_mats, int batch, const BrickGrid& g,
   // pixel id of a slice: 66 KB at n = 256).
   const size_t code_bytes = ((size_t)px.elements * 2 + 3) & ~(size_t)3;
   const int use_codes = g.nbricks < 65535 && hist_bytes + code_bytes <= 200 * 1024 ? 1 : 0;
-  // segment plan: the hit list and a bitmap of the bricks
-  const size_t smem_bytes = segments ? sizeof(int) * ((size_t)g.nbricks + ((size_t)g.nbricks + 31) / 32)
-                                     : hist_bytes + (use_codes ? code_bytes : 0);
   const int* d_order = nullptr;
   int st = brick_order(g, &d_order);
   if (st) return st;
@@ -642,13 +581,19 @@ int build_brick_plan(int op, const float* d_mats, int batch, const BrickGrid& g,
     // central bricks, which every slice crosses, keep single CTAs busy after
     // the others have finished.  The backprojector's are not cut below 512,
     // where its extra flushes by reductions cost more than they even out, and
-    // on volumes that only a forced path brings here items stay whole.
+    // where only a forced path comes here (small volumes, small batches)
+    // items stay whole.
     const double share = 0.4 * est * batch / (8.0 * sms);
     if (op == GTOMRLN_OP_PROJECT)
       chunk = (int)std::min<double>(chunk, std::max(128.0, share));
-    else if (g.V >= 256)
+    else if (g.V >= 256 || batch >= 2000)
       chunk = (int)std::min<double>(chunk, std::max(512.0, share));
   }
+  // segment plan: a slice's records (twice the average reserved, for
+  // orientations that cross more bricks; a slice with still more takes the
+  // direct path)
+  const int list_cap = (int)std::min<int64_t>({2 * (int64_t)g.nbricks, 2 * (int64_t)per_slice, 12288});
+  const size_t smem_bytes = segments ? sizeof(int2) * (size_t)list_cap : hist_bytes + (use_codes ? code_bytes : 0);
   int64_t bins_cap = std::max<int64_t>(1, (int64_t)batch * per_slice);
   if (entries_cap > 0x7fffffffLL || bins_cap > 0x7fffffffLL)
     return set_error(GTOMRLN_ERR_INVALID, "brick plan too large for one call; split the batch");
@@ -696,7 +641,7 @@ int build_brick_plan(int op, const float* d_mats, int batch, const BrickGrid& g,
     if (segments) {
       cudaFuncSetAttribute(segment_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
       segment_pairs_kernel<<<batch, kPairThreads, smem_bytes, stream>>>(
-          d_mats, g, px.pmax, limit, seg_bins, bins_cap, counters, counts, plan->fallback,
+          d_mats, g, px.pmax, limit, list_cap, seg_bins, bins_cap, counters, counts, plan->fallback,
           plan->nfallback, (float2*)zero_out, px, geom);
     } else if (op == GTOMRLN_OP_PROJECT) {
       cudaFuncSetAttribute(bin_slices_kernel<GTOMRLN_OP_PROJECT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -711,11 +656,11 @@ int build_brick_plan(int op, const float* d_mats, int batch, const BrickGrid& g,
           d_mats, g, px, limit, plan->entries, entries_cap, plan->bins, bins_cap, counters, counts,
           plan->fallback, plan->nfallback, use_codes);
     }
-    pairs_scan_kernel<<<1, kScanThreads, 0, stream>>>(counts, d_order, g.nbricks, geom.nvol, chunk, offsets,
-                                                      plan->items, cursor, plan->nitems);
+    launch_dependent(pairs_scan_kernel, 1, kScanThreads, 0, stream, counts, d_order, g.nbricks, geom.nvol, chunk,
+                     offsets, plan->items, cursor, plan->nitems);
     if (segments)
-      segment_fill_kernel<<<sms * 8, 256, 0, stream>>>(seg_bins, d_mats, counters, bins_cap, offsets, geom.negate,
-                                                       plan->recs);
+      launch_dependent(segment_fill_kernel, sms * 8, 256, 0, stream, seg_bins, d_mats, counters, bins_cap, offsets,
+                       geom.negate, plan->recs);
     else
       pairs_fill_kernel<<<sms * 4, 256, 0, stream>>>(plan->bins, counters, bins_cap, counts, offsets, cursor,
                                                      plan->pairs);

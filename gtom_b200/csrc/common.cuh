@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/gtomrln.h"
@@ -48,12 +49,11 @@ void matrices_from_angles(const float* angles, float supersample, unsigned batch
 int path_choice(int op);
 
 // Whether GTOMRLN_PATH_AUTO takes the brick-major (row-segment) kernels for
-// op on a cubic volume of edge V and a batch of 2D slices: they win once the
-// volume no longer fits in L2 and the batch amortises their plan, while the
-// direct kernels, whose gathers and reductions then stay in L2, win on
-// smaller volumes.  Thresholds from a B200 sweep of boxes 32-256 (V = 2n
-// or 2n + 1) and batches 100-10 000 (abi.cu).
-bool brick_path_pays(int op, int V, unsigned batch);
+// op on a cubic volume of edge V and a batch of 2D slices of radius rmax:
+// they win once the volume no longer fits in L2 and the samples amortise
+// their plan and the bricks' staging, while the direct kernels, whose
+// gathers and reductions then stay in L2, win on smaller work (abi.cu).
+bool brick_path_pays(int op, int V, double rmax, unsigned batch);
 
 // Launch shape of the brick kernels for op: brick edge in voxels, threads
 // per CTA, and the most slices one work item takes (gtomrln_set_brick_tuning).
@@ -110,7 +110,34 @@ inline cudaError_t upload_host_floats(float* dst, size_t count, cudaStream_t str
   return cudaMemcpyAsync(dst, h.data(), count * sizeof(float), cudaMemcpyHostToDevice, stream);
 }
 
+// Launches a kernel that may start while the one before it on the stream
+// drains (programmatic dependent launch): the kernel must call
+// grid_dependency_wait() before it touches anything its predecessors write.
+template <class... P, class... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream,
+                                    A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
 // ---------------------------------------------------------------- device --
+// In a kernel of launch_dependent: lets the next kernel's CTAs take the SMs'
+// free slots from now on (they wait in turn), and waits until the kernels
+// before this one have completed and their writes are visible.
+__device__ __forceinline__ void grid_dependency_wait() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 struct Mat3 {
   float m[9];  // column-major, as glm::mat3
 };

@@ -160,6 +160,7 @@ __global__ void __launch_bounds__(kProjThreads)
 project_listed_kernel(ArrayFetch fetch, float2* __restrict__ proj, const float* __restrict__ mats,
                       ProjArgs a, const int* __restrict__ list, const int* __restrict__ nlist,
                       Post post = Post()) {
+  grid_dependency_wait();
   const int64_t total = (int64_t)(*nlist) * a.tiles;
   for (int64_t w = blockIdx.x; w < total; w += gridDim.x)
     project_direct_tile<2>(fetch, proj, mats, a, __ldg(list + w / a.tiles), (int)(w % a.tiles), post);
@@ -270,6 +271,7 @@ project_segment_kernel(const float2* __restrict__ vol, float2* __restrict__ proj
                        const SegRec* __restrict__ recs, int* __restrict__ counter, Post post = Post()) {
   extern __shared__ float4 smem4[];  // record slots, then the brick
   __shared__ int item_s, next_s;
+  grid_dependency_wait();
   const int nitems = *nitems_ptr;
   const int B = EDGE ? EDGE : g.B, T = B + 1;
   const ProjPitch pitch = proj_pitch(EDGE);
@@ -414,16 +416,15 @@ static int project_brick(const float* d_volumeft, float* d_proj, const float* d_
     project_zero_kernel<<<sms * 8, 256, 0, stream>>>((float2*)d_proj, a, rows);
   }
   if (segments)
-    kern<<<sms * std::max(occ, 1), tune.threads, smem, stream>>>(
-        (const float2*)d_volumeft, (float2*)d_proj, a, g, px, plan.items, plan.nitems, plan.recs, plan.counter,
-        post);
+    launch_dependent(kern, sms * std::max(occ, 1), tune.threads, smem, stream, (const float2*)d_volumeft,
+                     (float2*)d_proj, a, g, px, plan.items, plan.nitems, plan.recs, plan.counter, post);
   else
     project_brick_kernel<<<sms * std::max(occ, 1), tune.threads, smem, stream>>>(
         (const float2*)d_volumeft, (float2*)d_proj, d_mats, a, g, plan.items, plan.nitems, plan.pairs, plan.bins,
         plan.entries, plan.counter);
   ArrayFetch f{(const float2*)d_volumeft, a.P, a.P / 2 + 1, a.nvox - 1};
-  project_listed_kernel<Post><<<sms * 4, kProjThreads, 0, stream>>>(f, (float2*)d_proj, d_mats, a, plan.fallback,
-                                                                     plan.nfallback, post);
+  launch_dependent(project_listed_kernel<Post>, sms * 4, kProjThreads, 0, stream, f, (float2*)d_proj, d_mats, a,
+                   plan.fallback, plan.nfallback, post);
   e = cudaGetLastError();
   free_brick_plan(&plan, stream);
   if (e != cudaSuccess)
@@ -559,7 +560,7 @@ int gtomrln_project(const float* d_volumeft, int vx, int vy, int vz, float* d_pr
   // the brick plans' integer square roots take radii below 4 096 (seg_isqrt)
   if (ndp == 2 && vx == vy && vx == vz && vx >= 4 && a.rmax2 <= (1 << 24) &&
       (choice == GTOMRLN_PATH_BRICK || choice == GTOMRLN_PATH_SEGMENT ||
-       (choice == GTOMRLN_PATH_AUTO && brick_path_pays(GTOMRLN_OP_PROJECT, vx, batch))))
+       (choice == GTOMRLN_PATH_AUTO && brick_path_pays(GTOMRLN_OP_PROJECT, vx, (double)a.rmax, batch))))
     return project_brick(d_volumeft, d_proj, d_matrices, a, batch, (cudaStream_t)stream,
                          choice == GTOMRLN_PATH_BRICK ? 0 : 1);
   ArrayFetch f{(const float2*)d_volumeft, a.P, a.P / 2 + 1, a.nvox - 1};
@@ -620,7 +621,7 @@ int gtomrln_project_shifted(const float* d_volumeft, int vx, int vy, int vz, flo
   // the brick plans' integer square roots take radii below 4 096 (seg_isqrt)
   if (ndp == 2 && vx == vy && vx == vz && vx >= 4 && a.rmax2 <= (1 << 24) &&
       (choice == GTOMRLN_PATH_BRICK || choice == GTOMRLN_PATH_SEGMENT ||
-       (choice == GTOMRLN_PATH_AUTO && brick_path_pays(GTOMRLN_OP_PROJECT, vx, batch))))
+       (choice == GTOMRLN_PATH_AUTO && brick_path_pays(GTOMRLN_OP_PROJECT, vx, (double)a.rmax, batch))))
     return project_brick(d_volumeft, d_proj, d_matrices, a, batch, (cudaStream_t)stream, 1,
                          ShiftPost{d_shifts, d_globalweights});
   ArrayFetch f{(const float2*)d_volumeft, a.P, a.P / 2 + 1, a.nvox - 1};
