@@ -117,12 +117,10 @@ __device__ __forceinline__ void split4(float4 v, float4& hi, float4& lo) {
   lo = make_float4(v.x - hi.x, v.y - hi.y, v.z - hi.z, v.w - hi.w);
 }
 
-// Two consecutive complex elements of a row, zero past the end.  vec: rows
-// start on 16-byte boundaries.
-__device__ __forceinline__ float4 load2(const float2* __restrict__ row, int64_t i, int64_t end, bool vec) {
-  if (vec && i + 1 < end) return __ldg(reinterpret_cast<const float4*>(row + i));
-  const float2 a = i < end ? __ldg(row + i) : make_float2(0.f, 0.f);
-  const float2 b = i + 1 < end ? __ldg(row + i + 1) : make_float2(0.f, 0.f);
+// Two consecutive complex elements, of which `left` exist.
+__device__ __forceinline__ float4 load2(const float2* __restrict__ p, int64_t left) {
+  const float2 a = left > 0 ? __ldg(p) : make_float2(0.f, 0.f);
+  const float2 b = left > 1 ? __ldg(p + 1) : make_float2(0.f, 0.f);
   return make_float4(a.x, a.y, b.x, b.y);
 }
 
@@ -135,10 +133,24 @@ struct TcArgs {
   const float2* refs;
   unsigned nparticles, nrefs, nshifts;
   int mtiles, ntiles, splits, cc, vec;
+  float2* ps;   // sqrt(w) particle, as particle
+  float* cs;    // sqrt(w) ctf: [particle][element]
   float* part;  // C: [split][particle][ref][shift]
   float* sa;    // A: [split][particle][ref]
   float* sb;    // B: [split][particle][shift]
 };
+
+// The per-particle factors of the operands (sqrt(w) = 1 for the
+// cross-correlation).
+__global__ void __launch_bounds__(256) diff2_tc_scale_kernel(const TcArgs a) {
+  const int64_t n = a.elements * a.nparticles;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const float w = a.cc || !a.minvsigma2 ? 1.f : sqrtf(__ldg(a.minvsigma2 + i % a.elements));
+    const float2 v = __ldg(a.particle + i);
+    a.ps[i] = make_float2(v.x * w, v.y * w);
+    a.cs[i] = (a.ctf ? __ldg(a.ctf + i) : 1.f) * w;
+  }
+}
 
 __global__ void __launch_bounds__(kThreads, 2) diff2_tc_kernel(const TcArgs a) {
   extern __shared__ unsigned char raw[];
@@ -175,44 +187,52 @@ __global__ void __launch_bounds__(kThreads, 2) diff2_tc_kernel(const TcArgs a) {
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const unsigned tmem = tmem_s;
+  grid_dependency_wait();
 
   // thread -> 16-byte unit j (two elements) of rows row0 + 32 k
   const int j = tid & 7, row0 = tid >> 3;
   const unsigned swz = (unsigned)((j ^ (row0 & 7)) << 4) + (unsigned)(row0 & 7) * 128 + (unsigned)(row0 >> 3) * 1024;
-  const float2* pp = a.particle + a.elements * p;
-  const float* cp = a.ctf ? a.ctf + a.elements * p : nullptr;
+  const float2* pp = a.ps + a.elements * p;
+  const float* cp = a.cs + a.elements * p;
   float sa[4] = {0.f, 0.f, 0.f, 0.f}, sb[2] = {0.f, 0.f};
   float acc[32];
 #pragma unroll
   for (int i = 0; i < 32; i++) acc[i] = 0.f;
 
-  float4 rv[4], sv[2], pv;
-  float cs[2];
-  auto fetch = [&](int t) {  // the raw operands of chunk t
-    const int64_t i = (c0 + t) * kE + 2 * j;
+  struct Raw {  // the raw operands of a chunk
+    float4 rv[4], sv[2], pv;
+    float cs[2];
+  };
+  // the thread's places in its first rows, and which of its rows exist
+  const int64_t at0 = c0 * kE + 2 * j, pitch = 32 * a.elements;
+  const float2* rrow = a.refs + a.elements * (r0 + row0) + at0;
+  const float2* srow = a.shifts + a.elements * (s0 + row0) + at0;
+  const float2* prow = pp + at0;
+  const float* crow = cp + at0;
+  const int nr = r0 + row0 < a.nrefs ? min(4u, (a.nrefs - r0 - row0 + 31) / 32) : 0;
+  const int ns = s0 + row0 < a.nshifts ? min(2u, (a.nshifts - s0 - row0 + 31) / 32) : 0;
+  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto fetch = [&](Raw& q, int t) {
+    const int i = t * kE;
+    if (a.vec && (c0 + t + 1) * kE <= end) {  // a whole chunk of 16-byte aligned rows
+      auto load = [&](const float2* p4) { return __ldg(reinterpret_cast<const float4*>(p4 + i)); };
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const unsigned r = r0 + row0 + 32 * k;
-      rv[k] = r < a.nrefs ? load2(a.refs + a.elements * r, i, end, a.vec) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
+      for (int k = 0; k < 4; k++) q.rv[k] = k < nr ? load(rrow + k * pitch) : zero4;
 #pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const unsigned s = s0 + row0 + 32 * k;
-      sv[k] = s < a.nshifts ? load2(a.shifts + a.elements * s, i, end, a.vec) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    pv = load2(pp, i, end, a.vec);
+      for (int k = 0; k < 2; k++) q.sv[k] = k < ns ? load(srow + k * pitch) : zero4;
+      q.pv = load(prow);
+      const float2 cv = __ldg(reinterpret_cast<const float2*>(crow + i));
+      q.cs[0] = cv.x;
+      q.cs[1] = cv.y;
+    } else {
+      const int64_t left = end - at0 - i;  // elements from this thread's first on
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const bool in = i + h < end;
-      const float w = a.cc || !a.minvsigma2 || !in ? 1.f : sqrtf(__ldg(a.minvsigma2 + i + h));
-      cs[h] = (cp && in ? __ldg(cp + i + h) : 1.f) * w;
-      if (h == 0) {
-        pv.x *= w;
-        pv.y *= w;
-      } else {
-        pv.z *= w;
-        pv.w *= w;
-      }
+      for (int k = 0; k < 4; k++) q.rv[k] = k < nr ? load2(rrow + k * pitch + i, left) : zero4;
+#pragma unroll
+      for (int k = 0; k < 2; k++) q.sv[k] = k < ns ? load2(srow + k * pitch + i, left) : zero4;
+      q.pv = load2(prow + i, left);
+#pragma unroll
+      for (int h = 0; h < 2; h++) q.cs[h] = h < left ? __ldg(crow + i + h) : 0.f;
     }
   };
   // warps 0-3 drain columns 0-31 of their lanes' rows, warps 4-7 the others
@@ -226,21 +246,22 @@ __global__ void __launch_bounds__(kThreads, 2) diff2_tc_kernel(const TcArgs a) {
 
   bool ok = true;
   int drained = 0;
-  if (nch > 0) fetch(0);
-  for (int t = 0; t < nch; t++) {
+  // chunk t from its raw operands, which are then those of chunk t + 2 (two
+  // chunks ahead: one does not cover the loads' latency)
+  auto step = [&](Raw& q, int t) {
     const int s = t & 1;
     if (t >= 2) {  // the stage's earlier matrix instructions are done
       const bool w = bar_wait(smem_u32(&bars[s]), (unsigned)((t >> 1) - 1) & 1u);
       if (!__syncthreads_and(w)) {
         ok = false;
-        break;
+        return;
       }
       if (t % kGroup == 1) drain(drained++);  // and with chunk t - 2 its accumulator set
     }
     unsigned char* st = stage0 + s * kStageBytes;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      const float4 v = make_float4(rv[k].x * cs[0], rv[k].y * cs[0], rv[k].z * cs[1], rv[k].w * cs[1]);
+      const float4 v = make_float4(q.rv[k].x * q.cs[0], q.rv[k].y * q.cs[0], q.rv[k].z * q.cs[1], q.rv[k].w * q.cs[1]);
       sa[k] = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, sa[k]))));
       float4 hi, lo;
       split4(v, hi, lo);
@@ -249,8 +270,8 @@ __global__ void __launch_bounds__(kThreads, 2) diff2_tc_kernel(const TcArgs a) {
     }
 #pragma unroll
     for (int k = 0; k < 2; k++) {
-      const float4 v = make_float4(pv.x * sv[k].x - pv.y * sv[k].y, pv.x * sv[k].y + pv.y * sv[k].x,
-                                   pv.z * sv[k].z - pv.w * sv[k].w, pv.z * sv[k].w + pv.w * sv[k].z);
+      const float4 v = make_float4(q.pv.x * q.sv[k].x - q.pv.y * q.sv[k].y, q.pv.x * q.sv[k].y + q.pv.y * q.sv[k].x,
+                                   q.pv.z * q.sv[k].z - q.pv.w * q.sv[k].w, q.pv.z * q.sv[k].w + q.pv.w * q.sv[k].z);
       sb[k] = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, sb[k]))));
       float4 hi, lo;
       split4(v, hi, lo);
@@ -277,7 +298,14 @@ __global__ void __launch_bounds__(kThreads, 2) diff2_tc_kernel(const TcArgs a) {
                        smem_u32(&bars[s]))
                    : "memory");
     }
-    if (t + 1 < nch) fetch(t + 1);
+    if (t + 2 < nch) fetch(q, t + 2);
+  };
+  Raw q0, q1;
+  if (nch > 0) fetch(q0, 0);
+  if (nch > 1) fetch(q1, 1);
+  for (int t = 0; t < nch && ok; t += 2) {
+    step(q0, t);
+    if (t + 1 < nch && ok) step(q1, t + 1);
   }
   // the last commit covers everything issued before it
   if (nch > 0 && ok) {
@@ -331,6 +359,7 @@ __global__ void __launch_bounds__(kThreads, 2) diff2_tc_kernel(const TcArgs a) {
 __global__ void __launch_bounds__(256)
 diff2_tc_combine_kernel(const TcArgs a, float* __restrict__ diff2, int* __restrict__ flags) {
   const int64_t n = (int64_t)a.nparticles * a.nrefs * a.nshifts;
+  grid_dependency_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t pr = i / a.nshifts;
     const unsigned s = (unsigned)(i - pr * a.nshifts);
@@ -370,7 +399,7 @@ int diff2_tensor(const float2* particle, const float* minvsigma2, const float* c
   a.mtiles = (int)((nrefs + kM - 1) / kM);
   a.ntiles = (int)((nshifts + kN - 1) / kN);
   a.cc = cc ? 1 : 0;
-  a.vec = elements % 2 == 0 && ((uintptr_t)particle | (uintptr_t)shifts | (uintptr_t)refs) % 16 == 0;
+  a.vec = elements % 2 == 0 && ((uintptr_t)shifts | (uintptr_t)refs) % 16 == 0;
   int dev = 0, sms = 148;
   GTOMRLN_CUDA_TRY(cudaGetDevice(&dev));
   GTOMRLN_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -392,13 +421,16 @@ int diff2_tensor(const float2* particle, const float* minvsigma2, const float* c
   const size_t tiles = (size_t)nparticles * ((nrefs + kDiffTile - 1) / kDiffTile) * ((nshifts + kDiffTile - 1) / kDiffTile);
   if (units * a.splits > 0x7fffffffLL) return set_error(GTOMRLN_ERR_INVALID, "squared differences: too many tiles");
   const size_t nsa = (size_t)nparticles * nrefs * a.splits, nsb = (size_t)nparticles * nshifts * a.splits;
+  const size_t npe = (size_t)nparticles * (size_t)elements;
   float* scratch = nullptr;
-  if (pool_alloc((void**)&scratch, sizeof(float) * ((size_t)n * a.splits + nsa + nsb + tiles), stream)) {
+  if (pool_alloc((void**)&scratch, sizeof(float) * (3 * npe + (size_t)n * a.splits + nsa + nsb + tiles), stream)) {
     clear_error();  // no room for the partial products: the direct kernel needs none
     return diff2_direct(particle, minvsigma2, ctf, elements, shifts, refs, diff2, nparticles, nrefs, nshifts, cc,
                         nullptr, stream);
   }
-  a.part = scratch;
+  a.ps = reinterpret_cast<float2*>(scratch);  // (pool allocations are 256-byte aligned)
+  a.cs = scratch + 2 * npe;
+  a.part = a.cs + npe;
   a.sa = a.part + (size_t)n * a.splits;
   a.sb = a.sa + nsa;
   int* flags = reinterpret_cast<int*>(a.sb + nsb);
@@ -406,9 +438,10 @@ int diff2_tensor(const float2* particle, const float* minvsigma2, const float* c
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(diff2_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
   if (e == cudaSuccess) {
-    diff2_tc_kernel<<<(unsigned)(units * a.splits), kThreads, kSmem, stream>>>(a);
-    diff2_tc_combine_kernel<<<(unsigned)std::min<int64_t>((n + 255) / 256, 16 * sms), 256, 0, stream>>>(a, diff2,
-                                                                                                      flags);
+    diff2_tc_scale_kernel<<<(unsigned)std::min<size_t>((npe + 255) / 256, 8 * (size_t)sms), 256, 0, stream>>>(a);
+    launch_dependent(diff2_tc_kernel, (unsigned)(units * a.splits), kThreads, kSmem, stream, a);
+    launch_dependent(diff2_tc_combine_kernel, (unsigned)std::min<int64_t>((n + 255) / 256, 16 * sms), 256, 0, stream, a,
+                     diff2, flags);
     e = cudaGetLastError();
   }
   int st = GTOMRLN_OK;

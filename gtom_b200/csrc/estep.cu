@@ -138,6 +138,7 @@ diff2_dense_tiled_kernel(const float2* __restrict__ particle, const float* __res
                          const float* __restrict__ ctf, int64_t elements, const float2* __restrict__ shifts,
                          const float2* __restrict__ refs, float* __restrict__ diff2, unsigned nrefs,
                          unsigned nshifts, const int* __restrict__ flags) {
+  grid_dependency_wait();
   if (flags && !flags[((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x]) return;
   __shared__ float2 As[kDK][kDT + 1];  // c * ref
   __shared__ float2 Bs[kDK][kDT + 1];  // particle * shift
@@ -405,11 +406,11 @@ int diff2_direct(const float2* particle, const float* minvsigma2, const float* c
                  unsigned nshifts, bool cc, const int* flags, cudaStream_t stream) {
   const dim3 grid((nshifts + kDT - 1) / kDT, (nrefs + kDT - 1) / kDT, nparticles);
   if (cc)
-    diff2_dense_tiled_kernel<true><<<grid, kDThreads, 0, stream>>>(particle, minvsigma2, ctf, elements, shifts, refs,
-                                                                   diff2, nrefs, nshifts, flags);
+    launch_dependent(diff2_dense_tiled_kernel<true>, grid, kDThreads, 0, stream, particle, minvsigma2, ctf, elements,
+                     shifts, refs, diff2, nrefs, nshifts, flags);
   else
-    diff2_dense_tiled_kernel<false><<<grid, kDThreads, 0, stream>>>(particle, minvsigma2, ctf, elements, shifts, refs,
-                                                                    diff2, nrefs, nshifts, flags);
+    launch_dependent(diff2_dense_tiled_kernel<false>, grid, kDThreads, 0, stream, particle, minvsigma2, ctf, elements,
+                     shifts, refs, diff2, nrefs, nshifts, flags);
   GTOMRLN_LAUNCH_CHECK("diff2_dense_tiled_kernel");
   return GTOMRLN_OK;
 }
