@@ -413,6 +413,7 @@ int release_ctf_plans(int dev, unsigned long long ctx);        // ctf.cu
 int release_brick_orders(int dev, unsigned long long ctx);     // brick_plan.cu
 int release_gridfft_tables(int dev, unsigned long long ctx);   // gridfft.cu
 int release_gridsym_caches(int dev, unsigned long long ctx);   // gridsym.cu
+int release_gridgen_caches(int dev, unsigned long long ctx);   // gridgen.cu
 
 static std::atomic<int> g_path[3] = {{GTOMRLN_PATH_AUTO}, {GTOMRLN_PATH_AUTO}, {GTOMRLN_PATH_AUTO}};
 
@@ -424,9 +425,9 @@ int path_choice(int op) { return (op >= 0 && op <= 2) ? g_path[op].load() : GTOM
 //                1 000: 318 vs 330, 3 000: 901 vs 640; n = 160: 1 000: 193 vs
 //                251, 3 000: 531 vs 505; n = 128: 3 000: 341 vs 396, 10 000:
 //                1 068 vs 898; n = 96, 10 000: 610 vs 645;
-// backprojector  n = 256: 100 slices 664 vs 851, 300: 1 769 vs 976; n = 192:
+// backprojector  n = 256: 100 slices 655 vs 750, 150: 921 vs 784; n = 192:
 //                100: 302 vs 408, 300: 773 vs 464; n = 160: 100: 170 vs 268,
-//                300: 388 vs 308; n = 128: 300: 187 vs 210, 1 000: 401 vs 315;
+//                300: 388 vs 308; n = 128: 300: 177 vs 210, 450: 248 vs 206;
 //                n = 96, 3 000: 477 vs 410; n = 64: 3 000: 240 vs 243, 10 000:
 //                670 vs 543; n = 48, 10 000: 407 vs 395 (below V = 321 the
 //                direct kernel reduces into a packed scratch).
@@ -435,7 +436,7 @@ int path_choice(int op) { return (op >= 0 && op <= 2) ? g_path[op].load() : GTOM
 bool brick_path_pays(int op, int V, double rmax, unsigned batch) {
   const double samples = 1.5707963 * rmax * rmax * batch;
   if (op == GTOMRLN_OP_BACKPROJECT)
-    return V >= 256 ? samples >= 2.5e6 : V >= 128 && batch >= 2000 && samples >= 6e6;
+    return V >= 256 ? samples >= (V >= 448 ? 3.1e6 : 2.5e6) : V >= 128 && batch >= 2000 && samples >= 6e6;
   return samples >= (V >= 512 ? 11e6 : V >= 384 ? 19e6 : V >= 320 ? 24e6 : V >= 256 ? 28e6 : 1e300);
 }
 
@@ -472,6 +473,7 @@ int gtomrln_release_caches(void) {
   if (!st) st = release_brick_orders(dev, ctx);
   if (!st) st = release_gridfft_tables(dev, ctx);
   if (!st) st = release_gridsym_caches(dev, ctx);
+  if (!st) st = release_gridgen_caches(dev, ctx);
   if (!st) st = release_scratch(dev, ctx);
   if (st) return st;
   release_stage(dev, ctx);

@@ -110,9 +110,13 @@ inline cudaError_t upload_host_floats(float* dst, size_t count, cudaStream_t str
   return cudaMemcpyAsync(dst, h.data(), count * sizeof(float), cudaMemcpyHostToDevice, stream);
 }
 
-// Launches a kernel that may start while the one before it on the stream
-// drains (programmatic dependent launch): the kernel must call
+// Launches a kernel under programmatic dependent launch: its launch overhead
+// runs under the one before it on the stream.  The kernel must call
 // grid_dependency_wait() before it touches anything its predecessors write.
+// No kernel lets its successor start early (griddepcontrol.launch_dependents):
+// waiting CTAs hold slots that the running grid's next CTAs need.  Ten
+// iterations at P = 512: 6.34 ms, 7.38 with the early start, 6.41 with plain
+// launches; at P = 64, 223, 270 and 300 us.
 template <class... P, class... A>
 inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream,
                                     A&&... args) {
@@ -130,11 +134,9 @@ inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, int threads
 }
 
 // ---------------------------------------------------------------- device --
-// In a kernel of launch_dependent: lets the next kernel's CTAs take the SMs'
-// free slots from now on (they wait in turn), and waits until the kernels
-// before this one have completed and their writes are visible.
+// In a kernel of launch_dependent: waits until the kernels before this one
+// have completed and their writes are visible.
 __device__ __forceinline__ void grid_dependency_wait() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 

@@ -43,12 +43,15 @@ double kaiser_fourier_value(double w, double a, double alpha, int m);  // below
 // (RecFourier.cu:287-291).  old* are the centred input dims.
 // One warp per (y, z) row of the P grid (lanes along x; grid (rows / 8,
 // volumes), 256 threads): the row's decentring and radii once, no index
-// divisions per element.
+// divisions per element.  sphere_only: the zeros outside the mask's sphere
+// (48 % of the grid) are left unwritten, for the symmetric path, which reads
+// weights inside it only, but for Fnw[P/2] (x = P/2 lies outside): the final
+// map's flag (gridsym_final_z_kernel).
 constexpr int kInitWarps = 8;
 __global__ void __launch_bounds__(32 * kInitWarps)
 grid_init_kernel(const float* __restrict__ weight, int oldx, int oldy, int oldz, float* __restrict__ Fw,
                  float* __restrict__ Fnw, float2* __restrict__ convft, GridGeom g, int maskr2, int write_conv,
-                 int64_t wstride) {
+                 int64_t wstride, int sphere_only) {
   const int64_t b = blockIdx.y;  // volume of a batch (stacks of equal volumes)
   weight += b * wstride;
   Fw += b * g.nc;
@@ -65,9 +68,11 @@ grid_init_kernel(const float* __restrict__ weight, int oldx, int oldy, int oldz,
   const float* wrow = weight + (in_yz ? ((int64_t)zi * oldy + yi) * (oldx / 2 + 1) : 0);
   const int64_t base = (int64_t)row * g.rowlen;
   const int yz2 = yp * yp + zp * zp;
+  if (sphere_only && row == 0 && lane == 0) Fnw[g.P / 2] = 0.f;
   for (int x = lane; x < g.rowlen; x += 32) {
     const float rr = r + (float)(x * x);
     const float mask = rr < (float)(g.P * g.P / 4) ? 1.f : 0.f;
+    if (sphere_only && mask == 0.f) break;  // zeros from here on, which nothing reads
     float w = 0.f;
     if (in_yz && x < oldx / 2 + 1) w = __ldg(wrow + x) * mask;
     Fw[base + x] = w;
@@ -443,6 +448,7 @@ static int reconstruct(const float* d_dataft, const float* d_weight, float* d_ou
   g.nr = (int64_t)P * P * P;
   int r_max = ori / 2;
   int maskr2 = (r_max * pad) * (r_max * pad);
+  g.maskr2 = maskr2;
 
   const float* table = nullptr;
   int st = get_table(radius * pad, alpha, order, &table);
@@ -465,13 +471,16 @@ static int reconstruct(const float* d_dataft, const float* d_weight, float* d_ou
   const int T = 256;
   unsigned bc = (unsigned)((g.nc + T - 1) / T);
   const unsigned init_blocks = (unsigned)((P * P + kInitWarps - 1) / kInitWarps);
-  // The symmetric-spectrum iteration (gridsym.cu; default on power-of-two
-  // grids P = 64 .. 512) or, when the caller chose it, the fused FFT
+  // The symmetric-spectrum iteration (gridsym.cu, gridgen.cu; the default on
+  // the grids they take) or, when the caller chose it, the fused FFT
   // iteration (gridfft.cu); cuFFT transforms otherwise and for the final map.
   const int gpath = path_choice(GTOMRLN_OP_GRIDDING);
   const bool sym = (gpath == GTOMRLN_PATH_SYMMETRIC || gpath == GTOMRLN_PATH_AUTO) && gridsym_available(P);
   const bool fused = !sym && gpath == GTOMRLN_PATH_FUSED && !measure_ref && gridfft_available(P, 1);
   bool need_first = true;  // both start with a transform along z
+  // (a predicted start reads neighbours outside the sphere, momentum copies
+  // the whole grid, and the caller's copies hold it)
+  const int sphere_only = sym && !warm && !momentum && !opt.out_fw && !opt.out_fnw;
   if (!sym) {  // the symmetric path makes the final map with its own transforms too
     if (!planf || !planb) GTOMRLN_STEP(get_plans(P, &plans));
     if (planf) plans.r2c = planf;
@@ -494,8 +503,8 @@ static int reconstruct(const float* d_dataft, const float* d_weight, float* d_ou
 
   // the first iteration's spectrum Fw * Fnw: the cuFFT and fused loops read
   // it; the symmetric loop makes its own first transform from Fw and Fnw
-  grid_init_kernel<<<init_blocks, 32 * kInitWarps, 0, stream>>>(d_weight, oldx, oldy, oldz, Fw, Fnw, convft, g,
-                                                                maskr2, iterations > 0 && !warm && !sym, 0);
+  grid_init_kernel<<<init_blocks, 32 * kInitWarps, 0, stream>>>(d_weight, oldx, oldy, oldz, Fw, Fnw, convft, g, maskr2,
+                                                                iterations > 0 && !warm && !sym, 0, sphere_only);
   GTOMRLN_STEP(launch_check("grid_init_kernel"));
   if (warm) {
     GTOMRLN_CUDA_TRY(cudaMemsetAsync(sums, 0, 2 * sizeof(double), stream));
@@ -543,7 +552,7 @@ static int reconstruct(const float* d_dataft, const float* d_weight, float* d_ou
         if (!(last_change <= (double)opt.residual_limit)) {
           // Rejected predicted start: the cold start (sphere mask) from scratch.
           grid_init_kernel<<<init_blocks, 32 * kInitWarps, 0, stream>>>(d_weight, oldx, oldy, oldz, Fw, Fnw,
-                                                                        convft, g, maskr2, !sym, 0);
+                                                                        convft, g, maskr2, !sym, 0, sphere_only);
           GTOMRLN_STEP(launch_check("grid_init_kernel"));
           need_first = true;
           if (momentum)
@@ -659,6 +668,7 @@ int gridding_batch_run(const GridBatch& b, const float2* data, const float* weig
   g.nr = (int64_t)b.P * b.P * b.P;
   const int r_max = b.ori / 2;
   const int maskr2 = (r_max * b.pad) * (r_max * b.pad);
+  g.maskr2 = maskr2;
   const int T = 256;
   dim3 gc((unsigned)((g.nc + T - 1) / T), (unsigned)b.count);
   const dim3 gi((unsigned)((b.P * b.P + kInitWarps - 1) / kInitWarps), (unsigned)b.count);
@@ -669,7 +679,7 @@ int gridding_batch_run(const GridBatch& b, const float2* data, const float* weig
   GTOMRLN_CUFFT_TRY(cufftSetStream(b.r2c, stream));
   GTOMRLN_CUFFT_TRY(cufftSetStream(b.c2r, stream));
   grid_init_kernel<<<gi, 32 * kInitWarps, 0, stream>>>(weight, b.D, b.D, b.D, b.Fw, b.Fnw, b.convft, g, maskr2,
-                                         iterations > 0 && !sym, b.wstride);
+                                                       iterations > 0 && !sym, b.wstride, sym);
   GTOMRLN_STEP(launch_check("grid_init_kernel"));
   if (fused && iterations > 0) GTOMRLN_STEP(gridfft_first(b.convft, g, b.count, stream));
   if (sym && iterations > 0) GTOMRLN_STEP(gridsym_first(b.convft, g, b.count, b.Fw, b.Fnw, nullptr, stream));

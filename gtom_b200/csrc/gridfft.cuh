@@ -14,6 +14,7 @@ struct GridGeom {
   int rowlen;    // P/2 + 1
   int64_t nc;    // rowlen * P * P complex elements
   int64_t nr;    // P^3 real elements
+  int maskr2;    // squared radius of the gridding sphere: the weights are 0 at or beyond it
 };
 
 // The reference's gridding is compiled with fast math (-use_fast_math,
@@ -31,6 +32,9 @@ __device__ __forceinline__ float grid_div(float a, float b) {
   asm("div.full.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
   return r;
 }
+
+// Asks the L2 for a line ahead of the loads that read it.
+__device__ __forceinline__ void grid_prefetch(const float* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // PrecomputeBlobKernel's table index (RecFourier.cu:243-262) at real-space
 // voxel (x, y, z) of the P grid, the radius evaluated as the reference's
@@ -195,8 +199,9 @@ int fft_twiddles(int N, const float2** out);
 // ------------------------------------------- symmetric-spectrum path --
 // The iteration on the Hermitian half along z of the real spectrum
 // (gridsym.cu): four passes over a (P/2+1) x P x (P/2+1) complex work array
-// W (which fits in the cuFFT path's spectrum buffer).  Power-of-two grids
-// P = 64 .. 512.
+// W (which fits in the cuFFT path's spectrum buffer).  Grids with compiled
+// transform lengths (multiples of 32 from 64 to 800, gridsym.cu) and, through
+// gridgen.cu, any other even grid of small prime factors.
 
 bool gridsym_available(int P);
 // Launch attributes and twiddle table of grid P on the current device, made
@@ -223,7 +228,42 @@ int gridsym_iteration(float2* W, const GridGeom& g, int count, const float* tabl
 // x = P/2 terms of each transformed row are taken as real: a spectrum whose
 // x = 0 plane is not Hermitian is transformed by its Hermitian part.
 int gridsym_final(float2* T, const GridGeom& g, int count, const float2* data, int oldx, int oldy, int oldz,
-                  int64_t wstride, const float* Fw, const float* Fnw, bool divide, int ori, float scale, float* out,
+                  int64_t wstride, const float* Fw, float* Fnw, bool divide, int ori, float scale, float* out,
                   float* const* outs, cudaStream_t stream);
+
+// What the final map's passes are given (gridsym.cu, gridgen.cu).
+struct GridFinalArgs {
+  const float2* data;  // centred input spectra (old box), volume stride wstride
+  int oldx, oldy, oldz;
+  int64_t wstride;
+  const float* Fw;     // P-grid weights, volume stride (P/2+1) P P
+  float* Fnw;          // element P/2: set where data outside the sphere are not finite
+  int divide;          // no iteration ran: divide by max(|Fw|, 1e-4)
+  int ori, off;        // output box and its offset in the P grid
+  float scale;
+  float* out;          // ori^3 output (one volume), or
+  float* const* outs;  // one output per volume
+};
+
+// The final map's data at or beyond the sphere (from (x, y, z) on the P grid)
+// count as zero times their value: 0, or NaN for an infinity or a NaN.
+__device__ __forceinline__ float grid_final_zero(const float2* __restrict__ data, const GridFinalArgs& f, int P, int x,
+                                                 int y, int z) {
+  const int64_t src = grid_final_source(f.oldx, f.oldy, f.oldz, P, x, y, z);
+  if (src < 0) return 0.f;
+  const float2 v = __ldg(data + src);
+  return v.x * 0.f + v.y * 0.f;
+}
+
+// ------------------------------------- any other even grid (gridgen.cu) --
+// The same iteration and final map with run-time transform lengths; the
+// functions are gridsym_*'s for the grids gridsym.cu has no compiled
+// transforms for.
+bool gridgen_available(int P);
+int gridgen_prepare(int P);
+int gridgen_first(float2* W, const GridGeom& g, int count, const float* Fw, float* Fnw, float* V, cudaStream_t stream);
+int gridgen_iteration(float2* W, const GridGeom& g, int count, const float* table, const float* Fw, float* Fnw, float* V,
+                      float beta, bool write_next, double* change, const float* ref, cudaStream_t stream);
+int gridgen_final(float2* T, int P, int count, const GridFinalArgs& f, cudaStream_t stream);
 
 }  // namespace gtomrln

@@ -18,12 +18,20 @@
 // leaves the chip.  The imaginary parts the cuFFT path computes and drops
 // are zero up to rounding; the kept real parts are the same sums.
 //
+// Why less than half.  The weights vanish at and beyond the gridding sphere's
+// radius (Fnweight starts there as 0 and stays 0, RecFourier.cu:140-156), at
+// most P/2: 48 % of the spectrum's elements, 21 % of its (kx, ky) columns and
+// all of kx = P/2.  The z pass touches no weight outside the sphere and no
+// column outside its circle (neither reading nor writing W there), the y
+// passes take and leave only the rows inside it, and kx = P/2 is never
+// stored: the skipped values are exact zeros.
+//
 // Per iteration (W: the (P/2+1) x P x (P/2+1) complex work array, layout
 // [z][y][x] with rows of P/2 + 4, the last three elements padding, so that
 // rows start on 32-byte boundaries):
 //   gridsym_y_tma_kernel<INV>  inverse transform along y of W (columns of 16
 //                          consecutive x at one z, staged in shared memory
-//                          by tensor copies, or of x = P/2 at 16 z);
+//                          by tensor copies);
 //   gridsym_x_kernel       per row (y, z): C2R along x, times blob(r)/P^3
 //                          (IFFT.cu:36-46 normalisation, RecFourier.cu:
 //                          243-262 table), R2C along x;
@@ -35,9 +43,14 @@
 //                          iteration and the real-to-Hermitian transform
 //                          along z of Fw * Fnw.
 // HBM bytes per iteration: W in and out in each pass (4 x 16 B per W
-// element) plus Fw in, Fnw in and out in the z pass (12 B per spectrum
-// element): 2.97 GB at P = 512, against ~8 GB for cuFFT's passes plus the
-// blob and update kernels.
+// element, 21 % less on the sides that face the spectrum) plus Fw in, Fnw in
+// and out in the z pass (12 B per element of the sphere): 2.4 GB at P = 512,
+// against ~8 GB for cuFFT's passes plus the blob and update kernels.
+// Measured at P = 512 (us): y 83 and 88 (76 at the copy rate), x 156 (85;
+// bound by its load/store and FP32 instructions), z 242 (132; 24 warps per SM
+// in phases of loads, two transforms and stores); with the whole grid they
+// were 100, 100, 156 and 335.  Ten iterations and the map 7.97 -> 6.39 ms;
+// P = 128 397 -> 228 us.
 //
 // Transforms.  A real transform of length P runs as a complex transform of
 // length H = P/2 on the packed pairs (x(2n), x(2n+1)) with the usual pre-
@@ -76,111 +89,6 @@ namespace {
 constexpr int kCols = 16;          // columns (y and z passes) or rows (x pass) per CTA
 constexpr int kPitch = kCols + 1;  // shared-memory stride between element indices (y, z passes), in float2
 
-// ---------------------------------------------- compile-time twiddles --
-constexpr double kPiD = 3.14159265358979323846264338327950288;
-
-// sin and cos by their Taylor series after reduction to [-pi, pi] (the
-// remaining error is far below FP32 rounding); compile-time only.
-constexpr double ce_sin(double x) {
-  while (x > kPiD) x -= 2 * kPiD;
-  while (x < -kPiD) x += 2 * kPiD;
-  double term = x, sum = x;
-  for (int k = 1; k < 20; k++) {
-    term *= -x * x / ((2.0 * k) * (2.0 * k + 1.0));
-    sum += term;
-  }
-  return sum;
-}
-constexpr double ce_cos(double x) { return ce_sin(x + kPiD / 2); }
-
-// Odd prime DFT of length R in registers (R = 3, 5), unnormalised, forward
-// (exp(-)) or inverse (exp(+)): X(k) = a(0) + sum over n = 1 .. (R-1)/2 of
-// (a(n) + a(R-n)) cos(2 pi k n / R) -+ i (a(n) - a(R-n)) sin(2 pi k n / R).
-template <int R, bool INV>
-__device__ __forceinline__ void dft_odd(float2* v) {
-  float2 sp[(R - 1) / 2], sm[(R - 1) / 2];
-#pragma unroll
-  for (int n = 1; n <= (R - 1) / 2; n++) {
-    sp[n - 1] = cadd(v[n], v[R - n]);
-    sm[n - 1] = csub(v[n], v[R - n]);
-  }
-  float2 out[R];
-  out[0] = v[0];
-#pragma unroll
-  for (int n = 0; n < (R - 1) / 2; n++) out[0] = cadd(out[0], sp[n]);
-#pragma unroll
-  for (int k = 1; k < R; k++) {
-    float2 re = v[0], im = make_float2(0.f, 0.f);  // re: cosine part, im: sine part (before the factor -+i)
-#pragma unroll
-    for (int n = 1; n <= (R - 1) / 2; n++) {
-      const float cs = (float)ce_cos(2 * kPiD * ((k * n) % R) / R);
-      const float sn = (float)ce_sin(2 * kPiD * ((k * n) % R) / R);
-      re = make_float2(fmaf(cs, sp[n - 1].x, re.x), fmaf(cs, sp[n - 1].y, re.y));
-      im = make_float2(fmaf(sn, sm[n - 1].x, im.x), fmaf(sn, sm[n - 1].y, im.y));
-    }
-    // forward: re - i im; inverse: re + i im
-    out[k] = INV ? make_float2(re.x - im.y, re.y + im.x) : make_float2(re.x + im.y, re.y - im.x);
-  }
-#pragma unroll
-  for (int k = 0; k < R; k++) v[k] = out[k];
-}
-
-// In-register DFT of length N (factors 2, 3, 5), unnormalised, forward
-// (exp(-)) or inverse (exp(+)), natural order in and out: decimation in
-// time by the smallest factor (2, then 3, then 5) down to the radix-8/4/2
-// kernels of fftcore.cuh and the odd prime kernels above, with the
-// combining twiddles as constants.
-template <int N, bool INV>
-__device__ __forceinline__ void dftr(float2* v) {
-  if constexpr (N == 1) {
-    return;
-  } else if constexpr (N == 2 || N == 4 || N == 8) {
-    dft<N, INV>(v);
-  } else if constexpr (N == 3 || N == 5) {
-    dft_odd<N, INV>(v);
-  } else {
-    constexpr int R = N % 2 == 0 ? 2 : (N % 3 == 0 ? 3 : 5);
-    constexpr int M = N / R;
-    static_assert(M * R == N, "dftr: lengths with factors 2, 3 and 5 only");
-    float2 sub[R][M];
-#pragma unroll
-    for (int r = 0; r < R; r++)
-#pragma unroll
-      for (int i = 0; i < M; i++) sub[r][i] = v[R * i + r];
-#pragma unroll
-    for (int r = 0; r < R; r++) dftr<M, INV>(sub[r]);
-#pragma unroll
-    for (int k = 0; k < M; k++) {
-      float2 u[R];
-#pragma unroll
-      for (int r = 0; r < R; r++) {
-        if (r * k == 0) {
-          u[r] = sub[r][k];
-        } else if (4 * r * k == N) {
-          u[r] = mul_mi<INV>(sub[r][k]);  // e(-+1/4) = -+i
-        } else if (8 * r * k == N || 8 * r * k == 3 * N) {
-          // e(-+1/8), e(-+3/8): (1 -+ i)/sqrt2, (-1 -+ i)/sqrt2, four operations
-          const float h = 0.70710678118654752440f;
-          const float2 a = sub[r][k];
-          const float2 p = 8 * r * k == N ? a : mul_mi<INV>(a);  // e(-+3/8) = -+i e(-+1/8)
-          u[r] = INV ? make_float2((p.x - p.y) * h, (p.x + p.y) * h) : make_float2((p.x + p.y) * h, (p.y - p.x) * h);
-        } else {
-          const float wr = (float)ce_cos(2 * kPiD * r * k / N);
-          const float wi = (float)(INV ? ce_sin(2 * kPiD * r * k / N) : -ce_sin(2 * kPiD * r * k / N));
-          u[r] = cmul(sub[r][k], make_float2(wr, wi));
-        }
-      }
-      if constexpr (R == 2) {
-        dft<2, INV>(u);
-      } else {
-        dft_odd<R, INV>(u);
-      }
-#pragma unroll
-      for (int q = 0; q < R; q++) v[k + M * q] = u[q];
-    }
-  }
-}
-
 // ------------------------------------------------------ four-step FFT --
 // N = N1 N2 with N2 threads per column and N1 a multiple of N2.
 template <int N>
@@ -193,12 +101,20 @@ struct Split;
 GTOMRLN_SPLIT(32, 8, 4)
 GTOMRLN_SPLIT(48, 12, 4)
 GTOMRLN_SPLIT(64, 8, 8)
+GTOMRLN_SPLIT(80, 20, 4)
 GTOMRLN_SPLIT(96, 24, 4)
 GTOMRLN_SPLIT(128, 16, 8)
+GTOMRLN_SPLIT(144, 12, 12)
+GTOMRLN_SPLIT(160, 40, 4)
 GTOMRLN_SPLIT(192, 24, 8)
 GTOMRLN_SPLIT(256, 16, 16)
+GTOMRLN_SPLIT(288, 24, 12)
+GTOMRLN_SPLIT(320, 40, 8)
+GTOMRLN_SPLIT(384, 48, 8)
 GTOMRLN_SPLIT(400, 20, 20)
 GTOMRLN_SPLIT(512, 32, 16)
+GTOMRLN_SPLIT(576, 24, 24)
+GTOMRLN_SPLIT(768, 48, 16)
 GTOMRLN_SPLIT(800, 40, 20)
 #undef GTOMRLN_SPLIT
 
@@ -295,33 +211,6 @@ __device__ __forceinline__ void four_step_rounds(float2* v, float2* xb, const fl
   for (int m = 0; m < N1; m++) v[m] = w[m];
 }
 
-// The pre-twiddle of a Hermitian-to-real transform of length P = 2H as an
-// H-point complex transform: Z(k) = (X(k) + conj X(H-k)) + i e(sg k/P)
-// (X(k) - conj X(H-k)) (sg = +1: the inverse C2R; -1: the forward sum); the
-// H-point transform of the same sign then gives x(2n) = Re z(n),
-// x(2n+1) = Im z(n).
-template <bool PLUS>
-__device__ __forceinline__ float2 c2r_pre(float2 xk, float2 xm, float2 w) {
-  if (PLUS) w.y = -w.y;  // the table holds e(-k/P)
-  const float2 a = make_float2(xk.x + xm.x, xk.y - xm.y);  // X(k) + conj X(H-k)
-  const float2 b = make_float2(xk.x - xm.x, xk.y + xm.y);  // X(k) - conj X(H-k)
-  const float2 wb = cmul(w, b);
-  return make_float2(a.x - wb.y, a.y + wb.x);  // a + i wb
-}
-
-// The post-twiddle of a real-to-Hermitian transform of length P computed as
-// an H-point complex transform of the packed pairs: Y(k) = (Z(k) + conj
-// Z(H-k)) / 2 - (i/2) e(sg k/P) (Z(k) - conj Z(H-k)) (Z indices mod H;
-// sg = -1: the forward R2C; +1: exp(+)).  Y(H) = Re Z(0) - Im Z(0).
-template <bool PLUS>
-__device__ __forceinline__ float2 r2c_post(float2 zk, float2 zm, float2 w) {
-  if (PLUS) w.y = -w.y;
-  const float2 a = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
-  const float2 b = make_float2(0.5f * (zk.x - zm.x), 0.5f * (zk.y + zm.y));
-  const float2 wb = cmul(w, b);
-  return make_float2(a.x + wb.y, a.y - wb.x);  // a - i wb
-}
-
 __device__ __forceinline__ void load_twiddles(float2* tw, const float2* __restrict__ twg, int P) {
   for (int m = threadIdx.x; m < P; m += blockDim.x) tw[m] = __ldg(twg + m);
 }
@@ -394,13 +283,32 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
 template <int P>
 constexpr int w_pitch() { return P / 2 + 4; }
 
+// CTAs per SM that the passes' registers are held to, by the elements a
+// thread holds (N1): 24 warps of the x and z passes where it holds 16, fewer
+// above.
+template <int P>
+constexpr int pass_blocks(int n1_24) {
+  constexpr int N1 = Split<P / 2>::N1, T = kCols * Split<P / 2>::N2;
+  return (N1 >= 40 ? 384 : N1 == 24 ? n1_24 : N1 == 20 ? 640 : 768) / T;
+}
+template <int P>
+constexpr int x_blocks() { return pass_blocks<P>(512); }
+template <int P>
+constexpr int z_blocks() { return pass_blocks<P>(640); }
+template <int P>
+constexpr int y_blocks() {
+  constexpr int N1 = Split<P>::N1, T = kCols * Split<P>::N2;
+  return P > 512 ? 1 : N1 >= 40 ? 384 / T : 2;
+}
+
 // Sizes of the staged y pass: a tile (16 columns x P rows) arrives as NB
-// tensor boxes of BOX rows (a box has at most 256 rows).
+// tensor boxes of BOX rows; the inverse pass asks only for the boxes that
+// reach into the sphere.
 template <int P>
 struct YStage {
-  static constexpr int NB = (P + 255) / 256;
-  static constexpr int BOX = P / NB;
-  static_assert(BOX * NB == P && BOX <= 256, "YStage: rows must split into equal boxes");
+  static constexpr int BOX = 32;
+  static constexpr int NB = P / BOX;
+  static_assert(BOX * NB == P, "YStage: rows must split into equal boxes");
   static constexpr int N2 = Split<P>::N2;
   static constexpr size_t stage_bytes = sizeof(float2) * kCols * P;
   static constexpr size_t xb_bytes = sizeof(float2) * kCols * N2 * N2;
@@ -408,27 +316,26 @@ struct YStage {
   static constexpr size_t smem = 1024 + stage_bytes + xb_bytes + sizeof(float2) * P;
 };
 
-// The y pass, persistent, over nyq + tiles work units: first the columns
-// x = P/2 (16 consecutive z of one volume per unit, plain loads), then the
-// tiles of 16 consecutive x < P/2 at one (volume, z), each of which arrives
-// in shared memory by tensor copies (map: W as floats, dims {2 w_pitch, P,
-// (P/2+1) volumes}, box {32, BOX, 1}).  CTA i starts with unit i and takes
-// the next from a counter as soon as it holds its current unit in
-// registers, starting the next tile's copy then, so the copy runs during the
-// transform and the stores and the slower x = P/2 units leave no tail.  The
-// counter and the count of finished CTAs sit in the padding element of W's
-// first row (the last CTA zeroes both for the next launch; the first
-// transform zeroes them once).  The transform is four_step_rounds (the
-// exchange buffer and the staging buffer fit two CTAs per SM at P = 512).
+// The y pass, persistent, over the tiles of 16 consecutive x < P/2 at one
+// (volume, z), each of which arrives in shared memory by tensor copies (map:
+// W as floats, dims {2 w_pitch, P, (P/2+1) volumes}, box {32, BOX, 1}).  CTA
+// i starts with tile i and takes the next from a counter as soon as it holds
+// its current tile in registers, starting the next tile's copy then, so the
+// copy runs during the transform and the stores.  The counter and the count
+// of finished CTAs sit in the padding element of W's first row (the last CTA
+// zeroes both for the next launch; the first transform zeroes them once).
+// The transform is four_step_rounds (the exchange buffer and the staging
+// buffer fit two CTAs per SM at P = 512).  On its spectrum side (the inverse's
+// input, the forward's output) rows outside the sphere (x^2 + y^2 >= r2) are
+// zero: not copied, not stored.
 template <int P, bool INV>
-__global__ void __launch_bounds__(kCols * Split<P>::N2, (P > 512 ? 1 : 2))
+__global__ void __launch_bounds__(kCols * Split<P>::N2, y_blocks<P>())
 gridsym_y_tma_kernel(const __grid_constant__ CUtensorMap map, float2* __restrict__ W,
-                     const float2* __restrict__ twg, int tiles, int nyq) {
+                     const float2* __restrict__ twg, int tiles, int r2) {
   using Y = YStage<P>;
   constexpr int H = P / 2, RW = w_pitch<P>();
   constexpr int N1 = Split<P>::N1, N2 = Split<P>::N2;
-  constexpr int XT = H / kCols;                    // tiles per (volume, z)
-  constexpr int NQ = (H + 1 + kCols - 1) / kCols;  // x = P/2 units per volume
+  constexpr int XT = H / kCols;  // tiles per (volume, z)
   extern __shared__ unsigned char sraw[];
   __shared__ unsigned long long bar;
   __shared__ int next_s;
@@ -438,67 +345,65 @@ gridsym_y_tma_kernel(const __grid_constant__ CUtensorMap map, float2* __restrict
   int* sched = reinterpret_cast<int*>(W + H + 1);  // {counter, finished CTAs}
   load_twiddles(tw, twg, P);
   const int c = threadIdx.x & (kCols - 1), t = threadIdx.x / kCols;
-  const int total = nyq + tiles;
   if (threadIdx.x == 0) mbar_init(&bar, 1);
   __syncthreads();
+  grid_dependency_wait();
   auto issue = [&](int tile) {  // one thread
-    const int vz = tile / XT, xt = tile - vz * XT;
+    const int vz = tile / XT, x0 = (tile - vz * XT) * kCols;
     fence_proxy_async();
-    mbar_expect_tx(&bar, (unsigned)Y::stage_bytes);
-#pragma unroll
+    // box k holds the rows k BOX .. (k+1) BOX - 1; its smallest |y|
+    auto needed = [&](int k) {
+      const int lo = k * Y::BOX, y = lo < H ? lo : P - (lo + Y::BOX - 1);
+      return !INV || y * y + x0 * x0 < r2;
+    };
+    unsigned bytes = 0;
+    for (int k = 0; k < Y::NB; k++) bytes += needed(k) ? Y::BOX * kCols * (unsigned)sizeof(float2) : 0u;
+    mbar_expect_tx(&bar, bytes);
     for (int k = 0; k < Y::NB; k++)
-      tma_load_3d(stage + k * Y::BOX * kCols, &map, xt * 2 * kCols, k * Y::BOX, vz, &bar);
+      if (needed(k)) tma_load_3d(stage + k * Y::BOX * kCols, &map, x0 * 2, k * Y::BOX, vz, &bar);
   };
-  // the next unit, and its copy when it is a tile (one thread)
+  // the next tile and its copy (one thread)
   auto take_next = [&]() {
     const int u = (int)gridDim.x + atomicAdd(sched, 1);
     next_s = u;
-    if (u >= nyq && u < total) issue(u - nyq);
+    if (u < tiles) issue(u);
   };
   int u = blockIdx.x;
-  if (threadIdx.x == 0 && u >= nyq && u < total) issue(u - nyq);
+  if (threadIdx.x == 0 && u < tiles) issue(u);
   unsigned parity = 0;
   bool fault = false;
-  while (u < total) {
+  while (u < tiles) {
     float2 v[N1];
-    float2* col;
-    bool in = true;
-    if (u >= nyq) {
-      const bool ok = mbar_wait(&bar, parity);
-      if (!__syncthreads_and(ok)) {
-        if (threadIdx.x == 0) atomicExch(&g_gridsym_fault, 1);
-        mbar_wait(&bar, parity);  // once more for the copy in flight, then leave
-        fault = true;
-        break;
-      }
-      parity ^= 1u;
-#pragma unroll
-      for (int m = 0; m < N1; m++) v[m] = stage[(t + N2 * m) * kCols + c];
-      __syncthreads();  // the staging buffer is read
-      if (threadIdx.x == 0) take_next();
-      const int tile = u - nyq, vz = tile / XT, xt = tile - vz * XT;
-      col = W + (int64_t)vz * P * RW + xt * kCols + c;
-    } else {
-      const int vol = u / NQ, z = (u - vol * NQ) * kCols + c;
-      in = z <= H;
-      col = W + ((int64_t)vol * (H + 1) + (in ? z : 0)) * P * RW + H;
-#pragma unroll
-      for (int m = 0; m < N1; m++) v[m] = in ? col[(int64_t)(t + N2 * m) * RW] : make_float2(0.f, 0.f);
-      __syncthreads();  // every thread has read next_s
-      if (threadIdx.x == 0) take_next();
+    const bool ok = mbar_wait(&bar, parity);
+    if (!__syncthreads_and(ok)) {
+      if (threadIdx.x == 0) atomicExch(&g_gridsym_fault, 1);
+      mbar_wait(&bar, parity);  // once more for the copy in flight, then leave
+      fault = true;
+      break;
     }
-    // no leading barrier: both branches end with one after every thread's
-    // reads of xb for the previous unit; next_s is visible after the rounds'
-    // own barriers
+    parity ^= 1u;
+    const int vz = u / XT, x = (u - vz * XT) * kCols + c;
+    const int ylim2 = r2 - x * x;  // rows with y^2 < ylim2 lie inside the sphere
+    auto inside = [&](int m) {
+      const int y = t + N2 * m, yp = y < H ? y : P - y;
+      return yp * yp < ylim2;
+    };
+#pragma unroll
+    for (int m = 0; m < N1; m++)
+      v[m] = !INV || inside(m) ? stage[(t + N2 * m) * kCols + c] : make_float2(0.f, 0.f);
+    __syncthreads();  // the staging buffer is read
+    if (threadIdx.x == 0) take_next();
+    float2* col = W + (int64_t)vz * P * RW + x;
+    // no leading barrier: the one above follows every thread's reads of xb
+    // for the previous tile; next_s is visible after the rounds' own barriers
     four_step_rounds<P, INV, false>(v, xb, tw, t, c);
-    if (in) {
 #pragma unroll
-      for (int m = 0; m < N1; m++) col[(int64_t)(t + N2 * m) * RW] = v[m];
-    }
+    for (int m = 0; m < N1; m++)
+      if (INV || inside(m)) col[(int64_t)(t + N2 * m) * RW] = v[m];
     u = next_s;
   }
   // the last CTA to finish zeroes the counter for the next launch (a CTA
-  // leaves the loop only once the counter is past the last unit)
+  // leaves the loop only once the counter is past the last tile)
   __syncthreads();
   if (threadIdx.x == 0 && !fault) {
     __threadfence();
@@ -511,14 +416,15 @@ gridsym_y_tma_kernel(const __grid_constant__ CUtensorMap map, float2* __restrict
 }
 
 // ------------------------------------------------------------ x pass --
-// Per row (y, z), z <= P/2: C2R along x, times blob(r) / P^3, R2C along x.
+// Per row (y, z), z <= P/2: C2R along x, times blob(r) / P^3, R2C along x
+// (of which x < P/2 is kept).
 // Grid: ((P/2 + 1) P / 16, volumes); a CTA takes 16 consecutive rows, the
 // N2 threads of a row consecutive lanes.  Where N2 divides 32 a row lies in
 // one warp (warp-synchronous exchanges, shuffles for the Hermitian
-// partners); else (P = 800) the block synchronises and the partners go
+// partners); else (N2 = 12, 20) the block synchronises and the partners go
 // through shared memory.
 template <int P>
-__global__ void __launch_bounds__(kCols * Split<P / 2>::N2, (P > 512 ? 2 : 3))
+__global__ void __launch_bounds__(kCols * Split<P / 2>::N2, x_blocks<P>())
 gridsym_x_kernel(float2* __restrict__ W, const float2* __restrict__ twg, const float* __restrict__ table,
                  float inv_n, float funcsampling) {
   constexpr int H = P / 2, RW = w_pitch<P>();
@@ -529,6 +435,7 @@ gridsym_x_kernel(float2* __restrict__ W, const float2* __restrict__ twg, const f
   float2* tw = smem;
   float2* xb = smem + P + P / 16;  // after the padded twiddle table
   load_twiddles_padded(tw, twg, P);
+  grid_dependency_wait();
   const int t = threadIdx.x % N2, r = threadIdx.x / N2;
   const unsigned lane = threadIdx.x & 31;
   const unsigned partner = WROW ? (lane & ~(unsigned)(N2 - 1)) | ((unsigned)(N2 - t) & (N2 - 1)) : lane;
@@ -537,9 +444,10 @@ gridsym_x_kernel(float2* __restrict__ W, const float2* __restrict__ twg, const f
   float2 v[N1];
 #pragma unroll
   for (int m = 0; m < N1; m++) v[m] = row[t + N2 * m];
-  // a C2R takes the x = 0 and x = P/2 terms as real (their imaginary parts,
-  // zero for a Hermitian spectrum, are dropped as cuFFT's C2R drops them)
-  const float2 xH = t == 0 ? make_float2(row[H].x, 0.f) : make_float2(0.f, 0.f);
+  // a C2R takes the x = 0 term as real (its imaginary part, zero for a
+  // Hermitian spectrum, is dropped as cuFFT's C2R drops it); the x = P/2 term
+  // lies outside the sphere
+  const float2 xH = make_float2(0.f, 0.f);
   if (t == 0) v[0].y = 0.f;
   __syncthreads();  // twiddles in place
   // pre-twiddle of the C2R.  The partner H - k of k = t + N2 m is element
@@ -644,7 +552,6 @@ gridsym_x_kernel(float2* __restrict__ W, const float2* __restrict__ twg, const f
   }
 #pragma unroll
   for (int m = 0; m < N1; m++) row[t + N2 * m] = y[m];
-  if (t == 0) row[H] = make_float2(v[0].x - v[0].y, 0.f);
 }
 
 // ------------------------------------------------------------ z pass --
@@ -655,13 +562,15 @@ enum : int { kZFirst = 0, kZIter = 1 };
 // Hermitian-to-real transform (exp(-)) of W, the update of Fnw (and V) from
 // its values, and with write_next the transform of the new S into W.
 // change (single volume): sums of grid_update_kernel; ref: the distance sums
-// to reference weights as well.  Grid: (tiles, volumes); tiles are 16
-// consecutive x < P/2 at one y, then x = P/2 at 16 consecutive y.
+// to reference weights as well.  Grid: (P (P/2) / 16, volumes): tiles of 16
+// consecutive x < P/2 at one y.  Elements with x^2 + y^2 + z^2 >= r2 (the
+// sphere) have zero weights and stay so: they are neither read nor written,
+// nor are W's columns outside the circle (P = 512: 0.85 instead of 1.36 GB).
 template <int P, int MODE, bool MOM>
-__global__ void __launch_bounds__(kCols * Split<P / 2>::N2, (P > 512 ? 2 : 3))
+__global__ void __launch_bounds__(kCols * Split<P / 2>::N2, z_blocks<P>())
 gridsym_z_kernel(float2* __restrict__ W, const float* __restrict__ Fw, float* __restrict__ Fnw,
                  float* __restrict__ V, const float2* __restrict__ twg, float beta, int write_next,
-                 double* __restrict__ change, const float* __restrict__ ref) {
+                 double* __restrict__ change, const float* __restrict__ ref, int r2s) {
   constexpr int H = P / 2, R = H + 1, RW = w_pitch<P>();
   constexpr int N1 = Split<H>::N1, N2 = Split<H>::N2;
   constexpr int64_t NC = (int64_t)R * P * P;         // spectrum elements per volume
@@ -672,19 +581,16 @@ gridsym_z_kernel(float2* __restrict__ W, const float* __restrict__ Fw, float* __
   float2* tw = smem;
   float2* xb = smem + P;
   load_twiddles(tw, twg, P);
+  grid_dependency_wait();
   const int c = threadIdx.x & (kCols - 1), t = threadIdx.x / kCols;
-  constexpr int kMain = P * (H / kCols);
-  const int b = blockIdx.x;
-  int x, y;
-  if (b < kMain) {
-    y = b / (H / kCols);
-    x = (b - y * (H / kCols)) * kCols + c;
-  } else {
-    y = (b - kMain) * kCols + c;
-    x = H;
-  }
+  const int y = blockIdx.x / (H / kCols);
+  const int x0 = (blockIdx.x - y * (H / kCols)) * kCols, x = x0 + c;
+  const int yp = y < H ? y : P - y;
+  if (x0 * x0 + yp * yp >= r2s) return;  // the whole tile is outside the circle
+  const int zlim2 = r2s - x * x - yp * yp;  // elements with z^2 < zlim2 lie inside the sphere
+  const bool in = zlim2 > 0;
   const int64_t vol = blockIdx.y;
-  if (MODE == kZFirst && b == 0 && vol == 0 && threadIdx.x == 0) {
+  if (MODE == kZFirst && blockIdx.x == 0 && vol == 0 && threadIdx.x == 0) {
     // the y pass's work counter (padding of W's first row): zero for its first launch
     int* sched = reinterpret_cast<int*>(W + H + 1);
     sched[0] = 0;
@@ -696,11 +602,11 @@ gridsym_z_kernel(float2* __restrict__ W, const float* __restrict__ Fw, float* __
   if (MODE == kZIter) {
     float2 xH = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int m = 0; m < N1; m++) v[m] = wc[(t + N2 * m) * EW];
+    for (int m = 0; m < N1; m++) v[m] = in ? wc[(t + N2 * m) * EW] : make_float2(0.f, 0.f);
     // the z = 0 and z = P/2 terms of a Hermitian column are real (their
     // imaginary parts are rounding, dropped as a C2R drops them)
     if (t == 0) {
-      xH = make_float2(wc[H * EW].x, 0.f);
+      if (in) xH = make_float2(wc[H * EW].x, 0.f);
       v[0].y = 0.f;
     }
     // pre-twiddle (exp(-) sum) with the partners H - k through shared memory
@@ -720,6 +626,10 @@ gridsym_z_kernel(float2* __restrict__ W, const float* __restrict__ Fw, float* __
   // the packed pairs is (S(2n), S(2n+1))
   double d2 = 0, o2 = 0, r2 = 0, q2 = 0;
   const bool dist = MODE == kZIter && change && ref;
+  auto inside = [&](int z) {
+    const int zp = z < H ? z : P - z;
+    return zp * zp < zlim2;
+  };
   constexpr int CH = N1 < 2 ? N1 : 2;
 #pragma unroll
   for (int m0 = 0; m0 < N1; m0 += CH) {
@@ -729,11 +639,13 @@ gridsym_z_kernel(float2* __restrict__ W, const float* __restrict__ Fw, float* __
     for (int q = 0; q < CH; q++) {
 #pragma unroll
       for (int h = 0; h < 2; h++) {
-        const int64_t gi = wo + (int64_t)(2 * (t + N2 * (m0 + q)) + h) * ES;
-        fw[q][h] = __ldg(Fw + gi);
-        old[q][h] = MODE == kZIter || !MOM ? Fnw[gi] : 0.f;
-        vv[q][h] = MOM ? V[gi] : 0.f;
-        rf[q][h] = dist ? __ldg(ref + gi) : 0.f;
+        const int z = 2 * (t + N2 * (m0 + q)) + h;
+        const int64_t gi = wo + (int64_t)z * ES;
+        const bool on = inside(z);
+        fw[q][h] = on ? __ldg(Fw + gi) : 0.f;
+        old[q][h] = on && (MODE == kZIter || !MOM) ? Fnw[gi] : 0.f;
+        vv[q][h] = on && MOM ? V[gi] : 0.f;
+        rf[q][h] = on && dist ? __ldg(ref + gi) : 0.f;
       }
     }
 #pragma unroll
@@ -742,19 +654,21 @@ gridsym_z_kernel(float2* __restrict__ W, const float* __restrict__ Fw, float* __
       float sv[2];
 #pragma unroll
       for (int h = 0; h < 2; h++) {
-        const int64_t gi = wo + (int64_t)(2 * (t + N2 * m) + h) * ES;
+        const int z = 2 * (t + N2 * m) + h;
+        const int64_t gi = wo + (int64_t)z * ES;
+        const bool on = inside(z);
         float next;
         if (MODE == kZIter) {
           const float cval = h ? v[m].y : v[m].x;
           float nw;
           if (MOM) {
             grid_update_momentum_value(cval, old[q][h], vv[q][h], beta, nw, next);
-            V[gi] = next;
+            if (on) V[gi] = next;
           } else {
             nw = grid_update_value(cval, old[q][h]);
             next = nw;
           }
-          Fnw[gi] = nw;
+          if (on) Fnw[gi] = nw;
           if (change) {
             const double d = (double)fw[q][h] * ((double)nw - (double)old[q][h]);
             const double o = (double)fw[q][h] * (double)old[q][h];
@@ -793,9 +707,10 @@ gridsym_z_kernel(float2* __restrict__ W, const float* __restrict__ Fw, float* __
 #pragma unroll
   for (int m = 0; m < N1; m++) {
     const int k = t + N2 * m, km = k == 0 ? 0 : H - k;
-    wc[k * EW] = r2c_post<true>(v[m], xb[km * kPitch + c], tw[k]);
+    const float2 w = r2c_post<true>(v[m], xb[km * kPitch + c], tw[k]);
+    if (in) wc[k * EW] = w;
   }
-  if (t == 0) wc[H * EW] = make_float2(v[0].x - v[0].y, 0.f);
+  if (t == 0 && in) wc[H * EW] = make_float2(v[0].x - v[0].y, 0.f);
 }
 
 // -------------------------------------------------------- final map --
@@ -805,25 +720,16 @@ gridsym_z_kernel(float2* __restrict__ W, const float* __restrict__ Fw, float* __
 // z planes and y rows of the crop are ever written.  T: the work array,
 // (P/2+1) x P x ori complex per volume, layout [zc][y][x] (rows of P/2 + 1),
 // inside the loop's W buffer.
-struct FinalArgs {
-  const float2* data;  // centred input spectra (old box), volume stride wstride
-  int oldx, oldy, oldz;
-  int64_t wstride;
-  const float* Fw;     // P-grid weights, volume stride (P/2+1) P P
-  const float* Fnw;
-  int divide;          // no iteration ran: divide by max(|Fw|, 1e-4)
-  int ori, off;        // output box and its offset in the P grid
-  float scale;
-  float* out;          // ori^3 output (one volume), or
-  float* const* outs;  // one output per volume
-};
-
 // Pass 1, per column (x, y) along z: the final spectrum's elements
 // (grid_final_value, straight from the caller's data), inverse transform,
-// the crop's z planes written.  Tiles as in gridsym_z_kernel.
+// the crop's z planes written.  Tiles as in gridsym_z_kernel; the data are
+// masked to r < P/2: weights are read in that sphere only and its circle of
+// columns transformed and written.  The data outside are read all the same:
+// one that is not finite makes the whole map NaN, as its product with zero
+// would (the flag Fnw[P/2], zeroed by grid_init_kernel).
 template <int P>
-__global__ void __launch_bounds__(kCols * Split<P>::N2, (P > 512 ? 1 : 2))
-gridsym_final_z_kernel(float2* __restrict__ T, FinalArgs f, const float2* __restrict__ twg) {
+__global__ void __launch_bounds__(kCols * Split<P>::N2, y_blocks<P>())
+gridsym_final_z_kernel(float2* __restrict__ T, GridFinalArgs f, const float2* __restrict__ twg) {
   constexpr int H = P / 2, R = H + 1;
   constexpr int N1 = Split<P>::N1, N2 = Split<P>::N2;
   constexpr int64_t NC = (int64_t)R * P * P;
@@ -831,24 +737,29 @@ gridsym_final_z_kernel(float2* __restrict__ T, FinalArgs f, const float2* __rest
   float2* tw = smem;
   float2* xb = smem + P;
   load_twiddles(tw, twg, P);
+  grid_dependency_wait();
   const int c = threadIdx.x & (kCols - 1), t = threadIdx.x / kCols;
-  constexpr int kMain = P * (H / kCols);
-  const int b = blockIdx.x;
-  int x, y;
-  if (b < kMain) {
-    y = b / (H / kCols);
-    x = (b - y * (H / kCols)) * kCols + c;
-  } else {
-    y = (b - kMain) * kCols + c;
-    x = H;
-  }
+  const int y = blockIdx.x / (H / kCols);
+  const int x0 = (blockIdx.x - y * (H / kCols)) * kCols, x = x0 + c;
+  const int yp = y < H ? y : P - y;
+  const int zlim2 = H * H - x * x - yp * yp;
   const int64_t vol = blockIdx.y;
   const float2* data = f.data + vol * f.wstride;
   const float* Fw = f.Fw + vol * NC;
-  const float* Fnw = f.Fnw + vol * NC;
+  float* Fnw = f.Fnw + vol * NC;
+  const bool rim = x0 + kCols == H && c == 0;  // also sees to x = P/2
+  if (x0 * x0 + yp * yp >= H * H || rim) {
+    float p = 0.f;
+#pragma unroll
+    for (int m = 0; m < N1; m++) {
+      if (x0 * x0 + yp * yp >= H * H) p += grid_final_zero(data, f, P, x, y, t + N2 * m);
+      if (rim) p += grid_final_zero(data, f, P, H, y, t + N2 * m);
+    }
+    if (p != 0.f) Fnw[H] = p;
+  }
+  if (x0 * x0 + yp * yp >= H * H) return;  // outside the mask's circle: read as zero by the y pass
   float2* tv = T + vol * ((int64_t)R * P * f.ori);
-  // the loads of CH elements first (an index outside the input box reads
-  // element 0, zeroed after), then their corrections
+  // the loads of CH elements first (those outside the input box are zero), then their corrections
   const float* wsrc = f.divide ? Fw : Fnw;
   constexpr int CH = N1 <= 20 ? N1 : (N1 % 20 == 0 ? 20 : (N1 % 16 == 0 ? 16 : 12));
   static_assert(N1 % CH == 0, "gridsym_final_z_kernel: chunks");
@@ -859,30 +770,36 @@ gridsym_final_z_kernel(float2* __restrict__ T, FinalArgs f, const float2* __rest
 #pragma unroll
     for (int q = 0; q < CH; q++) {
       const int z = t + N2 * (m0 + q);
+      const int zp = z < H ? z : P - z;
+      const bool on = zp * zp < zlim2;
       const int64_t src = grid_final_source(f.oldx, f.oldy, f.oldz, P, x, y, z);
-      v[m0 + q] = __ldg(data + (src >= 0 ? src : 0));
-      if (src < 0) v[m0 + q] = make_float2(0.f, 0.f);
-      wt[q] = __ldg(wsrc + ((int64_t)z * P + y) * R + x);
+      v[m0 + q] = src >= 0 ? __ldg(data + src) : make_float2(0.f, 0.f);
+      wt[q] = on ? __ldg(wsrc + ((int64_t)z * P + y) * R + x) : 0.f;
     }
 #pragma unroll
     for (int q = 0; q < CH; q++)
       v[m0 + q] = grid_final_apply(v[m0 + q], wt[q], P, x, y, t + N2 * (m0 + q), f.divide != 0);
+  }
+  if (zlim2 <= 0) {  // a column of zeros, or NaN
+    float p = 0.f;
+#pragma unroll
+    for (int m = 0; m < N1; m++) p += v[m].x + v[m].y;
+    if (p != 0.f) Fnw[H] = p;
   }
   __syncthreads();  // twiddles in place
   four_step<P, true, false, false, 1>(v, xb, tw, t, c);
 #pragma unroll
   for (int m = 0; m < N1; m++) {
     const int z = t + N2 * m - f.off;
-    if ((unsigned)z < (unsigned)f.ori) tv[((int64_t)z * P + y) * R + x] = v[m];
+    if (zlim2 > 0 && (unsigned)z < (unsigned)f.ori) tv[((int64_t)z * P + y) * R + x] = v[m];
   }
 }
 
 // Pass 2, per column (x, zc) along y: inverse transform, the crop's rows
 // written to rows 0 .. ori-1 of the plane (each CTA has read its whole
-// column before it writes).  Tiles: 16 consecutive x < P/2 at one zc, then
-// x = P/2 at 16 consecutive zc.
+// column before it writes).  Tiles: 16 consecutive x < P/2 at one zc.
 template <int P>
-__global__ void __launch_bounds__(kCols * Split<P>::N2, (P > 512 ? 1 : 2))
+__global__ void __launch_bounds__(kCols * Split<P>::N2, y_blocks<P>())
 gridsym_final_y_kernel(float2* __restrict__ T, int ori, int off, const float2* __restrict__ twg) {
   constexpr int H = P / 2, R = H + 1;
   constexpr int N1 = Split<P>::N1, N2 = Split<P>::N2;
@@ -890,39 +807,31 @@ gridsym_final_y_kernel(float2* __restrict__ T, int ori, int off, const float2* _
   float2* tw = smem;
   float2* xb = smem + P;
   load_twiddles(tw, twg, P);
+  grid_dependency_wait();
   const int c = threadIdx.x & (kCols - 1), t = threadIdx.x / kCols;
-  const int kMain = (H / kCols) * ori;
-  const int b = blockIdx.x;
-  int zc, x;
-  if (b < kMain) {
-    zc = b / (H / kCols);
-    x = (b - zc * (H / kCols)) * kCols + c;
-  } else {
-    zc = (b - kMain) * kCols + c;
-    x = H;
-  }
-  const bool in = zc < ori;
-  float2* col = T + (int64_t)blockIdx.y * ((int64_t)R * P * ori) + (in ? ((int64_t)zc * P * R + x) : 0);
+  const int zc = blockIdx.x / (H / kCols), x = (blockIdx.x - zc * (H / kCols)) * kCols + c;
+  float2* col = T + ((int64_t)blockIdx.y * ori + zc) * P * R + x;
   float2 v[N1];
 #pragma unroll
-  for (int m = 0; m < N1; m++) v[m] = in ? col[(int64_t)(t + N2 * m) * R] : make_float2(0.f, 0.f);
+  for (int m = 0; m < N1; m++) {
+    const int y = t + N2 * m, yp = y < H ? y : P - y;
+    v[m] = yp * yp + x * x < H * H ? col[(int64_t)y * R] : make_float2(0.f, 0.f);
+  }
   __syncthreads();  // twiddles in place
   four_step<P, true, false, false, 1>(v, xb, tw, t, c);
-  if (in) {
 #pragma unroll
-    for (int m = 0; m < N1; m++) {
-      const int yc = t + N2 * m - off;
-      if ((unsigned)yc < (unsigned)ori) col[(int64_t)yc * R] = v[m];
-    }
+  for (int m = 0; m < N1; m++) {
+    const int yc = t + N2 * m - off;
+    if ((unsigned)yc < (unsigned)ori) col[(int64_t)yc * R] = v[m];
   }
 }
 
-// Pass 3, per row (yc, zc): C2R along x (the x = 0 and x = P/2 terms taken
-// as real), the crop's x, the gridding correction and scale.  A CTA takes
+// Pass 3, per row (yc, zc): C2R along x (the x = 0 term taken as real, the
+// x = P/2 term zero), the crop's x, the gridding correction and scale.  A CTA takes
 // 16 consecutive rows of the ori x ori crop (rows past it idle).
 template <int P>
-__global__ void __launch_bounds__(kCols * Split<P / 2>::N2, (P > 512 ? 2 : 3))
-gridsym_final_x_kernel(const float2* __restrict__ T, FinalArgs f, const float2* __restrict__ twg) {
+__global__ void __launch_bounds__(kCols * Split<P / 2>::N2, x_blocks<P>())
+gridsym_final_x_kernel(const float2* __restrict__ T, GridFinalArgs f, const float2* __restrict__ twg) {
   constexpr int H = P / 2, R = H + 1;
   constexpr int N1 = Split<H>::N1, N2 = Split<H>::N2;
   constexpr bool WROW = 32 % N2 == 0;
@@ -931,6 +840,7 @@ gridsym_final_x_kernel(const float2* __restrict__ T, FinalArgs f, const float2* 
   float2* tw = smem;
   float2* xb = smem + P + P / 16;  // after the padded twiddle table
   load_twiddles_padded(tw, twg, P);
+  grid_dependency_wait();
   const int t = threadIdx.x % N2, r = threadIdx.x / N2;
   const unsigned lane = threadIdx.x & 31;
   const unsigned partner = WROW ? (lane & ~(unsigned)(N2 - 1)) | ((unsigned)(N2 - t) & (N2 - 1)) : lane;
@@ -943,7 +853,7 @@ gridsym_final_x_kernel(const float2* __restrict__ T, FinalArgs f, const float2* 
   float2 v[N1];
 #pragma unroll
   for (int m = 0; m < N1; m++) v[m] = in ? row[t + N2 * m] : make_float2(0.f, 0.f);
-  const float2 xH = t == 0 && in ? make_float2(row[H].x, 0.f) : make_float2(0.f, 0.f);
+  const float2 xH = make_float2(0.f, 0.f);  // x = P/2 lies outside the mask's sphere
   if (t == 0) v[0].y = 0.f;
   __syncthreads();  // twiddles in place
   {
@@ -972,8 +882,9 @@ gridsym_final_x_kernel(const float2* __restrict__ T, FinalArgs f, const float2* 
   }
   four_step<H, true, true, WROW, 2>(v, xb, tw, t, r);
   if (!in) return;  // after the last collective of the row's warp / block
-  // a y pass whose tensor copies did not complete left W unusable: NaN map
-  const bool fault = g_gridsym_fault != 0;
+  // a y pass whose tensor copies did not complete left W unusable: NaN map,
+  // and so do data outside the sphere that are not finite
+  const bool fault = g_gridsym_fault != 0 || f.Fnw[vol * ((int64_t)R * P * P) + H] != 0.f;
   float* out = f.outs ? f.outs[vol] : f.out;
   float* orow = out + ((int64_t)zc * ori + yc) * ori;
 #pragma unroll
@@ -995,7 +906,7 @@ struct SymSizes {
   static constexpr int y_threads = kCols * Split<P>::N2;
   static constexpr int xz_threads = kCols * Split<H>::N2;
   static constexpr int x_tiles = (H + 1) * P / kCols;
-  static constexpr int z_tiles = P * (H / kCols) + P / kCols;
+  static constexpr int z_tiles = P * (H / kCols);
   // twiddle table + exchange buffer
   static constexpr size_t y_smem = sizeof(float2) * (P + (size_t)P * kPitch);
   static constexpr size_t x_smem =
@@ -1090,23 +1001,24 @@ int y_stage_ctas(int* out) {
 }
 
 template <int P>
-int run_first(float2* W, int count, const float* Fw, float* Fnw, float* V, const float2* tw,
+int run_first(float2* W, int count, const float* Fw, float* Fnw, float* V, int r2, const float2* tw,
               cudaStream_t stream) {
   using Z = SymSizes<P>;
   const dim3 grid(Z::z_tiles, count);
   if (V)
-    gridsym_z_kernel<P, kZFirst, true><<<grid, Z::xz_threads, Z::z_smem, stream>>>(W, Fw, Fnw, V, tw, 0.f, 1,
-                                                                                   nullptr, nullptr);
+    launch_dependent(gridsym_z_kernel<P, kZFirst, true>, grid, Z::xz_threads, Z::z_smem, stream,
+                   W, Fw, Fnw, V, tw, 0.f, 1, nullptr, nullptr, r2);
   else
-    gridsym_z_kernel<P, kZFirst, false><<<grid, Z::xz_threads, Z::z_smem, stream>>>(W, Fw, Fnw, V, tw, 0.f, 1,
-                                                                                    nullptr, nullptr);
+    launch_dependent(gridsym_z_kernel<P, kZFirst, false>, grid, Z::xz_threads, Z::z_smem, stream,
+                   W, Fw, Fnw, V, tw, 0.f, 1, nullptr, nullptr, r2);
   GTOMRLN_LAUNCH_CHECK("gridsym_z_kernel (first)");
   return GTOMRLN_OK;
 }
 
 template <int P>
 int run_iteration(float2* W, int count, const float* table, const float* Fw, float* Fnw, float* V, float beta,
-                  bool write_next, double* change, const float* ref, const float2* tw, cudaStream_t stream) {
+                  bool write_next, double* change, const float* ref, int r2, const float2* tw,
+                  cudaStream_t stream) {
   using Z = SymSizes<P>;
   const float inv_n = 1.0f / ((float)P * (float)P * (float)P);
   const float funcsampling = (float)(0.5 / kBlobSamples);
@@ -1118,52 +1030,63 @@ int run_iteration(float2* W, int count, const float* table, const float* Fw, flo
   if (st) return st;
   const int tiles = (P / 2 / kCols) * (P / 2 + 1) * count;
   const unsigned grid_y = (unsigned)std::min(tiles, ctas);
-  const int nyq = (P / 2 + 1 + kCols - 1) / kCols * count;
-  gridsym_y_tma_kernel<P, true><<<grid_y, Z::y_threads, YStage<P>::smem, stream>>>(map, W, tw, tiles, nyq);
+  launch_dependent(gridsym_y_tma_kernel<P, true>, grid_y, Z::y_threads, YStage<P>::smem, stream,
+                   map, W, tw, tiles, r2);
   GTOMRLN_LAUNCH_CHECK("gridsym_y_tma_kernel (inverse)");
-  gridsym_x_kernel<P><<<dim3(Z::x_tiles, count), Z::xz_threads, Z::x_smem, stream>>>(W, tw, table, inv_n,
-                                                                                     funcsampling);
+  launch_dependent(gridsym_x_kernel<P>, dim3(Z::x_tiles, count), Z::xz_threads, Z::x_smem, stream,
+                   W, tw, table, inv_n, funcsampling);
   GTOMRLN_LAUNCH_CHECK("gridsym_x_kernel");
-  gridsym_y_tma_kernel<P, false><<<grid_y, Z::y_threads, YStage<P>::smem, stream>>>(map, W, tw, tiles, nyq);
+  launch_dependent(gridsym_y_tma_kernel<P, false>, grid_y, Z::y_threads, YStage<P>::smem, stream,
+                   map, W, tw, tiles, r2);
   GTOMRLN_LAUNCH_CHECK("gridsym_y_tma_kernel (forward)");
   const dim3 grid(Z::z_tiles, count);
   if (V)
-    gridsym_z_kernel<P, kZIter, true><<<grid, Z::xz_threads, Z::z_smem, stream>>>(W, Fw, Fnw, V, tw, beta,
-                                                                                  write_next, change, ref);
+    launch_dependent(gridsym_z_kernel<P, kZIter, true>, grid, Z::xz_threads, Z::z_smem, stream,
+                   W, Fw, Fnw, V, tw, beta, write_next, change, ref, r2);
   else
-    gridsym_z_kernel<P, kZIter, false><<<grid, Z::xz_threads, Z::z_smem, stream>>>(W, Fw, Fnw, V, tw, beta,
-                                                                                   write_next, change, ref);
+    launch_dependent(gridsym_z_kernel<P, kZIter, false>, grid, Z::xz_threads, Z::z_smem, stream,
+                   W, Fw, Fnw, V, tw, beta, write_next, change, ref, r2);
   GTOMRLN_LAUNCH_CHECK("gridsym_z_kernel");
   return GTOMRLN_OK;
 }
 
 template <int P>
-int run_final(float2* T, int count, const FinalArgs& f, const float2* tw, cudaStream_t stream) {
+int run_final(float2* T, int count, const GridFinalArgs& f, const float2* tw, cudaStream_t stream) {
   using Z = SymSizes<P>;
   constexpr int H = P / 2;
-  gridsym_final_z_kernel<P><<<dim3(Z::z_tiles, count), Z::y_threads, Z::y_smem, stream>>>(T, f, tw);
+  launch_dependent(gridsym_final_z_kernel<P>, dim3(Z::z_tiles, count), Z::y_threads, Z::y_smem, stream,
+                   T, f, tw);
   GTOMRLN_LAUNCH_CHECK("gridsym_final_z_kernel");
-  const unsigned ytiles = (unsigned)((H / kCols) * f.ori + (f.ori + kCols - 1) / kCols);
-  gridsym_final_y_kernel<P><<<dim3(ytiles, count), Z::y_threads, Z::y_smem, stream>>>(T, f.ori, f.off, tw);
+  const unsigned ytiles = (unsigned)((H / kCols) * f.ori);
+  launch_dependent(gridsym_final_y_kernel<P>, dim3(ytiles, count), Z::y_threads, Z::y_smem, stream,
+                   T, f.ori, f.off, tw);
   GTOMRLN_LAUNCH_CHECK("gridsym_final_y_kernel");
   const unsigned xtiles = (unsigned)(((int64_t)f.ori * f.ori + kCols - 1) / kCols);
-  gridsym_final_x_kernel<P><<<dim3(xtiles, count), Z::xz_threads, Z::x_smem, stream>>>(T, f, tw);
+  launch_dependent(gridsym_final_x_kernel<P>, dim3(xtiles, count), Z::xz_threads, Z::x_smem, stream,
+                   T, f, tw);
   GTOMRLN_LAUNCH_CHECK("gridsym_final_x_kernel");
   return GTOMRLN_OK;
 }
 
-// Dispatch over the supported grids.
+// Dispatch over the supported grids: the multiples of 32 whose length and
+// half have a Split (of radices 2, 3 and 5, up to 48 elements a thread).
 template <typename F>
-int with_grid(int P, F&& f) {
+bool with_grid(int P, F&& f) {
   switch (P) {
-    case 64: return f(std::integral_constant<int, 64>());
-    case 96: return f(std::integral_constant<int, 96>());
-    case 128: return f(std::integral_constant<int, 128>());
-    case 192: return f(std::integral_constant<int, 192>());
-    case 256: return f(std::integral_constant<int, 256>());
-    case 512: return f(std::integral_constant<int, 512>());
-    case 800: return f(std::integral_constant<int, 800>());
-    default: return set_error(GTOMRLN_ERR_INVALID, "gridsym: unsupported grid %d", P);
+    case 64: f(std::integral_constant<int, 64>()); return true;
+    case 96: f(std::integral_constant<int, 96>()); return true;
+    case 128: f(std::integral_constant<int, 128>()); return true;
+    case 160: f(std::integral_constant<int, 160>()); return true;
+    case 192: f(std::integral_constant<int, 192>()); return true;
+    case 256: f(std::integral_constant<int, 256>()); return true;
+    case 288: f(std::integral_constant<int, 288>()); return true;
+    case 320: f(std::integral_constant<int, 320>()); return true;
+    case 384: f(std::integral_constant<int, 384>()); return true;
+    case 512: f(std::integral_constant<int, 512>()); return true;
+    case 576: f(std::integral_constant<int, 576>()); return true;
+    case 768: f(std::integral_constant<int, 768>()); return true;
+    case 800: f(std::integral_constant<int, 800>()); return true;
+    default: return false;
   }
 }
 
@@ -1176,18 +1099,23 @@ int ensure_attributes(int P) {
   const auto key = std::make_tuple(dev, context_id(), P);
   std::lock_guard<std::mutex> lock(g_attr_mutex);
   if (g_attr_done.count(key)) return GTOMRLN_OK;
-  const int st = with_grid(P, [](auto p) { return set_attributes<decltype(p)::value>(); });
+  int st = GTOMRLN_OK;
+  with_grid(P, [&](auto p) { st = set_attributes<decltype(p)::value>(); });
   if (st == GTOMRLN_OK) g_attr_done[key] = true;
   return st;
 }
 
 }  // namespace
 
-bool gridsym_available(int P) {
-  return P == 64 || P == 96 || P == 128 || P == 192 || P == 256 || P == 512 || P == 800;
+// Grids with compiled transform lengths here; gridgen.cu takes other even ones.
+static bool compiled(int P) {
+  return with_grid(P, [](auto) {});
 }
 
+bool gridsym_available(int P) { return compiled(P) || gridgen_available(P); }
+
 int gridsym_prepare(int P) {
+  if (!compiled(P)) return gridgen_prepare(P);
   int st = ensure_attributes(P);
   if (st) return st;
   const float2* tw = nullptr;
@@ -1196,38 +1124,38 @@ int gridsym_prepare(int P) {
 
 int gridsym_first(float2* W, const GridGeom& g, int count, const float* Fw, float* Fnw, float* V,
                   cudaStream_t stream) {
+  if (!compiled(g.P)) return gridgen_first(W, g, count, Fw, Fnw, V, stream);
   int st = ensure_attributes(g.P);
   if (st) return st;
   const float2* tw = nullptr;
   st = fft_twiddles(g.P, &tw);
   if (st) return st;
-  return with_grid(g.P, [&](auto p) { return run_first<decltype(p)::value>(W, count, Fw, Fnw, V, tw, stream); });
+  with_grid(g.P, [&](auto p) { st = run_first<decltype(p)::value>(W, count, Fw, Fnw, V, g.maskr2, tw, stream); });
+  return st;
 }
 
 int gridsym_iteration(float2* W, const GridGeom& g, int count, const float* table, const float* Fw, float* Fnw,
                       float* V, float beta, bool write_next, double* change, const float* ref,
                       cudaStream_t stream) {
+  if (!compiled(g.P))
+    return gridgen_iteration(W, g, count, table, Fw, Fnw, V, beta, write_next, change, ref, stream);
   int st = ensure_attributes(g.P);
   if (st) return st;
   const float2* tw = nullptr;
   st = fft_twiddles(g.P, &tw);
   if (st) return st;
-  return with_grid(g.P, [&](auto p) {
-    return run_iteration<decltype(p)::value>(W, count, table, Fw, Fnw, V, beta, write_next, change, ref, tw,
-                                             stream);
+  with_grid(g.P, [&](auto p) {
+    st = run_iteration<decltype(p)::value>(W, count, table, Fw, Fnw, V, beta, write_next, change, ref, g.maskr2, tw,
+                                           stream);
   });
+  return st;
 }
 
 int gridsym_final(float2* T, const GridGeom& g, int count, const float2* data, int oldx, int oldy, int oldz,
-                  int64_t wstride, const float* Fw, const float* Fnw, bool divide, int ori, float scale, float* out,
+                  int64_t wstride, const float* Fw, float* Fnw, bool divide, int ori, float scale, float* out,
                   float* const* outs, cudaStream_t stream) {
   if (ori <= 0 || ori > g.P) return set_error(GTOMRLN_ERR_INVALID, "gridsym_final: output box %d", ori);
-  int st = ensure_attributes(g.P);
-  if (st) return st;
-  const float2* tw = nullptr;
-  st = fft_twiddles(g.P, &tw);
-  if (st) return st;
-  FinalArgs f;
+  GridFinalArgs f;
   f.data = data;
   f.oldx = oldx;
   f.oldy = oldy;
@@ -1241,7 +1169,14 @@ int gridsym_final(float2* T, const GridGeom& g, int count, const float2* data, i
   f.scale = scale;
   f.out = out;
   f.outs = outs;
-  return with_grid(g.P, [&](auto p) { return run_final<decltype(p)::value>(T, count, f, tw, stream); });
+  if (!compiled(g.P)) return gridgen_final(T, g.P, count, f, stream);
+  int st = ensure_attributes(g.P);
+  if (st) return st;
+  const float2* tw = nullptr;
+  st = fft_twiddles(g.P, &tw);
+  if (st) return st;
+  with_grid(g.P, [&](auto p) { st = run_final<decltype(p)::value>(T, count, f, tw, stream); });
+  return st;
 }
 
 // Forgets the launch attributes set on device dev (a context reset drops

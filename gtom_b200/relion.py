@@ -379,8 +379,8 @@ def set_path(op: str, path: str) -> None:
     "segment" (pixels found per brick by row segments; the backprojector's
     accumulates each work item in fixed point first), for "backproject" also
     "segment_fp32" (row segments, FP32 atomics only); of "gridding": "auto"
-    (default: "symmetric" on power-of-two grids P = 64 .. 512, cuFFT
-    elsewhere), "direct" (cuFFT transforms), "fused" (two fused passes per
+    (default: "symmetric" on even grids P = 16 .. 768 without a prime factor
+    above 13 and P = 800, cuFFT elsewhere), "direct" (cuFFT transforms), "fused" (two fused passes per
     iteration with the library's own transforms on power-of-two grids) or
     "symmetric" (four passes over the Hermitian half along z of the real
     iterated spectrum, the library's own transforms) (gtomrln_set_path)."""

@@ -79,8 +79,8 @@ GTOMRLN_API int gtomrln_release_caches(void);
 #define GTOMRLN_OP_PROJECT 0
 #define GTOMRLN_OP_BACKPROJECT 1
 /* op GTOMRLN_OP_GRIDDING: GTOMRLN_PATH_AUTO (default) runs the gridding
- * as GTOMRLN_PATH_SYMMETRIC (below) on the grids P = 64, 96, 128, 192, 256,
- * 512 and 800 and with cuFFT's 3D transforms elsewhere;
+ * as GTOMRLN_PATH_SYMMETRIC (below) on every grid that path takes and with
+ * cuFFT's 3D transforms elsewhere;
  * GTOMRLN_PATH_DIRECT always uses cuFFT; GTOMRLN_PATH_FUSED runs each
  * iteration as two fused passes with the library's own transforms on
  * power-of-two grids P = 64 .. 512 (cuFFT elsewhere). */
@@ -98,8 +98,9 @@ GTOMRLN_API int gtomrln_release_caches(void);
 /* op GTOMRLN_OP_GRIDDING: each iteration as four streaming passes over the
  * Hermitian half along z of the (real) iterated spectrum, and the final map
  * as three passes that write only the cropped output, all with the library's
- * own transforms (no cuFFT plan), on the grids P = 64, 96, 128, 192, 256,
- * 512 and 800 (cuFFT elsewhere). */
+ * own transforms (no cuFFT plan), on even grids P = 16 .. 768 without a prime
+ * factor above 13, and P = 800 (cuFFT elsewhere).  Weights outside the
+ * gridding sphere, which the reference multiplies by zero, are not read. */
 #define GTOMRLN_PATH_SYMMETRIC 6
 GTOMRLN_API int gtomrln_set_path(int op, int path);
 
