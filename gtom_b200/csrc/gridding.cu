@@ -69,10 +69,18 @@ grid_init_kernel(const float* __restrict__ weight, int oldx, int oldy, int oldz,
   const int64_t base = (int64_t)row * g.rowlen;
   const int yz2 = yp * yp + zp * zp;
   if (sphere_only && row == 0 && lane == 0) Fnw[g.P / 2] = 0.f;
-  for (int x = lane; x < g.rowlen; x += 32) {
+  int end = g.rowlen;
+  if (sphere_only) {  // zeros from the sphere on, which nothing reads
+    end = 0;
+    if (yz2 < g.P * g.P / 4) {
+      end = (int)sqrtf((float)(g.P * g.P / 4 - yz2)) + 1;  // above or one past the last x inside
+      if ((end - 1) * (end - 1) + yz2 >= g.P * g.P / 4) end--;
+    }
+  }
+#pragma unroll 4
+  for (int x = lane; x < end; x += 32) {
     const float rr = r + (float)(x * x);
     const float mask = rr < (float)(g.P * g.P / 4) ? 1.f : 0.f;
-    if (sphere_only && mask == 0.f) break;  // zeros from here on, which nothing reads
     float w = 0.f;
     if (in_yz && x < oldx / 2 + 1) w = __ldg(wrow + x) * mask;
     Fw[base + x] = w;

@@ -245,15 +245,32 @@ struct GridFinalArgs {
   float* const* outs;  // one output per volume
 };
 
-// The final map's data at or beyond the sphere (from (x, y, z) on the P grid)
-// count as zero times their value: 0, or NaN for an infinity or a NaN.
-__device__ __forceinline__ float grid_final_zero(const float2* __restrict__ data, const GridFinalArgs& f, int P, int x,
-                                                 int y, int z) {
-  const int64_t src = grid_final_source(f.oldx, f.oldy, f.oldz, P, x, y, z);
-  if (src < 0) return 0.f;
-  const float2 v = __ldg(data + src);
-  return v.x * 0.f + v.y * 0.f;
-}
+// The final map's data of one column (x, y) of the P grid: grid_final_source
+// with what does not depend on z formed once.
+struct GridColumn {
+  const float2* p;  // the column in the input box, at its lowest z
+  int64_t stride;
+  int oldz, P;      // oldz 0: the column lies outside the input box
+  __device__ __forceinline__ GridColumn(const GridFinalArgs& f, int64_t vol, int P_, int x, int y) : P(P_) {
+    const int yi = (y < P / 2 + 1 ? y : y - P) + f.oldy / 2, row = f.oldx / 2 + 1;
+    const bool in = yi >= 0 && yi < f.oldy && x < row;
+    stride = (int64_t)f.oldy * row;
+    oldz = in ? f.oldz : 0;
+    p = f.data + vol * f.wstride + (in ? (int64_t)yi * row + x : 0);
+    half = f.oldz / 2;
+  }
+  __device__ __forceinline__ float2 value(int z) const {
+    const int zi = (z < P / 2 + 1 ? z : z - P) + half;
+    return zi >= 0 && zi < oldz ? __ldg(p + zi * stride) : make_float2(0.f, 0.f);
+  }
+  // Data at or beyond the sphere count as zero times their value: 0, or NaN
+  // for an infinity or a NaN.
+  __device__ __forceinline__ float zero(int z) const {
+    const float2 v = value(z);
+    return v.x * 0.f + v.y * 0.f;
+  }
+  int half;
+};
 
 // ------------------------------------- any other even grid (gridgen.cu) --
 // The same iteration and final map with run-time transform lengths; the

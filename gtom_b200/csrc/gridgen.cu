@@ -14,7 +14,7 @@
 // 522 -> 283, P = 200 2.18 -> 0.93 ms, P = 286 10.9 -> 2.28, P = 480 26.9 ->
 // 11.1, P = 720 90.5 -> 36.9.  The compiled lengths of gridsym.cu, one round
 // trip per transform, are faster where they exist: P = 160 515 -> 403 us,
-// P = 320 2.89 -> 2.33 ms, P = 768 45.7 -> 32.2.
+// P = 320 2.89 -> 2.24 ms, P = 768 45.7 -> 32.2.
 #include <algorithm>
 #include <cstdint>
 #include <map>
@@ -269,29 +269,30 @@ gridgen_final_z_kernel(float2* __restrict__ T, const __grid_constant__ GridFinal
   const bool in = x0 + c < H && zlim2 > 0;
   const int x = in ? x0 + c : 0;
   const int64_t vol = blockIdx.y, NC = (int64_t)R * P * P;
-  const float2* data = f.data + vol * f.wstride;
   // data outside the sphere must be finite, as in gridsym_final_z_kernel
   // (columns x <= P/2; where the column is inside the circle they are part of
   // it; x = P/2 is the thread's after the last one's)
-  {
+  const GridColumn col(f, vol, P, x0 + c, y), rim(f, vol, P, H, y);
+  const bool out = x0 + c <= H && !in, last = H % kGenCols == 0 && x0 + kGenCols == H && c == 0;
+  if (out || last) {
     float p = 0.f;
+#pragma unroll 4
     for (int z = g; z < P; z += G) {
-      if (x0 + c <= H && !in) p += grid_final_zero(data, f, P, x0 + c, y, z);
-      if (H % kGenCols == 0 && x0 + kGenCols == H && c == 0) p += grid_final_zero(data, f, P, H, y, z);
+      if (out) p += col.zero(z);
+      if (last) p += rim.zero(z);
     }
     if (p != 0.f) f.Fnw[vol * NC + H] = p;
   }
   if (x0 * x0 + yp * yp >= gr.r2) return;  // outside the mask's circle: read as zero by the y pass
-  const float* wsrc = (f.divide ? f.Fw : f.Fnw) + vol * NC;
+  const float* wcol = (f.divide ? f.Fw : f.Fnw) + vol * NC + (int64_t)y * R + x;
   gen_twiddles(tw, gr.tw, P);
   grid_dependency_wait();
 #pragma unroll 8
   for (int z = g; z < P; z += G) {
     const int zp = z < H ? z : P - z;
     const bool on = in && zp * zp < zlim2;
-    const int64_t src = in ? grid_final_source(f.oldx, f.oldy, f.oldz, P, x, y, z) : -1;
-    const float2 v = src >= 0 ? __ldg(data + src) : make_float2(0.f, 0.f);
-    const float w = on ? __ldg(wsrc + ((int64_t)z * P + y) * R + x) : 0.f;
+    const float2 v = in ? col.value(z) : make_float2(0.f, 0.f);
+    const float w = on ? __ldg(wcol + (int64_t)z * (P * R)) : 0.f;
     a[z * CP + c] = grid_final_apply(v, w, P, x, y, z, f.divide != 0);
   }
   const float2* r = gen_fft<true, CP>(a, b, gr.y, tw, 1, g, c);

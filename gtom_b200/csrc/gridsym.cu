@@ -47,10 +47,10 @@
 // and out in the z pass (12 B per element of the sphere): 2.4 GB at P = 512,
 // against ~8 GB for cuFFT's passes plus the blob and update kernels.
 // Measured at P = 512 (us): y 83 and 88 (76 at the copy rate), x 156 (85;
-// bound by its load/store and FP32 instructions), z 242 (132; 24 warps per SM
+// bound by its load/store and FP32 instructions), z 233 (132; 24 warps per SM
 // in phases of loads, two transforms and stores); with the whole grid they
-// were 100, 100, 156 and 335.  Ten iterations and the map 7.97 -> 6.39 ms;
-// P = 128 397 -> 228 us.
+// were 100, 100, 156 and 335.  Ten iterations and the map 7.97 -> 6.24 ms;
+// P = 128 384 -> 221 us.
 //
 // Transforms.  A real transform of length P runs as a complex transform of
 // length H = P/2 on the packed pairs (x(2n), x(2n+1)) with the usual pre-
@@ -214,10 +214,27 @@ __device__ __forceinline__ void four_step_rounds(float2* v, float2* xb, const fl
 __device__ __forceinline__ void load_twiddles(float2* tw, const float2* __restrict__ twg, int P) {
   for (int m = threadIdx.x; m < P; m += blockDim.x) tw[m] = __ldg(twg + m);
 }
-// The padded copy (tw_pad) for the x passes: P + P/16 entries.
-__device__ __forceinline__ void load_twiddles_padded(float2* tw, const float2* __restrict__ twg, int P) {
-  for (int m = threadIdx.x; m < P; m += blockDim.x) tw[tw_pad(m)] = __ldg(twg + m);
-}
+// The same in two halves, so that a CTA's first loads are in flight before it
+// waits for its table: the constructor loads, store() writes the copy (PAD:
+// tw_pad, P + P/16 entries, for the x passes).  P = 512: z pass 242 -> 233 us;
+// P = 128, ten iterations: 228 -> 221.
+template <int P, int T>
+struct Twiddles {
+  float2 w[(P + T - 1) / T];
+  __device__ __forceinline__ explicit Twiddles(const float2* __restrict__ twg) {
+#pragma unroll
+    for (int k = 0; k < (P + T - 1) / T; k++)
+      if (P % T == 0 || threadIdx.x + T * k < P) w[k] = __ldg(twg + threadIdx.x + T * k);
+  }
+  template <bool PAD = false>
+  __device__ __forceinline__ void store(float2* tw) const {
+#pragma unroll
+    for (int k = 0; k < (P + T - 1) / T; k++) {
+      const int m = threadIdx.x + T * k;
+      if (P % T == 0 || m < P) tw[PAD ? tw_pad(m) : m] = w[k];
+    }
+  }
+};
 
 // ------------------------------------------------------- TMA staging --
 // Tensor copies global -> shared completed on an mbarrier (no multicast, no
@@ -299,6 +316,13 @@ template <int P>
 constexpr int y_blocks() {
   constexpr int N1 = Split<P>::N1, T = kCols * Split<P>::N2;
   return P > 512 ? 1 : N1 >= 40 ? 384 / T : 2;
+}
+
+// The same for the final map's z and y passes, whose threads hold Split<P>'s N1.
+template <int P>
+constexpr int final_blocks() {
+  constexpr int N1 = Split<P>::N1, T = kCols * Split<P>::N2;
+  return N1 >= 40 ? (P > 512 ? 1 : 384 / T) : (N1 > 24 ? 512 : N1 > 16 ? 640 : 768) / T;
 }
 
 // Sizes of the staged y pass: a tile (16 columns x P rows) arrives as NB
@@ -434,7 +458,7 @@ gridsym_x_kernel(float2* __restrict__ W, const float2* __restrict__ twg, const f
   extern __shared__ float2 smem[];
   float2* tw = smem;
   float2* xb = smem + P + P / 16;  // after the padded twiddle table
-  load_twiddles_padded(tw, twg, P);
+  const Twiddles<P, kCols * N2> table_part(twg);
   grid_dependency_wait();
   const int t = threadIdx.x % N2, r = threadIdx.x / N2;
   const unsigned lane = threadIdx.x & 31;
@@ -448,6 +472,7 @@ gridsym_x_kernel(float2* __restrict__ W, const float2* __restrict__ twg, const f
   // Hermitian spectrum, is dropped as cuFFT's C2R drops it); the x = P/2 term
   // lies outside the sphere
   const float2 xH = make_float2(0.f, 0.f);
+  table_part.template store<true>(tw);
   if (t == 0) v[0].y = 0.f;
   __syncthreads();  // twiddles in place
   // pre-twiddle of the C2R.  The partner H - k of k = t + N2 m is element
@@ -580,7 +605,7 @@ gridsym_z_kernel(float2* __restrict__ W, const float* __restrict__ Fw, float* __
   extern __shared__ float2 smem[];
   float2* tw = smem;
   float2* xb = smem + P;
-  load_twiddles(tw, twg, P);
+  const Twiddles<P, kCols * N2> table_part(twg);
   grid_dependency_wait();
   const int c = threadIdx.x & (kCols - 1), t = threadIdx.x / kCols;
   const int y = blockIdx.x / (H / kCols);
@@ -609,6 +634,7 @@ gridsym_z_kernel(float2* __restrict__ W, const float* __restrict__ Fw, float* __
       if (in) xH = make_float2(wc[H * EW].x, 0.f);
       v[0].y = 0.f;
     }
+    table_part.store(tw);
     // pre-twiddle (exp(-) sum) with the partners H - k through shared memory
     __syncthreads();  // twiddles in place
 #pragma unroll
@@ -697,7 +723,10 @@ gridsym_z_kernel(float2* __restrict__ W, const float* __restrict__ Fw, float* __
     }
   }
   if (MODE == kZIter && !write_next) return;  // uniform
-  if (MODE == kZFirst) __syncthreads();  // twiddles in place
+  if (MODE == kZFirst) {
+    table_part.store(tw);
+    __syncthreads();  // twiddles in place
+  }
   four_step<H, true, false, false, 2>(v, xb, tw, t, c);
   // post-twiddle (exp(+)) with the partners (H - k) mod H through shared memory
   __syncthreads();
@@ -728,7 +757,7 @@ gridsym_z_kernel(float2* __restrict__ W, const float* __restrict__ Fw, float* __
 // one that is not finite makes the whole map NaN, as its product with zero
 // would (the flag Fnw[P/2], zeroed by grid_init_kernel).
 template <int P>
-__global__ void __launch_bounds__(kCols * Split<P>::N2, y_blocks<P>())
+__global__ void __launch_bounds__(kCols * Split<P>::N2, final_blocks<P>())
 gridsym_final_z_kernel(float2* __restrict__ T, GridFinalArgs f, const float2* __restrict__ twg) {
   constexpr int H = P / 2, R = H + 1;
   constexpr int N1 = Split<P>::N1, N2 = Split<P>::N2;
@@ -736,7 +765,7 @@ gridsym_final_z_kernel(float2* __restrict__ T, GridFinalArgs f, const float2* __
   extern __shared__ float2 smem[];
   float2* tw = smem;
   float2* xb = smem + P;
-  load_twiddles(tw, twg, P);
+  const Twiddles<P, kCols * N2> table_part(twg);
   grid_dependency_wait();
   const int c = threadIdx.x & (kCols - 1), t = threadIdx.x / kCols;
   const int y = blockIdx.x / (H / kCols);
@@ -744,23 +773,25 @@ gridsym_final_z_kernel(float2* __restrict__ T, GridFinalArgs f, const float2* __
   const int yp = y < H ? y : P - y;
   const int zlim2 = H * H - x * x - yp * yp;
   const int64_t vol = blockIdx.y;
-  const float2* data = f.data + vol * f.wstride;
-  const float* Fw = f.Fw + vol * NC;
   float* Fnw = f.Fnw + vol * NC;
-  const bool rim = x0 + kCols == H && c == 0;  // also sees to x = P/2
-  if (x0 * x0 + yp * yp >= H * H || rim) {
+  const float* wcol = (f.divide ? f.Fw + vol * NC : Fnw) + (int64_t)y * R + x;
+  // the column's and x = P/2's data, signed z from the middle
+  const GridColumn col(f, vol, P, x, y), rim(f, vol, P, H, y);
+  const bool outside = x0 * x0 + yp * yp >= H * H;  // of the mask's circle: read as zero by the y pass
+  if (outside || (x0 + kCols == H && c == 0)) {
     float p = 0.f;
-#pragma unroll
+#pragma unroll 8
     for (int m = 0; m < N1; m++) {
-      if (x0 * x0 + yp * yp >= H * H) p += grid_final_zero(data, f, P, x, y, t + N2 * m);
-      if (rim) p += grid_final_zero(data, f, P, H, y, t + N2 * m);
+      const int z = t + N2 * m;
+      if (outside) p += col.zero(z);
+      if (x0 + kCols == H && c == 0) p += rim.zero(z);
     }
     if (p != 0.f) Fnw[H] = p;
+    if (outside) return;
   }
-  if (x0 * x0 + yp * yp >= H * H) return;  // outside the mask's circle: read as zero by the y pass
   float2* tv = T + vol * ((int64_t)R * P * f.ori);
-  // the loads of CH elements first (those outside the input box are zero), then their corrections
-  const float* wsrc = f.divide ? Fw : Fnw;
+  // the loads of CH elements first (those outside the input box are zero),
+  // then their corrections
   constexpr int CH = N1 <= 20 ? N1 : (N1 % 20 == 0 ? 20 : (N1 % 16 == 0 ? 16 : 12));
   static_assert(N1 % CH == 0, "gridsym_final_z_kernel: chunks");
   float2 v[N1];
@@ -771,10 +802,8 @@ gridsym_final_z_kernel(float2* __restrict__ T, GridFinalArgs f, const float2* __
     for (int q = 0; q < CH; q++) {
       const int z = t + N2 * (m0 + q);
       const int zp = z < H ? z : P - z;
-      const bool on = zp * zp < zlim2;
-      const int64_t src = grid_final_source(f.oldx, f.oldy, f.oldz, P, x, y, z);
-      v[m0 + q] = src >= 0 ? __ldg(data + src) : make_float2(0.f, 0.f);
-      wt[q] = on ? __ldg(wsrc + ((int64_t)z * P + y) * R + x) : 0.f;
+      v[m0 + q] = col.value(z);
+      wt[q] = zp * zp < zlim2 ? __ldg(wcol + (int64_t)z * (P * R)) : 0.f;
     }
 #pragma unroll
     for (int q = 0; q < CH; q++)
@@ -786,6 +815,7 @@ gridsym_final_z_kernel(float2* __restrict__ T, GridFinalArgs f, const float2* __
     for (int m = 0; m < N1; m++) p += v[m].x + v[m].y;
     if (p != 0.f) Fnw[H] = p;
   }
+  table_part.store(tw);
   __syncthreads();  // twiddles in place
   four_step<P, true, false, false, 1>(v, xb, tw, t, c);
 #pragma unroll
@@ -799,14 +829,14 @@ gridsym_final_z_kernel(float2* __restrict__ T, GridFinalArgs f, const float2* __
 // written to rows 0 .. ori-1 of the plane (each CTA has read its whole
 // column before it writes).  Tiles: 16 consecutive x < P/2 at one zc.
 template <int P>
-__global__ void __launch_bounds__(kCols * Split<P>::N2, y_blocks<P>())
+__global__ void __launch_bounds__(kCols * Split<P>::N2, final_blocks<P>())
 gridsym_final_y_kernel(float2* __restrict__ T, int ori, int off, const float2* __restrict__ twg) {
   constexpr int H = P / 2, R = H + 1;
   constexpr int N1 = Split<P>::N1, N2 = Split<P>::N2;
   extern __shared__ float2 smem[];
   float2* tw = smem;
   float2* xb = smem + P;
-  load_twiddles(tw, twg, P);
+  const Twiddles<P, kCols * N2> table_part(twg);
   grid_dependency_wait();
   const int c = threadIdx.x & (kCols - 1), t = threadIdx.x / kCols;
   const int zc = blockIdx.x / (H / kCols), x = (blockIdx.x - zc * (H / kCols)) * kCols + c;
@@ -817,6 +847,7 @@ gridsym_final_y_kernel(float2* __restrict__ T, int ori, int off, const float2* _
     const int y = t + N2 * m, yp = y < H ? y : P - y;
     v[m] = yp * yp + x * x < H * H ? col[(int64_t)y * R] : make_float2(0.f, 0.f);
   }
+  table_part.store(tw);
   __syncthreads();  // twiddles in place
   four_step<P, true, false, false, 1>(v, xb, tw, t, c);
 #pragma unroll
@@ -839,7 +870,7 @@ gridsym_final_x_kernel(const float2* __restrict__ T, GridFinalArgs f, const floa
   extern __shared__ float2 smem[];
   float2* tw = smem;
   float2* xb = smem + P + P / 16;  // after the padded twiddle table
-  load_twiddles_padded(tw, twg, P);
+  const Twiddles<P, kCols * N2> table_part(twg);
   grid_dependency_wait();
   const int t = threadIdx.x % N2, r = threadIdx.x / N2;
   const unsigned lane = threadIdx.x & 31;
@@ -854,6 +885,7 @@ gridsym_final_x_kernel(const float2* __restrict__ T, GridFinalArgs f, const floa
 #pragma unroll
   for (int m = 0; m < N1; m++) v[m] = in ? row[t + N2 * m] : make_float2(0.f, 0.f);
   const float2 xH = make_float2(0.f, 0.f);  // x = P/2 lies outside the mask's sphere
+  table_part.template store<true>(tw);
   if (t == 0) v[0].y = 0.f;
   __syncthreads();  // twiddles in place
   {
