@@ -13,8 +13,8 @@
 // iterations and the map (cuFFT against here): P = 40 393 -> 209 us, P = 88
 // 522 -> 283, P = 200 2.18 -> 0.93 ms, P = 286 10.9 -> 2.28, P = 480 26.9 ->
 // 11.1, P = 720 90.5 -> 36.9.  The compiled lengths of gridsym.cu, one round
-// trip per transform, are faster where they exist: P = 160 515 -> 403 us,
-// P = 320 2.89 -> 2.24 ms, P = 768 45.7 -> 32.2.
+// trip per transform, are faster where they exist: P = 160 515 -> 385 us,
+// P = 320 2.89 -> 2.16 ms, P = 768 45.7 -> 31.3.
 #include <algorithm>
 #include <cstdint>
 #include <map>

@@ -311,7 +311,7 @@ constexpr int pass_blocks(int n1_24) {
 template <int P>
 constexpr int x_blocks() { return pass_blocks<P>(512); }
 template <int P>
-constexpr int z_blocks() { return pass_blocks<P>(640); }
+constexpr int z_blocks() { return pass_blocks<P>(512 % (kCols * Split<P / 2>::N2) ? 640 : 512); }
 template <int P>
 constexpr int y_blocks() {
   constexpr int N1 = Split<P>::N1, T = kCols * Split<P>::N2;
@@ -656,7 +656,11 @@ gridsym_z_kernel(float2* __restrict__ W, const float* __restrict__ Fw, float* __
     const int zp = z < H ? z : P - z;
     return zp * zp < zlim2;
   };
-  constexpr int CH = N1 < 2 ? N1 : 2;
+  // The weights' loads in flight per thread, as many pairs as its registers
+  // take: the chunks' latencies follow one another (P = 320, 40 elements a
+  // thread: ten iterations 2.24 ms with two pairs, 2.16 with four, 2.41 with
+  // eight; P = 512, 16 elements: four no faster).
+  constexpr int CH = N1 >= 40 || N1 == 20 || (N1 == 24 && z_blocks<P>() * kCols * N2 <= 512) ? 4 : 2;
 #pragma unroll
   for (int m0 = 0; m0 < N1; m0 += CH) {
     // loads of CH pairs first (in flight together), then the updates
