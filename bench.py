@@ -528,8 +528,10 @@ def time_gridding(G, torch, acc_ft, acc_w, n, D, dev):
     # the default path on this grid: four passes over the (P/2+1) x P x
     # (P/2+1) complex work array W (16 B per element each) plus Fw in and Fnw
     # in and out (12 B per spectrum element) per iteration
-    nw = (P // 2 + 1) * P * (P // 2 + 1)
-    sym_bytes = 4 * 16 * nw + 12 * nc
+    # inside the sphere: columns x < P/2, and on the sides that face the
+    # spectrum only those inside its circle
+    nw, circle = (P // 2 + 1) * P * (P // 2), math.pi / 4
+    sym_bytes = int((4 + 4 * circle) * 8 * nw + 12 * (2 / 3) * math.pi * (P // 2) ** 3)
     per_it = (ms10 - ms1) / 9
     res = {"ms_10_iterations": round(ms10, 3), "ms_per_iteration": round(per_it, 4), "P": P,
            "path": "symmetric (four passes over the Hermitian half along z)" if P in (64, 128, 256, 512) else "cufft",
