@@ -272,6 +272,7 @@ gridgen_final_z_kernel(float2* __restrict__ T, const __grid_constant__ GridFinal
   // data outside the sphere must be finite, as in gridsym_final_z_kernel
   // (columns x <= P/2; where the column is inside the circle they are part of
   // it; x = P/2 is the thread's after the last one's)
+  grid_dependency_wait();  // the flag's zero is the predecessor's where no iteration ran
   const GridColumn col(f, vol, P, x0 + c, y), rim(f, vol, P, H, y);
   const bool out = x0 + c <= H && !in, last = H % kGenCols == 0 && x0 + kGenCols == H && c == 0;
   if (out || last) {
@@ -286,7 +287,6 @@ gridgen_final_z_kernel(float2* __restrict__ T, const __grid_constant__ GridFinal
   if (x0 * x0 + yp * yp >= gr.r2) return;  // outside the mask's circle: read as zero by the y pass
   const float* wcol = (f.divide ? f.Fw : f.Fnw) + vol * NC + (int64_t)y * R + x;
   gen_twiddles(tw, gr.tw, P);
-  grid_dependency_wait();
 #pragma unroll 8
   for (int z = g; z < P; z += G) {
     const int zp = z < H ? z : P - z;

@@ -94,16 +94,20 @@ def test_batch_matches_single_calls(gtom_lib, cuda):
         assert rel_l2(g.cpu().numpy(), s.out.cpu().numpy()) <= 1e-4
 
 
+@pytest.mark.parametrize("iterations", [0, 3])
 @pytest.mark.parametrize("ori", [20, 32])
 @pytest.mark.parametrize("at", ["corner", "column", "nyquist", "inside"])
-def test_data_that_are_not_finite_spread(gtom_lib, cuda, ori, at):
+def test_data_that_are_not_finite_spread(gtom_lib, cuda, ori, at, iterations):
     """Zero times a NaN is not zero: the map is NaN on every path, also for
-    data outside the sphere, whose columns the symmetric passes leave out."""
+    data outside the sphere, whose columns the symmetric passes leave out, and
+    also where no iteration lies between the start and the final map."""
     data, w, D = _inputs(ori)
     data = data.reshape(D, D, D // 2 + 1).copy()
     c = D // 2
-    data[{"corner": (1, 1, 0), "column": (c, 1, D // 2 - 1), "nyquist": (c, c, D // 2), "inside": (c, c + 2, 1)}[at]] = complex(np.nan, np.nan)
+    data[{"corner": (1, 1, 0), "column": (c, 1, D // 2 - 1), "nyquist": (c, c, D // 2),
+          "inside": (c, c + 2, 1)}[at]] = complex(np.nan, np.nan)
     for path in ("direct", "symmetric"):
         out = torch.zeros(ori ** 3, device="cuda")
-        _on(path, lambda: G.d_ReconstructGridding(_dev(data.reshape(-1)), _dev(w), out, (ori,) * 3, (D,) * 3, 2, 0, 0, 3))
+        _on(path, lambda: G.d_ReconstructGridding(_dev(data.reshape(-1)), _dev(w), out, (ori,) * 3, (D,) * 3, 2, 0, 0,
+                                                  iterations))
         assert not torch.isfinite(out).any()
