@@ -172,7 +172,8 @@ backproject_direct_kernel(float2* __restrict__ volft_base, float* __restrict__ v
 }
 
 // Adds the packed scratch to the volumes; voxels that received nothing are
-// left alone.
+// left alone.  By reductions, as the plain form's targets are added: calls
+// that overlap on other streams may insert into the same volumes.
 __global__ void __launch_bounds__(256)
 backproject_unpack_kernel(const float4* __restrict__ packed, float2* __restrict__ volft, float* __restrict__ volw,
                           int64_t n) {
@@ -180,9 +181,8 @@ backproject_unpack_kernel(const float4* __restrict__ packed, float2* __restrict_
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const float4 p = packed[i];
     if (p.x == 0.f && p.y == 0.f && p.z == 0.f) continue;
-    const float2 v = volft[i];
-    volft[i] = make_float2(v.x + p.x, v.y + p.y);
-    volw[i] += p.z;
+    red_add2((float*)(volft + i), p.x, p.y);
+    red_add(volw + i, p.z);
   }
 }
 

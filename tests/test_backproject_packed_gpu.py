@@ -54,3 +54,33 @@ def test_packed_matches_the_port(gtom_lib, cuda):
     of, ow = np.zeros(nvox, np.complex64), np.zeros(nvox, np.float32)
     O.backproject(of, ow, V, ft, None, n, n // 2, mats, decentered=False, fp32=True)
     assert rel_l2(vf.cpu().numpy(), of) <= 1e-5 and rel_l2(vw.cpu().numpy(), ow) <= 1e-5
+
+
+def test_overlapping_calls_lose_nothing(gtom_lib, cuda):
+    """Forty packed insertions on two streams into one pair of volumes: each
+    voxel holds all of them.  An addition lost to the other stream would miss
+    one call's share (a fortieth) of its voxel; the order of forty FP32 sums
+    makes 40 * 2^-24."""
+    rng = np.random.default_rng(8)
+    n, batch, V, calls = 32, 1300, 65, 20
+    e, nvox = O.elements_fft(n), (V // 2 + 1) * V * V
+    mats = torch.from_numpy(G.matrices_from_angles(random_angles(rng, batch), 2.0)).cuda().reshape(-1)
+    ft = torch.ones(batch * e, dtype=torch.complex64, device="cuda")
+
+    def insert(vf, vw):
+        G.d_rlnBackproject(vf, vw, (V, V, V), ft, None, (n, n, 1), n // 2, mats, None, (1, 0, 0, 1), 0.0, False, False,
+                           batch)
+
+    new = lambda: (torch.zeros(nvox, dtype=torch.complex64, device="cuda"), torch.zeros(nvox, device="cuda"))
+    one, both = new(), new()
+    insert(*one)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for _ in range(calls):
+        for s in streams:
+            with torch.cuda.stream(s):
+                insert(*both)
+    torch.cuda.synchronize()
+    want = 2 * calls * one[1].double()
+    assert ((both[1].double() - want).abs() <= 1e-5 * want).all()
+    assert rel_l2(both[0].cpu().numpy(), (2 * calls * one[0]).cpu().numpy()) <= 1e-5
