@@ -706,8 +706,10 @@ backproject_segment_kernel(float2* __restrict__ volft_base, float* __restrict__ 
                 val.y *= sv;
                 pw *= sw;
                 // larger terms (or non-finite ones) than the scale allows: the
-                // item is redone in FP32
-                if (!(fmaxf(fabsf(val.x), fmaxf(fabsf(val.y), fabsf(pw))) < 536870912.f)) danger |= 0x80000000u;
+                // item is redone in FP32 (each compared by itself: a maximum
+                // of the three would drop a NaN)
+                if (!(fabsf(val.x) < 536870912.f && fabsf(val.y) < 536870912.f && fabsf(pw) < 536870912.f))
+                  danger |= 0x80000000u;
               }
 #pragma unroll
               for (int i = 0; i < 8; i++) {
