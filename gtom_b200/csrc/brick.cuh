@@ -40,7 +40,6 @@ struct BrickItem {
   int brick;      // brick index
   int offset;     // first entry in the pair list (segment plan: first record)
   int count;      // bins (slice, pixel run) or records in this item
-  int exclusive;  // 1 if this is the brick's only item (no other CTA writes it)
 };
 
 // A (slice, brick) bin: `count` pixel ids starting at entries[start]; the

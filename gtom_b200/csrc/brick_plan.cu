@@ -457,7 +457,7 @@ pairs_scan_kernel(const int* __restrict__ counts, const int* __restrict__ order,
       cursor[b] = 0;
       const int size = ni ? (c + ni - 1) / ni : 0;  // equal shares
       for (int k = 0; k < ni; k++)
-        items[ioff + k] = {b, off + k * size, min(size, c - k * size), ni == 1 ? 1 : 0};
+        items[ioff + k] = {b, off + k * size, min(size, c - k * size)};
     }
     carry_c += __shfl_sync(0xffffffffu, wc, 31);
     carry_i += __shfl_sync(0xffffffffu, wi, 31);

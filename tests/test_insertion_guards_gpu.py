@@ -1,5 +1,5 @@
 """What an insertion must keep whichever kernel takes it: a value that is not
-finite reaches the map."""
+finite reaches the map, and calls that overlap on two streams lose nothing."""
 import numpy as np
 import pytest
 import torch
@@ -51,3 +51,37 @@ def test_not_finite_pixel_reaches_the_map(gtom_lib, cuda, n, where, value):
         vf, vw = _insert(path, V, n, mats, ft, w)
         bad.append(torch.stack([~torch.isfinite(vf.real), ~torch.isfinite(vf.imag), ~torch.isfinite(vw)]))
     assert bad[1].any() and torch.equal(bad[0], bad[1])
+
+
+@pytest.mark.parametrize("path", ["brick", "segment", "segment_fp32"])
+@pytest.mark.parametrize("decentered", [False, True])
+def test_overlapping_calls_lose_nothing(gtom_lib, cuda, path, decentered):
+    """Twenty insertions on two streams into one pair of volumes: an addition
+    lost to the other stream would miss a twentieth of its voxel."""
+    rng = np.random.default_rng(8)
+    n, batch, calls = 32, 300, 10
+    V = 2 * n if decentered else 2 * n + 1
+    nv = (V // 2 + 1) * V * V
+    mats = _mats(rng, batch)
+    ft = torch.ones(batch * O.elements_fft(n), dtype=torch.complex64, device="cuda")
+
+    def insert(vf, vw):
+        G.d_rlnBackproject(vf, vw, (V, V, V), ft, None, (n, n, 1), n // 2, mats, None, (1, 0, 0, 1), 0.0, decentered,
+                           False, batch)
+
+    new = lambda: (torch.zeros(nv, dtype=torch.complex64, device="cuda"), torch.zeros(nv, device="cuda"))
+    one, both = new(), new()
+    G.set_path("backproject", path)
+    try:
+        insert(*one)
+        torch.cuda.synchronize()
+        streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+        for _ in range(calls):
+            for s in streams:
+                with torch.cuda.stream(s):
+                    insert(*both)
+        torch.cuda.synchronize()
+    finally:
+        G.set_path("backproject", "auto")
+    want = 2 * calls * one[1].double()
+    assert ((both[1].double() - want).abs() <= 1e-4 * want).all()
