@@ -419,25 +419,50 @@ static std::atomic<int> g_path[3] = {{GTOMRLN_PATH_AUTO}, {GTOMRLN_PATH_AUTO}, {
 
 int path_choice(int op) { return (op >= 0 && op <= 2) ? g_path[op].load() : GTOMRLN_PATH_AUTO; }
 
-// Samples from which the row-segment kernels win, by volume edge, from sweeps
-// at padding 2 (n = V / 2; us, direct against segment):
-// projector      n = 256: 300 slices 282 vs 292, 1 000: 866 vs 493; n = 192:
-//                1 000: 318 vs 330, 3 000: 901 vs 640; n = 160: 1 000: 193 vs
-//                251, 3 000: 531 vs 505; n = 128: 3 000: 341 vs 396, 10 000:
-//                1 068 vs 898; n = 96, 10 000: 610 vs 645;
-// backprojector  n = 256: 100 slices 655 vs 750, 150: 921 vs 784; n = 192:
-//                100: 302 vs 408, 300: 773 vs 464; n = 160: 100: 170 vs 268,
-//                300: 388 vs 308; n = 128: 300: 177 vs 210, 450: 248 vs 206;
-//                n = 96, 3 000: 477 vs 410; n = 64: 3 000: 240 vs 243, 10 000:
-//                670 vs 543; n = 48, 10 000: 407 vs 395 (below V = 321 the
-//                direct kernel reduces into a packed scratch).
-// The direct kernels' cost per sample grows once the volume leaves L2; the
-// segment kernels pay a plan and the staging or flush of every brick first.
-bool brick_path_pays(int op, int V, double rmax, unsigned batch) {
-  const double samples = 1.5707963 * rmax * rmax * batch;
-  if (op == GTOMRLN_OP_BACKPROJECT)
-    return V >= 256 ? samples >= (V >= 448 ? 3.1e6 : 2.5e6) : V >= 128 && batch >= 2000 && samples >= 6e6;
+static double slice_samples(double rmax) { return 1.5707963 * rmax * rmax; }
+
+// Samples from which the row-segment projector wins, by volume edge, from
+// sweeps at padding 2 (n = V / 2; us, direct against segment):
+// n = 256: 300 slices 282 vs 292, 1 000: 866 vs 493; n = 192: 1 000: 318 vs
+// 330, 3 000: 901 vs 640; n = 160: 1 000: 193 vs 251, 3 000: 531 vs 505;
+// n = 128: 3 000: 341 vs 396, 10 000: 1 068 vs 898; n = 96, 10 000: 610 vs
+// 645.  The direct kernel's cost per sample grows once the volume leaves L2;
+// the segment kernel pays a plan and the staging of every brick first.
+bool project_segment_pays(int V, double rmax, unsigned batch) {
+  const double samples = slice_samples(rmax) * batch;
   return samples >= (V >= 512 ? 11e6 : V >= 384 ? 19e6 : V >= 320 ? 24e6 : V >= 256 ? 28e6 : 1e300);
+}
+
+// Insertions.  Fixed-point sums hold a small sum beside large ones to a step
+// of 2^-25 of the brick's largest sampled magnitude, where the direct
+// kernel's are FP32: AUTO takes them for large batches into large volumes
+// only (256^3, 10 000 slices: 4.64 ms, 7.9 with FP32 atomics, 57 direct).
+// Elsewhere the segment kernel sums in FP32, from the samples on with which
+// that wins (us, direct against segment):
+// n = 140 (V = 281): 300 slices 201 vs 216, 600: 372 vs 324; n = 150: 200:
+// 181 vs 211, 300: 257 vs 247; n = 160: 150: 193 vs 233, 300: 350 vs 283;
+// n = 180: 100: 211 vs 285, 200: 419 vs 326; n = 192: 100: 270 vs 329, 150:
+// 394 vs 353; n = 224: 100: 427 vs 477, 150: 610 vs 513; n = 256: 100: 591 vs
+// 672, 150: 886 vs 721; with magnification and curvature a tenth slower than
+// that.  Where the direct kernel has its packed scratch (V <= 275 for one
+// volume) it stays ahead (n = 128, 1 000: 372 vs 396; n = 100, 3 333: 542 vs
+// 728).  The samples are those of one volume: every volume has its own bricks
+// (n = 64, 4 096 slices into 1 024 volumes: 1.9 ms direct, 10 ms in bricks).
+InsertSums insert_auto(int V, double rmax, unsigned batch, int volumes, bool packed) {
+  if ((V >= 384 && batch >= 300) || (V >= 256 && batch >= 6000)) return InsertSums::kFixed;
+  if (packed || V < 256 || volumes < 1) return InsertSums::kDirect;
+  const double samples = slice_samples(rmax) * batch / volumes;
+  return samples >= (V >= 320 && V < 448 ? 2.3e6 : 3.3e6) ? InsertSums::kFp32 : InsertSums::kDirect;
+}
+
+// The shifted insertion (its direct kernel has no packed scratch, its segment
+// kernel FP32 sums only; us, direct against segment): n = 64: 2 000 slices
+// 282 vs 307, 3 333: 458 vs 291; n = 96: 1 000: 288 vs 624, 2 000: 544 vs
+// 472; n = 128: 300: 162 vs 206, 400: 210 vs 203; n = 160: 150: 195 vs 208,
+// 300: 356 vs 249; n = 256: 100: 613 vs 607, 150: 921 vs 653.
+bool insert_shifted_segment_pays(int V, double rmax, unsigned batch) {
+  const double samples = slice_samples(rmax) * batch;
+  return V >= 256 ? samples >= (V >= 448 ? 3.1e6 : 2.5e6) : V >= 128 && batch >= 2000 && samples >= 6e6;
 }
 
 // Defaults measured on the B200 at 256^3 (padding 2) with 10,000-slice

@@ -1198,13 +1198,25 @@ static int backproject_launch(float* d_volumeft, float* d_volumeweights, int vx,
   const int choice = path_choice(GTOMRLN_OP_BACKPROJECT);
   const bool plain = !d_ivolume && mag.x == 1.f && mag.y == 0.f && mag.z == 0.f && mag.w == 1.f &&
                      a.ewalddiaminv == 0.f;
+  // The direct kernel's packed scratch, where that pays: it halves the
+  // reductions (8 instead of 16 per sample, each ~5.5 ps of the L2's rate)
+  // for clearing and adding 16 bytes per voxel (~11 ps) and two small
+  // launches, and its reductions stay in L2 up to a scratch of 160 MB (of
+  // which a sphere is touched; V = 275 for one volume).  64^3, 1 000 slices:
+  // 145 -> 90 us; 100^3, 3 333 slices into two volumes: 985 -> 645 us.
+  const int known_vol = d_ivolume ? std::max(0, nvol_hint) : 1;
+  const double samples = (ndp == 3 ? 2.0943951 * rmax : 1.5707963) * (double)rmax * rmax * batch;
+  const int64_t voxels = a.nvox * (int64_t)known_vol;
+  const bool packs = d_volumeft && d_volumeweights && known_vol >= 1 && voxels <= (160 << 20) / 16 &&
+                     samples >= 0.5 * (double)voxels + 262144.0;
   // (the brick plans' integer square roots take radii below 4 096: seg_isqrt)
-  const bool brick = ndp == 2 && vx == vy && vx == vz && vx >= 4 && a.rmax2 <= (1 << 24) &&
-                     (d_volumeft || d_volumeweights) &&
-                     (choice == GTOMRLN_PATH_BRICK || choice == GTOMRLN_PATH_SEGMENT ||
-                      choice == GTOMRLN_PATH_SEGMENT_FP32 ||
-                      (choice == GTOMRLN_PATH_AUTO && brick_path_pays(GTOMRLN_OP_BACKPROJECT, vx, (double)rmax, batch)));
-  const bool fixed_point = choice != GTOMRLN_PATH_SEGMENT_FP32;
+  InsertSums sums = InsertSums::kDirect;
+  if (ndp == 2 && vx == vy && vx == vz && vx >= 4 && a.rmax2 <= (1 << 24) && (d_volumeft || d_volumeweights)) {
+    if (choice == GTOMRLN_PATH_AUTO) sums = insert_auto(vx, (double)rmax, batch, known_vol, packs);
+    if (choice == GTOMRLN_PATH_BRICK || choice == GTOMRLN_PATH_SEGMENT) sums = InsertSums::kFixed;
+    if (choice == GTOMRLN_PATH_SEGMENT_FP32) sums = InsertSums::kFp32;
+  }
+  const bool brick = sums != InsertSums::kDirect, fixed_point = sums == InsertSums::kFixed;
   if (brick && plain)
     return backproject_brick(d_volumeft, d_volumeweights, d_projft, d_projweights, d_matrices, a, (int)rmax,
                              decentered, square, batch, stream, choice == GTOMRLN_PATH_BRICK ? 0 : 1, false,
@@ -1238,19 +1250,10 @@ static int backproject_launch(float* d_volumeft, float* d_volumeweights, int vx,
                                decentered, square, batch, stream, 1, true, d_ivolume, nvol, fixed_point);
   }
 
-  // The direct kernel, through a packed scratch where that pays: it halves
-  // the reductions (8 instead of 16 per sample, each ~5.5 ps of the L2's
-  // rate) for clearing and adding 16 bytes per voxel (~11 ps) and two small
-  // launches, and its reductions stay in L2 up to a scratch of 160 MB (of
-  // which a sphere is touched).  64^3, 1 000 slices: 145 -> 94 us; 100^3,
-  // 3 333 slices into two volumes: 985 -> 656 us.  Not under stream capture,
-  // where the call allocates nothing.
-  const int nvol = d_ivolume ? nvol_hint : 1;
-  const double samples = (ndp == 3 ? 2.0943951 * rmax : 1.5707963) * (double)rmax * rmax * batch;
-  const int64_t voxels = a.nvox * (int64_t)nvol;
+  // The direct kernel.  No packed scratch under stream capture, where the
+  // call allocates nothing.
   const dim3 grid((unsigned)(a.tiles * (int64_t)batch));
-  if (d_volumeft && d_volumeweights && nvol >= 1 && voxels <= (160 << 20) / 16 &&
-      samples >= 0.5 * (double)voxels + 262144.0) {
+  if (packs) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     float4* packed = nullptr;
     if (cudaStreamIsCapturing(stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone &&
@@ -1362,7 +1365,7 @@ int gtomrln_backproject_shifted(float* d_volumeft, float* d_volumeweights, int v
   const int choice = path_choice(GTOMRLN_OP_BACKPROJECT);
   if (ndp == 2 && vx == vy && vx == vz && vx >= 4 && a.rmax2 <= (1 << 24) && (d_volumeft || d_volumeweights) &&
       (choice == GTOMRLN_PATH_BRICK || choice == GTOMRLN_PATH_SEGMENT ||
-       (choice == GTOMRLN_PATH_AUTO && brick_path_pays(GTOMRLN_OP_BACKPROJECT, vx, (double)rmax, batch))))
+       (choice == GTOMRLN_PATH_AUTO && insert_shifted_segment_pays(vx, (double)rmax, batch))))
     return backproject_shifted_brick(d_volumeft, d_volumeweights, d_projft, d_projweights, d_matrices, d_shifts,
                                      d_globalweights, a, (int)rmax, batch, (cudaStream_t)stream);
   dim3 grid((unsigned)(a.tiles * (int64_t)batch));

@@ -48,12 +48,17 @@ void matrices_from_angles(const float* angles, float supersample, unsigned batch
 // Implementation chosen for op (GTOMRLN_OP_*) by gtomrln_set_path.
 int path_choice(int op);
 
-// Whether GTOMRLN_PATH_AUTO takes the brick-major (row-segment) kernels for
-// op on a cubic volume of edge V and a batch of 2D slices of radius rmax:
-// they win once the volume no longer fits in L2 and the samples amortise
-// their plan and the bricks' staging, while the direct kernels, whose
-// gathers and reductions then stay in L2, win on smaller work (abi.cu).
-bool brick_path_pays(int op, int V, double rmax, unsigned batch);
+// What GTOMRLN_PATH_AUTO takes for a batch of 2D slices of radius rmax and a
+// cubic volume of edge V: the brick-major (row-segment) kernels win once the
+// volume no longer fits in L2 and the samples amortise their plan and the
+// bricks' staging, the direct kernels, whose gathers and reductions then stay
+// in L2, on smaller work (abi.cu).  volumes: the targets of the insertion, 0
+// if the call does not know; packed: whether the direct kernel has its packed
+// scratch.
+enum class InsertSums { kDirect, kFp32, kFixed };
+bool project_segment_pays(int V, double rmax, unsigned batch);
+InsertSums insert_auto(int V, double rmax, unsigned batch, int volumes, bool packed);
+bool insert_shifted_segment_pays(int V, double rmax, unsigned batch);
 
 // Launch shape of the brick kernels for op: brick edge in voxels, threads
 // per CTA, and the most slices one work item takes (gtomrln_set_brick_tuning).

@@ -560,7 +560,7 @@ int gtomrln_project(const float* d_volumeft, int vx, int vy, int vz, float* d_pr
   // the brick plans' integer square roots take radii below 4 096 (seg_isqrt)
   if (ndp == 2 && vx == vy && vx == vz && vx >= 4 && a.rmax2 <= (1 << 24) &&
       (choice == GTOMRLN_PATH_BRICK || choice == GTOMRLN_PATH_SEGMENT ||
-       (choice == GTOMRLN_PATH_AUTO && brick_path_pays(GTOMRLN_OP_PROJECT, vx, (double)a.rmax, batch))))
+       (choice == GTOMRLN_PATH_AUTO && project_segment_pays(vx, (double)a.rmax, batch))))
     return project_brick(d_volumeft, d_proj, d_matrices, a, batch, (cudaStream_t)stream,
                          choice == GTOMRLN_PATH_BRICK ? 0 : 1);
   ArrayFetch f{(const float2*)d_volumeft, a.P, a.P / 2 + 1, a.nvox - 1};
@@ -621,7 +621,7 @@ int gtomrln_project_shifted(const float* d_volumeft, int vx, int vy, int vz, flo
   // the brick plans' integer square roots take radii below 4 096 (seg_isqrt)
   if (ndp == 2 && vx == vy && vx == vz && vx >= 4 && a.rmax2 <= (1 << 24) &&
       (choice == GTOMRLN_PATH_BRICK || choice == GTOMRLN_PATH_SEGMENT ||
-       (choice == GTOMRLN_PATH_AUTO && brick_path_pays(GTOMRLN_OP_PROJECT, vx, (double)a.rmax, batch))))
+       (choice == GTOMRLN_PATH_AUTO && project_segment_pays(vx, (double)a.rmax, batch))))
     return project_brick(d_volumeft, d_proj, d_matrices, a, batch, (cudaStream_t)stream, 1,
                          ShiftPost{d_shifts, d_globalweights});
   ArrayFetch f{(const float2*)d_volumeft, a.P, a.P / 2 + 1, a.nvox - 1};

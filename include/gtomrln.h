@@ -67,9 +67,13 @@ GTOMRLN_API int gtomrln_release_caches(void);
  * GTOMRLN_OP_BACKPROJECT; path: GTOMRLN_PATH_AUTO (default: brick-major with
  * row segments for 2D slices whose geometry allows it, once the volume is
  * too large for L2 and the batch's samples (pi / 2 rmax^2 per slice)
- * amortise the plan — backprojector: edge >= 256 and 2.5 M samples, or
- * edge >= 128 with 2 000 slices and 6 M samples; projector: 11 M samples from edge 512, 19 M from 384, 24 M from 320, 28 M
- * from 256 — else direct),
+ * amortise the plan — backprojector: with fixed-point sums from edge 384 and
+ * 300 slices or edge 256 and 6 000, with FP32 sums (as
+ * GTOMRLN_PATH_SEGMENT_FP32) from edge 276 and 3.3 M samples per volume (2.3 M
+ * between edges 320 and 447); shifted backprojector: edge 256 and 2.5 M
+ * samples, or edge 128 with 2 000 slices and 6 M samples; projector: 11 M
+ * samples from edge 512, 19 M from 384, 24 M from 320, 28 M from 256 — else
+ * direct),
  * GTOMRLN_PATH_DIRECT (one thread per slice element, global gathers /
  * reductions), GTOMRLN_PATH_BRICK (brick-major, shared-memory staging, pixels
  * binned per brick by a planning pass; falls back to direct where the
@@ -91,9 +95,11 @@ GTOMRLN_API int gtomrln_release_caches(void);
 #define GTOMRLN_PATH_SEGMENT 3
 #define GTOMRLN_PATH_FUSED 4
 /* op GTOMRLN_OP_BACKPROJECT: the row-segment kernel with FP32 shared-memory
- * atomics only (GTOMRLN_PATH_SEGMENT and AUTO first accumulate each work
- * item in fixed point with int32 atomics, at the FP32 path's accuracy, and
- * fall back to FP32 for an item whose sums could overflow). */
+ * atomics only.  GTOMRLN_PATH_SEGMENT, and AUTO for large batches, first
+ * accumulate each work item in fixed point with int32 atomics, in steps of
+ * 2^-25 of the brick's largest sampled magnitude (norm-wise the FP32 path's
+ * accuracy, less for a small sum beside large ones), and fall back to FP32
+ * for an item whose sums could overflow or whose data are not finite. */
 #define GTOMRLN_PATH_SEGMENT_FP32 5
 /* op GTOMRLN_OP_GRIDDING: each iteration as four streaming passes over the
  * Hermitian half along z of the (real) iterated spectrum, and the final map
