@@ -427,8 +427,11 @@ static double slice_samples(double rmax) { return 1.5707963 * rmax * rmax; }
 // 330, 3 000: 901 vs 640; n = 160: 1 000: 193 vs 251, 3 000: 531 vs 505;
 // n = 128: 3 000: 341 vs 396, 10 000: 1 068 vs 898; n = 96, 10 000: 610 vs
 // 645.  The direct kernel's cost per sample grows once the volume leaves L2;
-// the segment kernel pays a plan and the staging of every brick first.
-bool project_segment_pays(int V, double rmax, unsigned batch) {
+// the segment kernel pays a plan and the staging of every brick first.  Under
+// stream capture the plan's scratch becomes the graph's own memory: large
+// batches only.
+bool project_segment_pays(int V, double rmax, unsigned batch, bool capturing) {
+  if (capturing) return (V >= 512 && batch >= 1000) || (V >= 384 && batch >= 6000);
   const double samples = slice_samples(rmax) * batch;
   return samples >= (V >= 512 ? 11e6 : V >= 384 ? 19e6 : V >= 320 ? 24e6 : V >= 256 ? 28e6 : 1e300);
 }
@@ -447,10 +450,13 @@ bool project_segment_pays(int V, double rmax, unsigned batch) {
 // that.  Where the direct kernel has its packed scratch (V <= 275 for one
 // volume) it stays ahead (n = 128, 1 000: 372 vs 396; n = 100, 3 333: 542 vs
 // 728).  The samples are those of one volume: every volume has its own bricks
-// (n = 64, 4 096 slices into 1 024 volumes: 1.9 ms direct, 10 ms in bricks).
-InsertSums insert_auto(int V, double rmax, unsigned batch, int volumes, bool packed) {
-  if ((V >= 384 && batch >= 300) || (V >= 256 && batch >= 6000)) return InsertSums::kFixed;
-  if (packed || V < 256 || volumes < 1) return InsertSums::kDirect;
+// (n = 64, 4 096 slices into 1 024 volumes: 1.9 ms direct, 10 ms in bricks).  Under
+// stream capture as the projector.
+static bool insert_large(int V, unsigned batch) { return (V >= 384 && batch >= 300) || (V >= 256 && batch >= 6000); }
+
+InsertSums insert_auto(int V, double rmax, unsigned batch, int volumes, bool packed, bool capturing) {
+  if (insert_large(V, batch)) return InsertSums::kFixed;
+  if (capturing || packed || V < 256 || volumes < 1) return InsertSums::kDirect;
   const double samples = slice_samples(rmax) * batch / volumes;
   return samples >= (V >= 320 && V < 448 ? 2.3e6 : 3.3e6) ? InsertSums::kFp32 : InsertSums::kDirect;
 }
@@ -460,7 +466,8 @@ InsertSums insert_auto(int V, double rmax, unsigned batch, int volumes, bool pac
 // 282 vs 307, 3 333: 458 vs 291; n = 96: 1 000: 288 vs 624, 2 000: 544 vs
 // 472; n = 128: 300: 162 vs 206, 400: 210 vs 203; n = 160: 150: 195 vs 208,
 // 300: 356 vs 249; n = 256: 100: 613 vs 607, 150: 921 vs 653.
-bool insert_shifted_segment_pays(int V, double rmax, unsigned batch) {
+bool insert_shifted_segment_pays(int V, double rmax, unsigned batch, bool capturing) {
+  if (capturing) return insert_large(V, batch);
   const double samples = slice_samples(rmax) * batch;
   return V >= 256 ? samples >= (V >= 448 ? 3.1e6 : 2.5e6) : V >= 128 && batch >= 2000 && samples >= 6e6;
 }

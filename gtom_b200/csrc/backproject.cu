@@ -1212,51 +1212,51 @@ static int backproject_launch(float* d_volumeft, float* d_volumeweights, int vx,
   // (the brick plans' integer square roots take radii below 4 096: seg_isqrt)
   InsertSums sums = InsertSums::kDirect;
   if (ndp == 2 && vx == vy && vx == vz && vx >= 4 && a.rmax2 <= (1 << 24) && (d_volumeft || d_volumeweights)) {
-    if (choice == GTOMRLN_PATH_AUTO) sums = insert_auto(vx, (double)rmax, batch, known_vol, packs);
+    if (choice == GTOMRLN_PATH_AUTO) sums = insert_auto(vx, (double)rmax, batch, known_vol, packs, stream_capturing(stream));
     if (choice == GTOMRLN_PATH_BRICK || choice == GTOMRLN_PATH_SEGMENT) sums = InsertSums::kFixed;
     if (choice == GTOMRLN_PATH_SEGMENT_FP32) sums = InsertSums::kFp32;
   }
   const bool brick = sums != InsertSums::kDirect, fixed_point = sums == InsertSums::kFixed;
-  if (brick && plain)
-    return backproject_brick(d_volumeft, d_volumeweights, d_projft, d_projweights, d_matrices, a, (int)rmax,
-                             decentered, square, batch, stream, choice == GTOMRLN_PATH_BRICK ? 0 : 1, false,
-                             nullptr, 1, fixed_point);
+  if (brick && plain) {
+    const int st = backproject_brick(d_volumeft, d_volumeweights, d_projft, d_projweights, d_matrices, a, (int)rmax,
+                                     decentered, square, batch, stream, choice == GTOMRLN_PATH_BRICK ? 0 : 1, false,
+                                     nullptr, 1, fixed_point);
+    if (choice != GTOMRLN_PATH_AUTO || !plan_refused(st)) return st;
+    clear_error();
+  }
   // The general geometry (magnification, Ewald curvature, per-slice volumes)
   // takes the row-segment kernel for centred output when the magnification
   // is well conditioned; per-slice volumes need their count (from the host
   // array, else read back from the device, which waits for the stream and
   // is skipped under stream capture).
-  if (brick && !decentered && choice != GTOMRLN_PATH_BRICK && mag_smin2(mag) > 1e-4 &&
+  if (brick && !plain && !decentered && choice != GTOMRLN_PATH_BRICK && mag_smin2(mag) > 1e-4 &&
       std::fabs(a.ewalddiaminv) < 1.f) {
     int nvol = 1;
     if (d_ivolume) {
       nvol = nvol_hint;
       if (nvol <= 0) {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) {
-          cudaGetLastError();
-          cs = cudaStreamCaptureStatusActive;
-        }
         int mx = -1;
-        if (cs == cudaStreamCaptureStatusNone) {
+        if (!stream_capturing(stream)) {
           int st = device_max_index(d_ivolume, batch, stream, &mx);
           if (st) return st;
         }
         nvol = mx + 1;
       }
     }
-    if (nvol >= 1 && nvol <= 4096)
-      return backproject_brick(d_volumeft, d_volumeweights, d_projft, d_projweights, d_matrices, a, (int)rmax,
-                               decentered, square, batch, stream, 1, true, d_ivolume, nvol, fixed_point);
+    if (nvol >= 1 && nvol <= 4096) {
+      const int st = backproject_brick(d_volumeft, d_volumeweights, d_projft, d_projweights, d_matrices, a, (int)rmax,
+                                       decentered, square, batch, stream, 1, true, d_ivolume, nvol, fixed_point);
+      if (choice != GTOMRLN_PATH_AUTO || !plan_refused(st)) return st;
+      clear_error();
+    }
   }
 
   // The direct kernel.  No packed scratch under stream capture, where the
   // call allocates nothing.
   const dim3 grid((unsigned)(a.tiles * (int64_t)batch));
   if (packs) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     float4* packed = nullptr;
-    if (cudaStreamIsCapturing(stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone &&
+    if (!stream_capturing(stream) &&
         pool_alloc((void**)&packed, sizeof(float4) * (size_t)voxels, stream) == GTOMRLN_OK) {
       cudaError_t e = cudaMemsetAsync(packed, 0, sizeof(float4) * (size_t)voxels, stream);
       launch_bp_direct_any<true>(grid, stream, (float2*)packed, nullptr, (const float2*)d_projft, d_projweights,
@@ -1365,9 +1365,13 @@ int gtomrln_backproject_shifted(float* d_volumeft, float* d_volumeweights, int v
   const int choice = path_choice(GTOMRLN_OP_BACKPROJECT);
   if (ndp == 2 && vx == vy && vx == vz && vx >= 4 && a.rmax2 <= (1 << 24) && (d_volumeft || d_volumeweights) &&
       (choice == GTOMRLN_PATH_BRICK || choice == GTOMRLN_PATH_SEGMENT ||
-       (choice == GTOMRLN_PATH_AUTO && insert_shifted_segment_pays(vx, (double)rmax, batch))))
-    return backproject_shifted_brick(d_volumeft, d_volumeweights, d_projft, d_projweights, d_matrices, d_shifts,
-                                     d_globalweights, a, (int)rmax, batch, (cudaStream_t)stream);
+       (choice == GTOMRLN_PATH_AUTO &&
+        insert_shifted_segment_pays(vx, (double)rmax, batch, stream_capturing((cudaStream_t)stream))))) {
+    const int st = backproject_shifted_brick(d_volumeft, d_volumeweights, d_projft, d_projweights, d_matrices, d_shifts,
+                                             d_globalweights, a, (int)rmax, batch, (cudaStream_t)stream);
+    if (choice != GTOMRLN_PATH_AUTO || !plan_refused(st)) return st;
+    clear_error();
+  }
   dim3 grid((unsigned)(a.tiles * (int64_t)batch));
   if (ndp == 2)
     backproject_shifted_kernel<2><<<grid, kBpThreads, 0, (cudaStream_t)stream>>>(

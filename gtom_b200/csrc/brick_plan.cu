@@ -501,7 +501,7 @@ int release_brick_orders(int dev, unsigned long long ctx) {
   return GTOMRLN_OK;
 }
 
-static int brick_order(const BrickGrid& g, const int** out) {
+static int brick_order(const BrickGrid& g, cudaStream_t stream, const int** out) {
   int dev = 0;
   GTOMRLN_CUDA_TRY(cudaGetDevice(&dev));
   const unsigned long long ctx = context_id();
@@ -512,6 +512,8 @@ static int brick_order(const BrickGrid& g, const int** out) {
     *out = it->second;
     return GTOMRLN_OK;
   }
+  if (stream_capturing(stream))  // its allocation and copy would end the capture
+    return set_error(GTOMRLN_ERR_ALLOC, "brick plan: the first call with a grid cannot be captured");
   std::vector<int> order(g.nbricks);
   std::vector<float> d2(g.nbricks);
   for (int b = 0; b < g.nbricks; b++) {
@@ -546,7 +548,7 @@ int build_brick_plan(int op, const float* d_mats, int batch, const BrickGrid& g,
   const size_t code_bytes = ((size_t)px.elements * 2 + 3) & ~(size_t)3;
   const int use_codes = g.nbricks < 65535 && hist_bytes + code_bytes <= 200 * 1024 ? 1 : 0;
   const int* d_order = nullptr;
-  int st = brick_order(g, &d_order);
+  int st = brick_order(g, stream, &d_order);
   if (st) return st;
   // Capacities: the projector bins each pixel once; the backprojector's
   // pixels land in ~1.2-1.5 bricks on average (8 at most), so twice the

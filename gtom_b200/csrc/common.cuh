@@ -56,9 +56,22 @@ int path_choice(int op);
 // if the call does not know; packed: whether the direct kernel has its packed
 // scratch.
 enum class InsertSums { kDirect, kFp32, kFixed };
-bool project_segment_pays(int V, double rmax, unsigned batch);
-InsertSums insert_auto(int V, double rmax, unsigned batch, int volumes, bool packed);
-bool insert_shifted_segment_pays(int V, double rmax, unsigned batch);
+bool project_segment_pays(int V, double rmax, unsigned batch, bool capturing);
+InsertSums insert_auto(int V, double rmax, unsigned batch, int volumes, bool packed, bool capturing);
+bool insert_shifted_segment_pays(int V, double rmax, unsigned batch, bool capturing);
+
+// Whether a status is that of a brick plan that could not be had (no scratch
+// for it, or more bricks or records than it takes): nothing has reached the
+// outputs then, and AUTO takes the direct kernel instead.
+inline bool plan_refused(int status) { return status == GTOMRLN_ERR_ALLOC || status == GTOMRLN_ERR_INVALID; }
+
+// Whether the stream is being captured (or cannot say).
+inline bool stream_capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &cs) == cudaSuccess) return cs != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
 
 // Launch shape of the brick kernels for op: brick edge in voxels, threads
 // per CTA, and the most slices one work item takes (gtomrln_set_brick_tuning).

@@ -464,8 +464,7 @@ int gtomrln_squared_differences(const float* d_particleft, const float* d_minvsi
   // second pass (a few microseconds), outside stream capture (they need
   // scratch).
   cudaStream_t s = (cudaStream_t)stream;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusActive;
-  if (elements >= 512 && cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone)
+  if (elements >= 512 && !stream_capturing(s))
     return diff2_tensor((const float2*)d_particleft, d_minvsigma2, d_ctf, elements, (const float2*)d_precalcshifts,
                         (const float2*)d_refft, d_diff2, nparticles, nrefs, nshifts, dofirstitercc != 0, s);
   return diff2_direct((const float2*)d_particleft, d_minvsigma2, d_ctf, elements, (const float2*)d_precalcshifts,

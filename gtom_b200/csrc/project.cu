@@ -560,9 +560,13 @@ int gtomrln_project(const float* d_volumeft, int vx, int vy, int vz, float* d_pr
   // the brick plans' integer square roots take radii below 4 096 (seg_isqrt)
   if (ndp == 2 && vx == vy && vx == vz && vx >= 4 && a.rmax2 <= (1 << 24) &&
       (choice == GTOMRLN_PATH_BRICK || choice == GTOMRLN_PATH_SEGMENT ||
-       (choice == GTOMRLN_PATH_AUTO && project_segment_pays(vx, (double)a.rmax, batch))))
-    return project_brick(d_volumeft, d_proj, d_matrices, a, batch, (cudaStream_t)stream,
-                         choice == GTOMRLN_PATH_BRICK ? 0 : 1);
+       (choice == GTOMRLN_PATH_AUTO &&
+        project_segment_pays(vx, (double)a.rmax, batch, stream_capturing((cudaStream_t)stream))))) {
+    st = project_brick(d_volumeft, d_proj, d_matrices, a, batch, (cudaStream_t)stream,
+                       choice == GTOMRLN_PATH_BRICK ? 0 : 1);
+    if (choice != GTOMRLN_PATH_AUTO || !plan_refused(st)) return st;
+    clear_error();
+  }
   ArrayFetch f{(const float2*)d_volumeft, a.P, a.P / 2 + 1, a.nvox - 1};
   return launch_project(f, ndp, d_proj, d_matrices, a, batch, (cudaStream_t)stream);
 }
@@ -621,9 +625,13 @@ int gtomrln_project_shifted(const float* d_volumeft, int vx, int vy, int vz, flo
   // the brick plans' integer square roots take radii below 4 096 (seg_isqrt)
   if (ndp == 2 && vx == vy && vx == vz && vx >= 4 && a.rmax2 <= (1 << 24) &&
       (choice == GTOMRLN_PATH_BRICK || choice == GTOMRLN_PATH_SEGMENT ||
-       (choice == GTOMRLN_PATH_AUTO && project_segment_pays(vx, (double)a.rmax, batch))))
-    return project_brick(d_volumeft, d_proj, d_matrices, a, batch, (cudaStream_t)stream, 1,
-                         ShiftPost{d_shifts, d_globalweights});
+       (choice == GTOMRLN_PATH_AUTO &&
+        project_segment_pays(vx, (double)a.rmax, batch, stream_capturing((cudaStream_t)stream))))) {
+    st = project_brick(d_volumeft, d_proj, d_matrices, a, batch, (cudaStream_t)stream, 1,
+                       ShiftPost{d_shifts, d_globalweights});
+    if (choice != GTOMRLN_PATH_AUTO || !plan_refused(st)) return st;
+    clear_error();
+  }
   ArrayFetch f{(const float2*)d_volumeft, a.P, a.P / 2 + 1, a.nvox - 1};
   return launch_project(f, ndp, d_proj, d_matrices, a, batch, (cudaStream_t)stream,
                         ShiftPost{d_shifts, d_globalweights});
