@@ -7,30 +7,38 @@
 // elements terms (real and imaginary parts), which runs as tcgen05.mma
 // (kind::tf32, FP32 accumulators in tensor memory).
 //
-// Precision.  Every operand is split exactly into hi (its leading 11 bits)
-// and lo (the rest, of which the instruction keeps 11 bits), and hi hi +
-// hi lo + lo hi is accumulated: 22 bits of each product.  hi hi and the
-// cross terms have accumulators of their own, and every 64 elements (16
-// steps of 8) the accumulators are added to FP32 sums in registers with
-// round-to-nearest, because the tensor core's own additions truncate: left
-// alone for the whole sum their bias would reach 1e-4.  A, B and the final
-// combination are summed in double.  The expansion cancels where a and b are
-// close, so a tile of outputs with any diff2 below a quarter of (A + B) / 2
-// (or not finite) is computed again by the direct kernel (estep.cu), whose
-// FP32 sums of |a - b|^2 do not cancel: the relative error stays below the
-// direct kernel's everywhere.  In single-particle data the noise alone keeps
-// diff2 well above that.
+// Precision.  Every operand is split exactly into hi (rounded to 11 bits) and
+// lo (the rest, of either sign, of which the instruction keeps 11 bits), and
+// hi hi + hi lo + lo hi is accumulated: 22 bits of each product.  The tensor
+// core's own additions truncate, so hi hi is added to FP32 sums in registers
+// with round-to-nearest every 32 elements (8 steps); the cross terms, 2^-11 of
+// it, have one accumulator for the whole range.  A and B are FP32 sums of a
+// thread's terms of the range, then of its eight lanes; ranges and the final
+// combination are summed in double.
+//
+// The expansion cancels where a and b are close, so a tile of outputs with
+// any diff2 below half of (A + B) / 2 (or not finite) is computed again by
+// the direct kernel (estep.cu), whose FP32 sums of |a - b|^2 do not cancel.
+// Relative error (rms) against 64 bits by diff2 / ((A + B) / 2), direct and
+// here, at 544 elements, the shortest sums but the least favourable (at 8 320
+// the direct kernel's are 1.1e-6 throughout, at 33 024 4e-6):
+//   0.97: 2.5e-7, 0.4e-7   0.67: 2.3e-7, 1.0e-7   0.50: 2.6e-7, 1.7e-7
+//   0.33: 2.4e-7, 4.3e-7 (and so redone); cross-correlations of the operands'
+//   power: 0.73 of the largest: 2.4e-7, 1.4e-7.
+// (Parts by truncation, drained every 64 elements: 0.50: 6.0e-7.  Drained
+// every 16 elements: 1.0e-7, but 349 instead of 300 us below.)  In
+// single-particle data the noise alone keeps diff2 near (A + B) / 2.
 //
 // One CTA: 128 references x 64 shifts of one particle over a range of
 // elements (split so that every SM has two CTAs' work).  Its 256 threads
 // form the operands of 16 elements at a time in shared memory (128-byte
 // swizzled rows, hi and lo, 48 KB a stage, two stages), one thread issues
 // the 12 matrix instructions of a stage, and a commit on the stage's
-// mbarrier frees it.  Two accumulator sets in tensor memory alternate, so a
-// set is drained while the next is filled.
+// mbarrier frees it.  Two hi hi accumulators in tensor memory alternate, so
+// one is drained while the other is filled.
 //
 // 16 particles x 600 references x 49 shifts at 128^2: 1.54 ms by the direct
-// kernel (bound by its FP32 instructions), 0.29 ms here (bound by the
+// kernel (bound by its FP32 instructions), 0.30 ms here (bound by the
 // instructions that form and split the operands).
 #include <algorithm>
 #include <cstdint>
@@ -44,13 +52,14 @@ namespace {
 
 constexpr int kM = 128, kN = 64, kE = 16;  // references, shifts, elements per stage
 constexpr int kThreads = 256;
-constexpr int kGroup = 4;  // stages per accumulator set
+constexpr int kGroup = 2;  // stages per hi hi accumulator
 constexpr unsigned kABytes = kM * kE * 8, kBBytes = kN * kE * 8;  // one of hi, lo
 constexpr unsigned kStageBytes = 2 * (kABytes + kBBytes);
-constexpr unsigned kTmemCols = 4 * kN;  // two sets of (hi hi, cross terms)
+constexpr unsigned kCross = 2 * kN;     // column of the cross terms, after the two hi hi accumulators
+constexpr unsigned kTmemCols = 4 * kN;  // (a power of two)
 constexpr size_t kSmem = 1024 + 2 * kStageBytes;
 constexpr unsigned long long kWaitNs = 1000000000ull;  // 1 s
-constexpr float kCloseFraction = 0.25f;
+constexpr float kCloseFraction = 0.5f;
 
 // kind::tf32, FP32 accumulators, both operands K-major, 128 x 64.
 constexpr unsigned kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((kN / 8) << 17) | ((kM / 16) << 24);
@@ -111,9 +120,10 @@ __device__ __forceinline__ void tmem_load32(unsigned addr, float* v) {
   for (int i = 0; i < 32; i++) v[i] += __uint_as_float(r[i]);
 }
 
-// Splits v into its leading 11 bits and the exact rest.
+// Splits v into its value rounded to 11 bits and the exact rest (NaN where the
+// rounding overflows).
 __device__ __forceinline__ void split4(float4 v, float4& hi, float4& lo) {
-  auto top = [](float x) { return __uint_as_float(__float_as_uint(x) & 0xffffe000u); };
+  auto top = [](float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); };
   hi = make_float4(top(v.x), top(v.y), top(v.z), top(v.w));
   lo = make_float4(v.x - hi.x, v.y - hi.y, v.z - hi.z, v.w - hi.w);
 }
@@ -237,11 +247,10 @@ __global__ void __launch_bounds__(kThreads, 2) diff2_tc_kernel(const TcArgs a) {
     }
   };
   // warps 0-3 drain columns 0-31 of their lanes' rows, warps 4-7 the others
+  const unsigned lane_tmem = tmem + (unsigned)((warp >> 2) * 32) + ((unsigned)(warp & 3) << 21);
   auto drain = [&](int group) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const unsigned at = tmem + (unsigned)((group & 1) * 2 * kN + (warp >> 2) * 32) + ((unsigned)(warp & 3) << 21);
-    tmem_load32(at, acc);
-    tmem_load32(at + kN, acc);
+    tmem_load32(lane_tmem + (unsigned)((group & 1) * kN), acc);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   };
 
@@ -257,7 +266,7 @@ __global__ void __launch_bounds__(kThreads, 2) diff2_tc_kernel(const TcArgs a) {
         ok = false;
         return;
       }
-      if (t % kGroup == 1) drain(drained++);  // and with chunk t - 2 its accumulator set
+      if ((t - 1) % kGroup == 0) drain(drained++);  // and with chunk t - 2 its accumulator
     }
     unsigned char* st = stage0 + s * kStageBytes;
 #pragma unroll
@@ -287,13 +296,13 @@ __global__ void __launch_bounds__(kThreads, 2) diff2_tc_kernel(const TcArgs a) {
       const unsigned sb0 = base + s * kStageBytes;
       const unsigned long long ah = tile_desc(sb0), al = tile_desc(sb0 + kABytes), bh = tile_desc(sb0 + 2 * kABytes),
                                bl = tile_desc(sb0 + 2 * kABytes + kBBytes);
-      const unsigned d = tmem + (unsigned)(((t / kGroup) & 1) * 2 * kN);
+      const unsigned d = tmem + (unsigned)(((t / kGroup) & 1) * kN), dc = tmem + kCross;
       const unsigned first = t % kGroup == 0;
 #pragma unroll
       for (int k = 0; k < 4; k++) {  // 8 values (32 bytes) a step
         mma_tf32(d, ah + 2 * k, bh + 2 * k, !(first && k == 0));
-        mma_tf32(d + kN, ah + 2 * k, bl + 2 * k, !(first && k == 0));
-        mma_tf32(d + kN, al + 2 * k, bh + 2 * k, 1);
+        mma_tf32(dc, ah + 2 * k, bl + 2 * k, t > 0 || k > 0);
+        mma_tf32(dc, al + 2 * k, bh + 2 * k, 1);
       }
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                        smem_u32(&bars[s]))
@@ -313,8 +322,12 @@ __global__ void __launch_bounds__(kThreads, 2) diff2_tc_kernel(const TcArgs a) {
     const int t = nch - 1;
     ok = bar_wait(smem_u32(&bars[t & 1]), (unsigned)(t >> 1) & 1u);
     ok = __syncthreads_and(ok);
-    if (ok)
+    if (ok) {
       while (drained <= t / kGroup) drain(drained++);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      tmem_load32(lane_tmem + kCross, acc);
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    }
   }
   // a wait that ran out (nothing of this kernel's own can cause it): NaN,
   // after one more wait for the matrix instructions in flight
