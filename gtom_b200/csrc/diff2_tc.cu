@@ -64,6 +64,13 @@ constexpr float kCloseFraction = 0.5f;
 // kind::tf32, FP32 accumulators, both operands K-major, 128 x 64.
 constexpr unsigned kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((kN / 8) << 17) | ((kM / 16) << 24);
 
+// The last of `issued` chunks (more than s) in stage s; chunk t is in stage
+// t & 1, as that stage's phase t >> 1.
+__host__ __device__ constexpr int last_chunk(int issued, int s) { return issued - 1 - ((issued - 1 - s) & 1); }
+static_assert(last_chunk(1, 0) == 0 && last_chunk(2, 0) == 0 && last_chunk(2, 1) == 1 && last_chunk(5, 0) == 4 &&
+                  last_chunk(5, 1) == 3 && last_chunk(6, 0) == 4 && last_chunk(6, 1) == 5,
+              "last_chunk: the latest chunk of the stage");
+
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 // Shared-memory descriptor of a K-major tile of 128-byte swizzled rows
@@ -255,7 +262,7 @@ __global__ void __launch_bounds__(kThreads, 2) diff2_tc_kernel(const TcArgs a) {
   };
 
   bool ok = true;
-  int drained = 0;
+  int drained = 0, issued = 0;  // accumulators read back; chunks whose matrix instructions were issued
   // chunk t from its raw operands, which are then those of chunk t + 2 (two
   // chunks ahead: one does not cover the loads' latency)
   auto step = [&](Raw& q, int t) {
@@ -308,6 +315,7 @@ __global__ void __launch_bounds__(kThreads, 2) diff2_tc_kernel(const TcArgs a) {
                        smem_u32(&bars[s]))
                    : "memory");
     }
+    issued = t + 1;
     if (t + 2 < nch) fetch(q, t + 2);
   };
   Raw q0, q1;
@@ -329,9 +337,12 @@ __global__ void __launch_bounds__(kThreads, 2) diff2_tc_kernel(const TcArgs a) {
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
   }
-  // a wait that ran out (nothing of this kernel's own can cause it): NaN,
-  // after one more wait for the matrix instructions in flight
-  if (!ok) bar_wait(smem_u32(&bars[0]), 0u);
+  // a wait that ran out (nothing of this kernel's own can cause it): NaN, after
+  // one more wait for the last matrix instructions of either stage, which must
+  // not be in flight when the tensor memory is given back
+  if (!ok)
+    for (int s = 0; s < 2; s++)
+      if (issued > s) bar_wait(smem_u32(&bars[s]), (unsigned)(last_chunk(issued, s) >> 1) & 1u);
   const float bad = ok ? 0.f : __int_as_float(0x7fc00000);
   {
     const unsigned r = r0 + (warp & 3) * 32 + lane;
