@@ -483,7 +483,10 @@ static int reconstruct(const float* d_dataft, const float* d_weight, float* d_ou
   // the grids they take) or, when the caller chose it, the fused FFT
   // iteration (gridfft.cu); cuFFT transforms otherwise and for the final map.
   const int gpath = path_choice(GTOMRLN_OP_GRIDDING);
-  const bool sym = (gpath == GTOMRLN_PATH_SYMMETRIC || gpath == GTOMRLN_PATH_AUTO) && gridsym_available(P);
+  // (Under stream capture a grid whose twiddle table is still to be made stays
+  // with cuFFT: the caller may hold plans, or they are in the cache.)
+  const bool sym = (gpath == GTOMRLN_PATH_SYMMETRIC || gpath == GTOMRLN_PATH_AUTO) && gridsym_available(P) &&
+                   (fft_twiddles_known(P) || !stream_capturing(stream));
   const bool fused = !sym && gpath == GTOMRLN_PATH_FUSED && !measure_ref && gridfft_available(P, 1);
   bool need_first = true;  // both start with a transform along z
   // (a predicted start reads neighbours outside the sphere, momentum copies

@@ -544,4 +544,12 @@ int release_gridfft_tables(int dev, unsigned long long ctx) { return release_tab
 
 int fft_twiddles(int N, const float2** out) { return twiddles(N, out); }
 
+bool fft_twiddles_known(int N) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  const auto key = std::make_tuple(dev, context_id(), N);
+  std::lock_guard<std::mutex> lock(g_tw_mutex);
+  return g_tw.count(key) != 0;
+}
+
 }  // namespace gtomrln

@@ -195,6 +195,8 @@ int gridfft_iteration(float2* data, const GridGeom& g, int count, const float* t
 // per device, context and N in double precision; freed by the library's
 // cache release).
 int fft_twiddles(int N, const float2** out);
+// Whether it is there already (making it allocates, which no capture allows).
+bool fft_twiddles_known(int N);
 
 // ------------------------------------------- symmetric-spectrum path --
 // The iteration on the Hermitian half along z of the real spectrum

@@ -10,6 +10,7 @@ import pytest
 import torch
 
 import gtom_b200 as G
+from gtom_b200 import _lib
 from gtom_b200 import batch as GB
 from oracle import oracle as O
 from tests.helpers import rel_l2
@@ -111,3 +112,24 @@ def test_data_that_are_not_finite_spread(gtom_lib, cuda, ori, at, iterations):
         _on(path, lambda: G.d_ReconstructGridding(_dev(data.reshape(-1)), _dev(w), out, (ori,) * 3, (D,) * 3, 2, 0, 0,
                                                   iterations))
         assert not torch.isfinite(out).any()
+
+
+@pytest.mark.parametrize("ori", [44, 160])
+def test_captured_call_before_the_tables(gtom_lib, cuda, ori):
+    """A captured call with cuFFT's plans at hand, on a grid the symmetric path
+    has not seen: its twiddle table cannot be made there, so the plans do the
+    work."""
+    data, w, D = _inputs(ori)
+    d_data, d_w, out = _dev(data), _dev(w), torch.zeros(ori ** 3, device="cuda")
+    run = lambda: G.d_ReconstructGridding(d_data, d_w, out, (ori,) * 3, (D,) * 3, 2, 0, 0, 3)
+    torch.cuda.synchronize()
+    _lib.call("gtomrln_release_caches")
+    _on("direct", run)
+    want = out.clone()
+    out.zero_()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        run()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert rel_l2(out.cpu().numpy(), want.cpu().numpy()) <= 1e-6
