@@ -507,6 +507,16 @@ def small_config_ours(G, torch, dev):
                    "total": round(sum(best), 4)}}
 
 
+def symmetric_grid(P):
+    """Whether the default gridding path on grid P is the symmetric one: even,
+    16 .. 768, no prime factor above 13, or 800 (GTOMRLN_PATH_SYMMETRIC)."""
+    rest = P
+    for p in (2, 3, 5, 7, 11, 13):
+        while rest % p == 0:
+            rest //= p
+    return P == 800 or (P % 2 == 0 and 16 <= P <= 768 and rest == 1)
+
+
 def time_gridding(G, torch, acc_ft, acc_w, n, D, dev):
     out = torch.empty(n ** 3, dtype=torch.float32, device=dev)
     G.d_ReconstructGridding(acc_ft, acc_w, out, (n,) * 3, (D,) * 3, PAD, 0, 0, 1)  # plans, pool
@@ -534,7 +544,7 @@ def time_gridding(G, torch, acc_ft, acc_w, n, D, dev):
     sym_bytes = int((4 + 4 * circle) * 8 * nw + 12 * (2 / 3) * math.pi * (P // 2) ** 3)
     per_it = (ms10 - ms1) / 9
     res = {"ms_10_iterations": round(ms10, 3), "ms_per_iteration": round(per_it, 4), "P": P,
-           "path": "symmetric (four passes over the Hermitian half along z)" if P in (64, 128, 256, 512) else "cufft",
+           "path": "symmetric (four passes over the Hermitian half along z)" if symmetric_grid(P) else "cufft",
            "compulsory_bytes_per_iteration": compulsory, "path_bytes_per_iteration": sym_bytes,
            "path_gbs": round(sym_bytes / (per_it * 1e-3) / 1e9, 1), "to_1e-4": {}}
     hbm, hbm_kind = measured_peaks()

@@ -582,9 +582,10 @@ int build_brick_plan(int op, const float* d_mats, int batch, const BrickGrid& g,
     // item, which costs as much as a few dozen records): with larger ones the
     // central bricks, which every slice crosses, keep single CTAs busy after
     // the others have finished.  The backprojector's are not cut below 512,
-    // where its extra flushes by reductions cost more than they even out, and
-    // where only a forced path comes here (small volumes, small batches)
-    // items stay whole.
+    // where its extra flushes cost more than they even out.  Below edge 256
+    // and 2 000 slices, where only a forced path comes here, its items stay
+    // whole: the FP32 sums of a whole item follow the port's serial order more
+    // closely where thousands of equal terms meet in one voxel.
     const double share = 0.4 * est * batch / (8.0 * sms);
     if (op == GTOMRLN_OP_PROJECT)
       chunk = (int)std::min<double>(chunk, std::max(128.0, share));

@@ -102,7 +102,8 @@ __global__ void ctf_simulate_kernel(float* __restrict__ out, const float2* __res
 // particle is evaluated as ctf_simulate_kernel does for that address.  Bound
 // by issue (58 % busy) and latency: with four particles and sixteen loads of
 // parameters each it took 102 instructions per element.  2 000 particles of
-// 256^2, both FFT passes included: 795 -> 749 us.
+// 256^2, both FFT passes included: 795 -> 749 us on one GPU (830 -> 788 on
+// another).
 constexpr int kPrePB = 8;
 __global__ void __launch_bounds__(256, 4)
 preprocess_kernel(float2* __restrict__ ft, float* __restrict__ weights, int n, int batch,

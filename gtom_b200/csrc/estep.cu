@@ -460,9 +460,12 @@ int gtomrln_squared_differences(const float* d_particleft, const float* d_minvsi
   if (nparticles > 65535)
     return set_error(GTOMRLN_ERR_INVALID, "squared_differences: more than 65535 particles per call");
   // The dense layout does not depend on the group size.  The tensor cores
-  // take it where the sums are long enough to pay for the partial products'
-  // second pass (a few microseconds), outside stream capture (they need
-  // scratch).
+  // take it from 512 elements on, outside stream capture (they need scratch):
+  // the direct kernel's time grows with the elements of one tile whatever the
+  // counts (us, particles x references x shifts, direct against tensor cores:
+  // 544 elements: 1 x 1 x 1 66 vs 39, 64 x 64 x 30 68 vs 45, 400 x 1 x 1 157
+  // vs 101; 8 320: 1 x 1 x 1 824 vs 43, 400 x 1 x 1 2 217 vs 1 100; at 312 the
+  // direct kernel needs 44).
   cudaStream_t s = (cudaStream_t)stream;
   if (elements >= 512 && !stream_capturing(s))
     return diff2_tensor((const float2*)d_particleft, d_minvsigma2, d_ctf, elements, (const float2*)d_precalcshifts,

@@ -49,8 +49,8 @@
 // Measured at P = 512 (us): y 83 and 88 (76 at the copy rate), x 156 (85;
 // bound by its load/store and FP32 instructions), z 233 (132; 24 warps per SM
 // in phases of loads, two transforms and stores); with the whole grid they
-// were 100, 100, 156 and 335.  Ten iterations and the map 7.97 -> 6.24 ms;
-// P = 128 384 -> 221 us.
+// were 100, 100, 156 and 335.  Ten iterations and the map 7.97 -> 6.2 ms
+// (8.1 -> 6.6 on another GPU); P = 128 384 -> 221 us.
 //
 // Transforms.  A real transform of length P runs as a complex transform of
 // length H = P/2 on the packed pairs (x(2n), x(2n+1)) with the usual pre-

@@ -112,7 +112,9 @@ GTOMRLN_API int gtomrln_set_path(int op, int path);
 
 /* Extension (no reference counterpart): launch shape of the brick-major
  * kernels of op for the calling process — brick edge in voxels, threads per
- * CTA (multiple of 32, <= 1024) and the most slices one work item takes.
+ * CTA (multiple of 32, <= 1024) and the most slices one work item takes
+ * (row segments: the most records, of which a batch's plan may take fewer so
+ * that its items fill the GPU).
  * 0 keeps the built-in default for that field.  Results do not depend on
  * these (the projector's are bit-identical for any shape); speed does.
  * Returns GTOMRLN_ERR_INVALID for shapes whose shared memory exceeds a CTA's. */
@@ -190,8 +192,12 @@ GTOMRLN_API int gtomrln_project_tex_angles(unsigned long long t_volumeRe, unsign
  * a half-complex volume and a weight volume, accumulated in place.
  * d_projft == NULL inserts (1, 0); d_projweights == NULL inserts weight 1;
  * d_volumeft or d_volumeweights == NULL skips that output.  d_ivolume
- * (optional) selects a target volume per slice.  The trilinear weights are
- * rounded through binary16 exactly as the reference does
+ * (optional) selects a target volume per slice; given on the
+ * device, its largest index is read back, which waits for the stream, where
+ * AUTO uses fixed-point sums or a brick path is forced.  All
+ * additions to the volumes are reductions: calls that overlap on different
+ * streams may insert into the same ones.  The trilinear weights are rounded
+ * through binary16 exactly as the reference does
  * (src/Relion/Backproject.cu:224-238).
  * ------------------------------------------------------------------------- */
 

@@ -295,3 +295,22 @@ def test_fixed_point_falls_back_to_fp32(cuda, kind):
     O.backproject(of, ow, V, projft, projw, n, n // 2, mats, decentered=False, fp32=True)
     assert np.all(np.isfinite(fx[0])) and np.all(np.isfinite(fx[1]))
     assert rel_l2(fx[0], of) <= 1e-5 and rel_l2(fx[1], ow) <= 1e-5
+
+
+def test_cut_items_fall_back_to_fp32(cuda):
+    """2 500 slices of one orientation with identical data: the bricks' records
+    are cut into several items, whose fixed-point sums could overflow, so each
+    is accumulated again in FP32.  The result is 2 500 times one slice's, to
+    the rounding of 2 500 FP32 additions (2 500 * 2^-24 = 1.5e-4); an item
+    missed or added twice would be off by a share of 1 / items or more."""
+    rng = np.random.default_rng(78)
+    n, V, batch = 64, 129, 2500
+    e = O.elements_fft(n)
+    m = O.matrices_f64(random_angles(rng, 1), 2.0).astype(np.float32)
+    one = (rng.normal(size=(1, e)) + 1j * rng.normal(size=(1, e))).astype(np.complex64)
+    w = rng.uniform(0.5, 1.0, size=(1, e)).astype(np.float32)
+    single = _bp_segment("direct", V, n, m, one, w)
+    got = _bp_segment("segment", V, n, np.repeat(m, batch, 0), np.repeat(one, batch, 0), np.repeat(w, batch, 0))
+    want = batch * single[1].astype(np.float64)
+    assert np.all(np.abs(got[1] - want) <= 1.5e-4 * want + 1e-30)
+    assert rel_l2(got[0], batch * single[0].astype(np.complex128)) <= 1.5e-4
